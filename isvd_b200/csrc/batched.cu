@@ -701,28 +701,30 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
     }
     P.l1.run(st, true);
     P.l2.run(st, true);
-    // the steps grouped by their number of 32 x 32 product tiles, nt = ceil(l / 32)^2, one launch
-    // per group with the cluster size c that minimises waves x tiles per CTA,
-    // ceil(count c / SMs) ceil(nt / c) (one 1024-thread CTA per SM); the groups (at most three for
-    // l <= 96) run side by side, the largest on the library stream, the others on side streams
-    auto tiles_of = [](const KnStep &s) { return ((s.l + 31) / 32) * ((s.l + 31) / 32); };
+    // the steps grouped by ceil(l / 32), one launch per group with the cluster size c that minimises
+    // waves x time of a product, ceil(count c / SMs) (rows l^2 / 66 + 700) cycles: a CTA's rows =
+    // 8 ceil(l / 8 / c) of an l x l product at 66 FP64 FMAs per cycle, and the barrier and latency
+    // between two products (one CTA per SM); the groups (at most three for l <= 96) run side by
+    // side, the largest on the library stream, the others on side streams
+    auto class_of = [](const KnStep &s) { return (s.l + 31) / 32; };
     std::stable_sort(hsteps.begin(), hsteps.end(),
-                     [&](const KnStep &x, const KnStep &y) { return tiles_of(x) > tiles_of(y); });
+                     [&](const KnStep &x, const KnStep &y) { return class_of(x) > class_of(y); });
     P.steps.upload(hsteps, st);
     P.make_side_streams();
     CK(cudaEventRecord(P.fork, st));
     int group = 0;
     const int sms = rt.num_sms;
     for (size_t g0 = 0; g0 < hsteps.size(); ++group) {
-      const int nt = tiles_of(hsteps[g0]);
+      const int cls = class_of(hsteps[g0]);
       size_t g1 = g0;
       int lmax = 0;
-      while (g1 < hsteps.size() && tiles_of(hsteps[g1]) == nt) lmax = std::max(lmax, hsteps[g1++].l);
+      while (g1 < hsteps.size() && class_of(hsteps[g1]) == cls) lmax = std::max(lmax, hsteps[g1++].l);
       const long long cnt = (long long)(g1 - g0);
       int best_c = 1;
       long long best = -1;
-      for (int c = 1; c <= 8 && c <= nt; c *= 2) {
-        const long long cost = ((cnt * c + sms - 1) / sms) * ((nt + c - 1) / c);
+      for (int c = 1; c <= 8 && 8 * c <= lmax + 7; c *= 2) {
+        const long long rows = 8 * (((lmax + 7) / 8 + c - 1) / c);
+        const long long cost = ((cnt * c + sms - 1) / sms) * (rows * lmax * lmax / 66 + 700);
         if (best < 0 || cost < best) { best = cost; best_c = c; }
       }
       cudaStream_t gs = st;

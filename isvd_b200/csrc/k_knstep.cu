@@ -11,13 +11,25 @@
 // sum_{n>d} max(|c_n|, |d_n|) (rho / 4)^n is below the target.  When no degree up to the table
 // size reaches it (rho close to 1), the step runs the Newton-Schulz iteration instead.
 //
-// The cost of the step is the chain of dependent l x l products, not their flops (2 l^3 = 4 MFLOP
-// at l = 128).  All phases run in one cluster of up to 16 CTAs: operands stay in L2, a product is
-// split in 32 x 32 output tiles spread over the CTAs, and phases are separated by the hardware
-// cluster barrier (release / acquire at cluster scope), which costs a fraction of a microsecond
-// where a grid-wide barrier through global atomics costs several.  Every CTA follows the same
-// control flow (degrees and step counts are read from memory after a barrier), and there is no
-// software spin-wait.
+// The cost of the step is the chain of dependent l x l products and the barriers between them, not
+// their flops (2 l^3 = 4 MFLOP at l = 128).  Every matrix of the chain is a polynomial in the
+// symmetric Z, so the chain is cut by rows (kn_rows_kernel, l <= 128): a CTA of the cluster owns
+// eight (or more) rows of every matrix in shared memory and holds one whole right operand (Z, then
+// Z^4 or Z^8, then Dc) beside them.  A product of its rows with the whole operand is then local to
+// the CTA, a __syncthreads() apart from the next one; only a new right operand is exchanged (rows
+// written to L2, one hardware cluster barrier, read back whole).  A step near convergence makes two
+// such exchanges where the tile-split form below made one per product.  l in (128, 160] keeps that
+// form (kn_cluster_kernel): the whole operand and the rows do not fit in shared memory together.
+// Every CTA follows the same control flow (decisions come from values that all CTAs compute alike),
+// and there is no software spin-wait.
+//
+// What bounds a step: at l = 128 a CTA's product of eight rows, 2000 cycles of the SM's FP64 pipe (66
+// FMA per cycle); at l <= 32 the latency of a product (about 0.3 us) and of the two exchanges (2 us
+// each).  Measured per step, the first step of a loop / one near convergence, tile-split form ->
+// rows: l = 11 107 / 29 -> 24 / 11 us, l = 32 341 / 34 -> 28 / 12, l = 65 548 / 42 -> 59 / 17,
+// l = 96 593 / 45 -> 80 / 21, l = 128 649 / 48 -> 141 / 28 (the first steps took Newton-Schulz for
+// want of the sharper bound on ||4 Z||_2 below and of a table of 128 coefficients).  Clusters of
+// fewer, longer row blocks are slower: l = 96 near convergence 27 us on 8 CTAs, 34 on 4.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -43,19 +55,7 @@ constexpr int kKsPer = (32 * kKsMaxL + kKsThreads - 1) / kKsThreads;
 struct Ks {
   int l, nr, cs, rank;
   double *As, *Bs, *part;
-  // one-CTA steps (cs == 1) with l <= kKsFullL: both operands of a product staged whole in shared
-  // memory (A: roundup(l, 32) rows of row stride ald, B: l4 rows of row stride bld), so that the
-  // CTA's nr^2 tiles read L2 once per product instead of once per tile
-  bool full;
-  int ald, bld;
 };
-constexpr int kKsFullL = 96;
-__host__ __device__ constexpr int ks_full_ld(int l) { return (l + 31) / 32 * 32 + 4; }  // 4 (mod 16) doubles
-// dynamic shared memory of the whole-operand layout: A, B and the two halves' 32 x 32 partial sums
-__host__ __device__ constexpr size_t ks_full_smem(int l) {
-  return ((size_t)((l + 31) / 32 * 32) * ks_full_ld(l) + (size_t)((l + 3) & ~3) * ks_full_ld(l) + 2 * 1024) *
-         sizeof(double);
-}
 
 // C = alpha A B + beta Cin + diag I on the 32 x 32 output tiles [tile_begin, tile_end) of a phase
 // (tiles numbered across the products of the phase); CTA r takes the tiles t = r mod cs.
@@ -72,47 +72,6 @@ __device__ void ks_mm(const Ks &k, int tile_begin, int tile_end, double alpha, c
   const int lane = tid & 31, half = ty >> 4, mt = ty & 15, ti = mt >> 2, tj = mt & 3;  // warp: 8 x 8 tile, half
   const int l4 = (l + 3) & ~3, kh = ((l4 >> 1) + 3) & ~3;
   const int kb = half * kh, ke = min(l4, kb + kh);
-  if (k.full) {  // cs == 1: every tile of [tile_begin, tile_end) in this CTA, operands staged once
-    const int lr = (l + 31) & ~31;
-    __syncthreads();  // the previous product's reads of the staged operands are done
-    for (int e = tid; e < lr * k.ald; e += kKsThreads) {  // A rows [0, lr) x columns [0, ald), zero outside l x l
-      const int r = e / k.ald, cc = e - r * k.ald;
-      k.As[e] = (r < l && cc < l) ? __ldcg(A + (size_t)r * l + cc) : 0.0;
-    }
-    for (int e = tid; e < l4 * k.bld; e += kKsThreads) {  // B rows [0, l4) x columns [0, bld)
-      const int r = e / k.bld, cc = e - r * k.bld;
-      k.Bs[e] = (r < l && cc < l) ? __ldcg(B + (size_t)r * l + cc) : 0.0;
-    }
-    __syncthreads();
-    for (int t = tile_begin; t < tile_end; ++t) {
-      const int tt = t - tile_begin;
-      const int i0 = (tt / k.nr) * 32, j0 = (tt % k.nr) * 32;
-      const int i = i0 + ty, j = j0 + tx;
-      const double cin = (beta != 0.0 && i < l && j < l) ? __ldcg(Cin + (size_t)i * l + j) : 0.0;
-      double d[2] = {0.0, 0.0};
-      const double *ap = k.As + (i0 + ti * 8 + (lane >> 2)) * k.ald + (lane & 3);
-      const double *bq = k.Bs + (lane & 3) * k.bld + j0 + tj * 8 + (lane >> 2);
-      for (int kk = kb; kk < ke; kk += 4)
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                     : "+d"(d[0]), "+d"(d[1])
-                     : "d"(ap[kk]), "d"(bq[kk * k.bld]));
-      double *part = k.part + half * 1024;
-      const int orow = ti * 8 + (lane >> 2), ocol = tj * 8 + 2 * (lane & 3);
-      __syncthreads();  // the previous tile's epilogue reads of the partial sums are done
-      part[orow * 32 + ocol] = d[0];
-      part[orow * 32 + ocol + 1] = d[1];
-      __syncthreads();
-      const int o = ty * 32 + tx;
-      const double acc = k.part[o] + k.part[1024 + o];
-      if (i < l && j < l) {
-        const double v = alpha * acc + beta * cin + (i == j ? diag : 0.0);
-        C[(size_t)i * l + j] = v;
-        if (C2) C2[(size_t)i * l + j] = v;
-        if (C3) C3[(size_t)i * l + j] = v;
-      }
-    }
-    return;
-  }
   const int first = tile_begin + (((k.rank - tile_begin) % k.cs) + k.cs) % k.cs;
   for (int t = first; t < tile_end; t += k.cs) {
     const int tt = t - tile_begin;
@@ -196,36 +155,42 @@ __device__ double ks_cluster_sum(const Ks &k, cg::cluster_group &cluster, double
 }
 
 // Series degree for rho >= ||4 Z||_2: the smallest d whose tail bound
-//   tail(d) = sum_{d < n < 64} max(|c_n|, |d_n|) (rho / 4)^n + (table remainder)
+//   tail(d) = sum_{d < n < 32 PER} max(|c_n|, |d_n|) (rho / 4)^n + (table remainder)
 // is below the target, or -1 (the remainder beyond the table is bounded by the last term times
-// rho / (1 - rho)).  Evaluated by one warp: lane j holds the terms 2j and 2j + 1, suffix sums by
-// shuffles, and tail is decreasing in d, so the degree is the first d whose bound passes.
+// rho / (1 - rho)).  Evaluated by one warp: lane j holds the terms PER j .. PER j + PER - 1, suffix
+// sums by shuffles, and tail is decreasing in d, so the degree is the first d whose bound passes.
+template <int PER>
 __device__ int ks_degree_warp(const KnSeries &ser, double rho, double target) {
   if (!(rho < 0.9)) return -1;
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, n0 = 2 * lane;
+  const int lane = threadIdx.x & 31, n0 = PER * lane;
   const double x = 0.25 * rho;
-  double xn = 1.0, b = x;  // x^(2 lane) by repeated squaring
+  double xn = 1.0, b = x;  // x^(PER lane) by repeated squaring
   for (int e = n0; e; e >>= 1, b *= b)
     if (e & 1) xn *= b;
-  const double t0 = fmax(fabs(ser.c[n0]), fabs(ser.d[n0])) * xn;
-  const double t1 = fmax(fabs(ser.c[n0 + 1]), fabs(ser.d[n0 + 1])) * (xn * x);
-  const double rem = __shfl_sync(full, t1, 31) * rho / (1.0 - rho);
+  double t[PER], sum = 0.0;
+#pragma unroll
+  for (int u = 0; u < PER; ++u, xn *= x) {
+    t[u] = fmax(fabs(ser.c[n0 + u]), fabs(ser.d[n0 + u])) * xn;
+    sum += t[u];
+  }
+  const double rem = __shfl_sync(full, t[PER - 1], 31) * rho / (1.0 - rho);
   if (rem > target) return -1;
-  // suf = sum of the pairs of lanes lane..31
-  double suf = t0 + t1;
+  double suf = sum;  // sum of the terms of lanes lane..31
   for (int o = 1; o < 32; o <<= 1) {
     const double v = __shfl_down_sync(full, suf, o);
     if (lane + o < 32) suf += v;
   }
-  const double after = __shfl_down_sync(full, suf, 1);  // pairs of lanes lane+1..31
-  const double tail_odd = rem + (lane < 31 ? after : 0.0);  // d = 2 lane + 1
-  const double tail_even = tail_odd + t1;                     // d = 2 lane
-  const unsigned ok_even = __ballot_sync(full, tail_even <= target);
-  const unsigned ok_odd = __ballot_sync(full, tail_odd <= target);
-  const int le = ok_even ? __ffs(ok_even) - 1 : 64, lo = ok_odd ? __ffs(ok_odd) - 1 : 64;
-  const int d = min(2 * le, 2 * lo + 1);
-  return d < 64 ? d : 63;
+  const double after = __shfl_down_sync(full, suf, 1);  // terms of lanes lane+1..31
+  double tail = rem + (lane < 31 ? after : 0.0);        // d = n0 + PER - 1
+  int d = PER * 32;
+#pragma unroll
+  for (int u = PER - 1; u >= 0; --u) {
+    const unsigned ok = __ballot_sync(full, tail <= target);
+    if (ok) d = min(d, PER * (__ffs(ok) - 1) + u);
+    tail += t[u];
+  }
+  return min(d, PER * 32 - 1);
 }
 
 // Block size s of the Paterson-Stockmeyer scheme: fewest dependent products, then the smallest.
@@ -242,7 +207,7 @@ __device__ int ks_block_size(int deg) {
   return sb;
 }
 
-__device__ __forceinline__ void kn_cluster_body(const KnStep &a, const KnSeries &ser, bool full = false) {
+__global__ void __launch_bounds__(kKsThreads, 1) kn_cluster_kernel(KnStep a, KnSeries ser) {
   extern __shared__ double sm[];
   __shared__ double red[kKsThreads / 32];
   __shared__ int plan[3];  // degree (-1: Newton-Schulz), block size, Newton-Schulz steps
@@ -250,14 +215,7 @@ __device__ __forceinline__ void kn_cluster_body(const KnStep &a, const KnSeries 
   const int l = a.l;
   const size_t ll = (size_t)l * l;
   Ks k{l, (l + 31) / 32, (int)cluster.num_blocks(), (int)cluster.block_rank(), sm, sm + 32 * kAld,
-         sm + 32 * kAld + (kKsMaxL + 4) * kBld, false, kAld, kBld};
-  if (full) {  // the whole-operand layout (the launch sized the dynamic shared memory for it)
-    k.full = true;
-    k.ald = k.bld = ks_full_ld(l);
-    k.As = sm;
-    k.Bs = sm + (size_t)((l + 31) / 32 * 32) * k.ald;
-    k.part = k.Bs + (size_t)((l + 3) & ~3) * k.bld;
-  }
+         sm + 32 * kAld + (kKsMaxL + 4) * kBld};
   const int nt = k.nr * k.nr;
   const int gtid = k.rank * kKsThreads + threadIdx.x, gstride = k.cs * kKsThreads;
   // work: Z | P_1..P_8 | accC x2 | accCi x2 | BC_0..BC_7 | BI_0..BI_7 (Newton-Schulz: P_1..P_5), then
@@ -277,7 +235,7 @@ __device__ __forceinline__ void kn_cluster_body(const KnStep &a, const KnSeries 
   }
   const double rho = sqrt(ks_cluster_sum(k, cluster, f, slots, red));
   if (threadIdx.x < 32) {
-    const int d = ks_degree_warp(ser, rho, a.ns_target);
+    const int d = ks_degree_warp<2>(ser, rho, a.ns_target);  // blocks B_0..B_7: degree < 64
     if (threadIdx.x == 0) {
       plan[0] = d;
       plan[1] = ks_block_size(d);
@@ -389,14 +347,428 @@ __device__ __forceinline__ void kn_cluster_body(const KnStep &a, const KnSeries 
   }
 }
 
-__global__ void __launch_bounds__(kKsThreads, 1) kn_cluster_kernel(KnStep a, KnSeries ser) { kn_cluster_body(a, ser); }
+// ------------------------------------------------------------------------------------------
+// The step cut by rows.  CTA `rank` owns rows [r0, r0 + rb) of every matrix, kept as blocks of rb
+// rows in shared memory; `full` holds one whole l x l right operand.  Row stride ld = 4 (mod 16)
+// doubles: the mma.sync fragment reads hit 16 distinct bank pairs.  Columns and rows between l and
+// its next multiple of 8 are zero.
+constexpr int kKrThreads = 512;
+constexpr int kKrWarps = kKrThreads / 32;
+constexpr int kKrMaxL = 128;
+constexpr int kKrBlocks = 8;       // Z, Z^2, Z^3, scratch, accumulators of C and C^-1 (two each)
+constexpr int kKrBlocksWide = 12;  // Z .. Z^7, scratch and the accumulators: Horner steps of Z^8
+
+__host__ __device__ constexpr int kr_ld(int l) { return (l + 15) / 16 * 16 + 4; }
+__host__ __device__ constexpr int kr_rows(int l, int cs) { return 8 * (((l + 7) / 8 + cs - 1) / cs); }
+__host__ __device__ constexpr size_t kr_bytes(int l, int cs, int blocks) {
+  return ((size_t)((l + 7) / 8 * 8) * kr_ld(l) + (size_t)blocks * kr_rows(l, cs) * kr_ld(l)) * sizeof(double);
+}
+
+struct Kr {
+  int l, lr, l4, ld, rb, r0, cs, rank, mt, nt;  // mt x nt: 8 x 8 tiles of this CTA's rows
+  double *full, *blk;
+  __device__ double *block(int i) const { return blk + (size_t)i * rb * ld; }
+};
+
+// One 8 x 8 tile of rows (A) times the whole operand's columns (B), two accumulation chains.
+__device__ __forceinline__ void kr_tile(const Kr &k, const double *A, const double *B, double (&d)[2]) {
+  const int lane = threadIdx.x & 31;
+  const double *ap = A + (lane >> 2) * k.ld + (lane & 3);
+  const double *bp = B + (lane & 3) * k.ld + (lane >> 2);
+  const int sb = 4 * k.ld;
+  double e[2] = {0.0, 0.0};
+  d[0] = d[1] = 0.0;
+  int kk = 0;
+#pragma unroll 4
+  for (; kk + 8 <= k.l4; kk += 8, ap += 8, bp += 2 * sb) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(ap[0]), "d"(bp[0]));
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(e[0]), "+d"(e[1])
+                 : "d"(ap[4]), "d"(bp[sb]));
+  }
+  if (kk < k.l4)
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(ap[0]), "d"(bp[0]));
+  d[0] += e[0];
+  d[1] += e[1];
+}
+
+// epi(i, j, v) for the entries (local row i < 8 mt, column j < lr) of A (row block, or the rows of
+// `full` at r0) times `full`.
+template <class Epi>
+__device__ __forceinline__ void kr_mm(const Kr &k, const double *A, Epi epi) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int t = warp; t < k.mt * k.nt; t += kKrWarps) {
+    const int m0 = (t / k.nt) * 8, n0 = (t % k.nt) * 8;
+    double d[2];
+    kr_tile(k, A + (size_t)m0 * k.ld, k.full + n0, d);
+    epi(m0 + (lane >> 2), n0 + 2 * (lane & 3), d[0]);
+    epi(m0 + (lane >> 2), n0 + 2 * (lane & 3) + 1, d[1]);
+  }
+}
+
+// Whole l x l matrix (written by every CTA of the cluster, so read through L2) into `full`.
+__device__ __forceinline__ void kr_load(const Kr &k, const double *src) {
+  const int l = k.l;
+  if ((l & 1) == 0) {
+    const int l2 = l >> 1, total = l * l2;
+    for (int e0 = threadIdx.x; e0 < total; e0 += 8 * kKrThreads) {
+      double2 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int e = e0 + u * kKrThreads;
+        if (e < total) v[u] = __ldcg((const double2 *)src + e);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int e = e0 + u * kKrThreads;
+        if (e < total) {
+          const int i = e / l2, j = 2 * (e - i * l2);
+          *(double2 *)(k.full + (size_t)i * k.ld + j) = v[u];
+        }
+      }
+    }
+  } else {
+    for (int e = threadIdx.x; e < l * l; e += kKrThreads) {
+      const int i = e / l, j = e - i * l;
+      k.full[(size_t)i * k.ld + j] = __ldcg(src + e);
+    }
+  }
+}
+
+// The symmetric completion of the upper triangle of src (as syev 'U' reads Z) into `full`; returns
+// this thread's part of the sum of its squares.
+__device__ __forceinline__ double kr_load_sym(const Kr &k, const double *src) {
+  const int l = k.l, total = l * l;
+  double f = 0.0;
+  for (int e0 = threadIdx.x; e0 < total; e0 += 8 * kKrThreads) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * kKrThreads;
+      v[u] = e < total ? __ldcg(src + e) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * kKrThreads;
+      const int i = e / l, j = e - i * l;
+      if (e < total && i <= j) {
+        k.full[(size_t)i * k.ld + j] = v[u];
+        if (i != j) k.full[(size_t)j * k.ld + i] = v[u];
+        f += (i == j ? 1.0 : 2.0) * v[u] * v[u];
+      }
+    }
+  }
+  return f;
+}
+
+__device__ __forceinline__ double kr_block_sum(double v, double *red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = red[0];
+#pragma unroll
+  for (int i = 1; i < kKrWarps; ++i) s += red[i];
+  return s;
+}
+
+// Sum over the cluster of the CTAs' values, the same in every CTA; everything that the CTAs wrote
+// to global memory before it is visible to all after it.
+__device__ __forceinline__ double kr_cluster_sum(const Kr &k, cg::cluster_group &cluster, double v, double *slots,
+                                                 double *red) {
+  v = kr_block_sum(v, red);
+  if (threadIdx.x == 0) slots[k.rank] = v;
+  cluster.sync();
+  double s = 0.0;
+  for (int r = 0; r < k.cs; ++r) s += __ldcg(slots + r);
+  return s;
+}
+
+// Degree of the series: at most kKrChain by the chain of powers Z^t = Z^(t-1) Z, each added to both
+// sums as it comes (one product per degree, no exchange); above it by Horner steps in Z^4 (two
+// products per four degrees after one exchange), above kKrSb8 in Z^8 where the blocks fit.  With
+// rho >= ||4 Z||_2 from the Frobenius norm of Z above kKrRefine degrees, the norm of Z^4 gives the
+// sharper rho = 4 ||Z^4||_F^(1/4) (Z is positive semidefinite), which cuts most degrees in half.
+constexpr int kKrRefine = 7, kKrChain = 11, kKrSb8 = 31;
+
+__device__ __forceinline__ void kn_rows_body(const KnStep &a, const KnSeries &ser, int blocks) {
+  extern __shared__ double sm[];
+  __shared__ double red[kKrWarps];
+  __shared__ int plan[2];  // degree (-1: Newton-Schulz), Newton-Schulz steps
+  cg::cluster_group cluster = cg::this_cluster();
+  const int l = a.l, tid = threadIdx.x;
+  const size_t ll = (size_t)l * l;
+  Kr k;
+  k.l = l; k.lr = (l + 7) & ~7; k.l4 = (l + 3) & ~3; k.ld = kr_ld(l);
+  k.cs = (int)cluster.num_blocks(); k.rank = (int)cluster.block_rank();
+  k.rb = kr_rows(l, k.cs); k.r0 = k.rank * k.rb;
+  k.mt = max(0, min(k.rb, k.lr - k.r0)) / 8; k.nt = k.lr / 8;
+  k.full = sm; k.blk = sm + (size_t)k.lr * k.ld;
+  const int ld = k.ld, r0 = k.r0, rows = 8 * k.mt;
+  const bool wide = blocks >= kKrBlocksWide;
+  // block 0: scratch; blocks 1 .. 3 (wide: 1 .. 7): powers of Z
+  double *acc = k.block(blocks - 4), *acc2 = k.block(blocks - 2);  // C rows, then C^-1 rows
+  const size_t accn = (size_t)k.rb * ld;
+  // global: Z | Z^4 | Z^8 | Newton-Schulz Y, Q (two each); partial sums of the cluster reductions
+  double *Zg = a.work, *P4g = Zg + ll, *P8g = P4g + ll, *NSg = P8g + ll;
+  double *slots = a.work + (size_t)kKnWorkMatrices * ll;
+
+  // entries of this CTA's rows: f(local row, column, row, column valid)
+  auto each = [&](auto f) {
+    for (int e = tid; e < rows * k.lr; e += kKrThreads) {
+      const int i = e / k.lr, j = e - i * k.lr;
+      f(i, j, r0 + i < l && j < l);
+    }
+  };
+  auto publish = [&](const double *blkp, double *dst) {
+    each([&](int i, int j, bool in) {
+      if (in) dst[(size_t)(r0 + i) * l + j] = blkp[(size_t)i * ld + j];
+    });
+  };
+
+  for (int e = tid; e < k.lr * ld; e += kKrThreads) k.full[e] = 0.0;
+  __syncthreads();
+  kr_load(k, a.Dc);
+  __syncthreads();
+  // Z = Dgc - Dc Dc (:184-190)
+  kr_mm(k, k.full + (size_t)r0 * ld, [&](int i, int j, double v) {
+    if (r0 + i < l && j < l) {
+      const size_t e = (size_t)(r0 + i) * l + j;
+      Zg[e] = __ldcg(a.Dgc + e) - v;
+    }
+  });
+  cluster.sync();
+  const double f1 = kr_load_sym(k, Zg);
+  double rho = 4.0 * sqrt(kr_block_sum(f1, red));  // ||4 Z||_F >= ||4 Z||_2; also: `full` is complete
+  auto decide = [&](double r) {
+    __syncthreads();
+    if (tid < 32) {
+      const int d = ks_degree_warp<kSeriesLen / 32>(ser, r, a.ns_target);
+      if (tid == 0) {
+        plan[0] = d;
+        plan[1] = d < 0 ? kn_ns_steps(r, a.ns_target) : 0;
+      }
+    }
+    __syncthreads();
+    return plan[0];
+  };
+  int deg = decide(rho);
+  double *P1 = k.block(1);
+  each([&](int i, int j, bool) { P1[(size_t)i * ld + j] = k.full[(size_t)(r0 + i) * ld + j]; });
+  __syncthreads();
+  int have = 1;  // powers of Z in blocks
+  if (deg < 0 || deg > kKrRefine) {
+    // Z^2, Z^3 in blocks 2 and 3, Z^4 in the scratch block
+    double n4 = 0.0;
+    for (int t = 2; t <= 4; ++t) {
+      double *dst = k.block(t & 3);
+      kr_mm(k, k.block(t - 1), [&](int i, int j, double v) {
+        dst[(size_t)i * ld + j] = v;
+        if (t == 4) {
+          n4 += v * v;
+          if (r0 + i < l && j < l) P4g[(size_t)(r0 + i) * l + j] = v;
+        }
+      });
+      __syncthreads();
+    }
+    const double s4 = kr_cluster_sum(k, cluster, n4, slots, red);
+    rho = fmin(rho, 4.0 * sqrt(sqrt(sqrt(s4))));
+    deg = decide(rho);
+    have = 4;
+  }
+  const double *C, *Ci;
+  if (deg >= 0 && deg <= kKrChain) {
+    const int h = min(have, deg);
+    each([&](int i, int j, bool in) {
+      const double dg = (in && r0 + i == j) ? 1.0 : 0.0;
+      double vc = ser.c[0] * dg, vd = ser.d[0] * dg;
+      for (int t = 1; t <= h; ++t) {
+        const double p = k.block(t & 3)[(size_t)i * ld + j];
+        vc += ser.c[t] * p;
+        vd += ser.d[t] * p;
+      }
+      acc[(size_t)i * ld + j] = vc;
+      acc[accn + (size_t)i * ld + j] = vd;
+    });
+    __syncthreads();
+    for (int t = have + 1; t <= deg; ++t) {  // each thread adds to the entries of its own tiles
+      double *dst = k.block(t & 3);
+      const double ct = ser.c[t], dt = ser.d[t];
+      kr_mm(k, k.block((t - 1) & 3), [&](int i, int j, double v) {
+        const size_t e = (size_t)i * ld + j;
+        dst[e] = v;
+        acc[e] += ct * v;
+        acc[accn + e] += dt * v;
+      });
+      __syncthreads();
+    }
+    C = acc;
+    Ci = acc + accn;
+  } else if (deg >= 0) {
+    // Paterson-Stockmeyer: B_b = sum_{t<sb} coef[b sb + t] Z^t (b = 0..q); acc = B_q; acc = acc Z^sb + B_b
+    kr_load(k, P4g);
+    __syncthreads();
+    int sb = 4;
+    if (wide && deg > kKrSb8) {
+      // Z^5, Z^6, Z^7 in their blocks (Z^4 moves to block 4 first), Z^8 published
+      double *P4 = k.block(4);
+      each([&](int i, int j, bool) { P4[(size_t)i * ld + j] = k.block(0)[(size_t)i * ld + j]; });
+      __syncthreads();
+      for (int t = 5; t <= 8; ++t) {
+        double *dst = k.block(t & 7);
+        kr_mm(k, k.block(t - 4), [&](int i, int j, double v) {
+          dst[(size_t)i * ld + j] = v;
+          if (t == 8 && r0 + i < l && j < l) P8g[(size_t)(r0 + i) * l + j] = v;
+        });
+      }
+      cluster.sync();
+      kr_load(k, P8g);
+      __syncthreads();
+      sb = 8;
+    }
+    const int q = deg / sb;
+    auto coef_block = [&](int b, int i, int j, double &vc, double &vd) {
+      const double dg = (r0 + i == j && j < l) ? 1.0 : 0.0;
+      vc = ser.c[b * sb] * dg;
+      vd = ser.d[b * sb] * dg;
+      for (int t = 1; t < sb && b * sb + t <= deg; ++t) {
+        const double p = k.block(t)[(size_t)i * ld + j];
+        vc += ser.c[b * sb + t] * p;
+        vd += ser.d[b * sb + t] * p;
+      }
+    };
+    each([&](int i, int j, bool) {
+      double vc, vd;
+      coef_block(q, i, j, vc, vd);
+      acc[(size_t)i * ld + j] = vc;
+      acc[accn + (size_t)i * ld + j] = vd;
+    });
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31;
+    for (int b = q - 1; b >= 0; --b) {
+      // both sums at once: tiles of the C rows, then of the C^-1 rows
+      for (int t = warp; t < 2 * k.mt * k.nt; t += kKrWarps) {
+        const int inv = t >= k.mt * k.nt, tt = t - inv * k.mt * k.nt;
+        const int m0 = (tt / k.nt) * 8, n0 = (tt % k.nt) * 8;
+        double d[2];
+        kr_tile(k, acc + inv * accn + (size_t)m0 * ld, k.full + n0, d);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = m0 + (lane >> 2), j = n0 + 2 * (lane & 3) + u;
+          double vc, vd;
+          coef_block(b, i, j, vc, vd);
+          acc2[inv * accn + (size_t)i * ld + j] = d[u] + (inv ? vd : vc);
+        }
+      }
+      __syncthreads();
+      double *t1 = acc; acc = acc2; acc2 = t1;
+    }
+    C = acc;
+    Ci = acc + accn;
+  } else {
+    // Two coupled Newton-Schulz square roots (Higham, Functions of Matrices, eq. 6.35):
+    //   Y <- (3 I - Y Q) Y / 2,  Q <- (3 I - Q Y) Q / 2   ->  Y -> X^(1/2), Q -> X^(-1/2),
+    // first of X = I - 4 Z (sqrt(I/4 - Z) = Y/2), then of P = I/2 + Y/2.  Both iterates are exchanged
+    // once per step (two global buffers in turn); S = Y Q and T = Q Y are local rows.
+    double *Y = acc, *Q = acc + accn, *S = k.block(2), *T = k.block(3);
+    each([&](int i, int j, bool in) {
+      const double dg = (in && r0 + i == j) ? 1.0 : 0.0;
+      Y[(size_t)i * ld + j] = dg - 4.0 * P1[(size_t)i * ld + j];
+      Q[(size_t)i * ld + j] = dg;
+    });
+    __syncthreads();
+    int steps = plan[1], par = 0;
+    for (int stage = 0; stage < 2; ++stage) {
+      for (int it = 0; it < steps; ++it, par ^= 1) {
+        double *Yg = NSg + 2 * par * ll, *Qg = Yg + ll;
+        publish(Y, Yg);
+        publish(Q, Qg);
+        cluster.sync();
+        kr_load(k, Qg);
+        __syncthreads();
+        kr_mm(k, Y, [&](int i, int j, double v) { S[(size_t)i * ld + j] = v; });
+        __syncthreads();
+        kr_load(k, Yg);
+        __syncthreads();
+        kr_mm(k, Q, [&](int i, int j, double v) { T[(size_t)i * ld + j] = v; });
+        kr_mm(k, S, [&](int i, int j, double v) {
+          const size_t e = (size_t)i * ld + j;
+          Y[e] = 1.5 * Y[e] - 0.5 * v;
+        });
+        __syncthreads();
+        kr_load(k, Qg);
+        __syncthreads();
+        kr_mm(k, T, [&](int i, int j, double v) {
+          const size_t e = (size_t)i * ld + j;
+          Q[e] = 1.5 * Q[e] - 0.5 * v;
+        });
+        __syncthreads();
+      }
+      if (stage == 0) {
+        double d2 = 0.0;
+        each([&](int i, int j, bool in) {
+          const size_t e = (size_t)i * ld + j;
+          const double dg = (in && r0 + i == j) ? 1.0 : 0.0;
+          const double pv = 0.5 * Y[e] + 0.5 * dg;
+          Y[e] = pv;
+          Q[e] = dg;
+          d2 += (dg - pv) * (dg - pv);
+        });
+        steps = kn_ns_steps(fmin(sqrt(kr_cluster_sum(k, cluster, d2, slots + 16, red)), 0.5), a.ns_target);
+      }
+    }
+    C = Y;
+    Ci = Q;
+  }
+  // C, C^-1, F = C - Dc C^-1 (:218) and the stacked copies, err = ||C - I||_F (:230-234).  C, C^-1 and
+  // Dc are symmetric: the rows of F' = C - C^-1 Dc are the columns of F.
+  kr_load(k, a.Dc);
+  double e2 = 0.0;
+  each([&](int i, int j, bool in) {
+    if (!in) return;
+    const size_t e = (size_t)(r0 + i) * l + j;
+    const double cv = C[(size_t)i * ld + j], ci = Ci[(size_t)i * ld + j];
+    a.C[e] = cv;
+    a.Cinv[e] = ci;
+    if (a.fstack) {
+      a.fstack[ll + e] = a.fstack_scale * ci;
+      a.fstack[3 * ll + e] = ci;
+    }
+    const double d = cv - (r0 + i == j ? 1.0 : 0.0);
+    e2 += d * d;
+  });
+  __syncthreads();
+  kr_mm(k, Ci, [&](int i, int j, double v) {
+    if (r0 + i < l && j < l) {
+      const size_t e = (size_t)j * l + r0 + i;
+      const double fv = C[(size_t)i * ld + j] - v;
+      a.F[e] = fv;
+      if (a.fstack) {
+        a.fstack[e] = fv;
+        a.fstack[2 * ll + e] = fv;
+      }
+    }
+  });
+  const double err = sqrt(kr_cluster_sum(k, cluster, e2, slots + 32, red));
+  if (k.rank == 0 && tid == 0) {
+    *a.err = err;
+    if (!(err == err)) atomicExch(a.status, kErrNumerical);
+  }
+}
+
+__global__ void __launch_bounds__(kKrThreads, 1) kn_rows_kernel(KnStep a, KnSeries ser, int blocks) {
+  kn_rows_body(a, ser, blocks);
+}
 
 // One cluster per step of steps[] (grid = count x cluster size): many independent problems.
-// full: one-CTA clusters with the whole-operand product layout (every l <= kKsFullL).
-__global__ void __launch_bounds__(kKsThreads, 1) kn_cluster_grouped_kernel(const KnStep *steps, KnSeries ser,
-                                                                         int full) {
+__global__ void __launch_bounds__(kKrThreads, 1) kn_rows_grouped_kernel(const KnStep *steps, KnSeries ser, int blocks) {
   const KnStep a = steps[blockIdx.x / cg::this_cluster().num_blocks()];
-  kn_cluster_body(a, ser, full != 0);
+  kn_rows_body(a, ser, blocks);
 }
 
 // Coefficients of g(z)^(1/2) and g(z)^(-1/2), g(z) = 1 - sum_{n>=1} Cat(n-1) z^n: for h = f^alpha
@@ -461,28 +833,32 @@ int choose_cluster_size(const KnStep &a, cudaStream_t st) {
 
 }  // namespace
 
-void kn_step_grouped(const KnStep *steps, int count, int max_l, int cluster, cudaStream_t st) {
-  if (count <= 0) return;
-  if (max_l > kKsMaxL) fail(kErrUnsupported, "Kolmogorov-Nagumo step: l = %d > %d", max_l, kKsMaxL);
-  KnStep probe;
-  probe.l = max_l;
-  int cs = choose_cluster_size(probe, st);
-  if (cs == 0) fail(kErrUnsupported, "grouped Kolmogorov-Nagumo step: no thread-block cluster launch on this device");
-  const size_t smem_max = std::max(kKsSmem, ks_full_smem(kKsFullL));
-  static bool attr = false;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(kn_cluster_grouped_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(kn_cluster_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-    attr = true;
-  }
-  // many clusters run side by side: `cluster` CTAs each (default eight)
-  cs = std::min(cs, cluster > 0 ? cluster : 8);
-  const int full = (cs == 1 && max_l <= kKsFullL) ? 1 : 0;
-  static const KnSeries series = make_series();
+namespace {
+
+int kr_blocks(int l, int cs) {
+  const size_t cap = Runtime::get().smem_optin - 1024;
+  if (kr_bytes(l, cs, kKrBlocksWide) <= cap) return kKrBlocksWide;
+  return kr_bytes(l, cs, kKrBlocks) <= cap ? kKrBlocks : 0;
+}
+
+// Cluster size of a row-cut step: one CTA per eight rows (a power of two, at most `want`, at least
+// what the shared memory needs), or 0 when there is none.
+int kr_cluster(int l, int want) {
+  if (l > kKrMaxL) return 0;
+  int cs = 1;
+  while (cs < want && kr_rows(l, cs) > 8) cs *= 2;
+  while (cs < 16 && kr_blocks(l, cs) == 0) cs *= 2;
+  return kr_blocks(l, cs) ? cs : 0;
+}
+
+template <class Kern, class Arg>
+void kr_launch(Kern kern, int cs, int grid, int l, cudaStream_t st, Arg a, const KnSeries &series) {
+  const int blocks = kr_blocks(l, cs);
+  const int bytes = (int)kr_bytes(l, cs, blocks);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(count * cs);
-  cfg.blockDim = dim3(kKsThreads);
-  cfg.dynamicSmemBytes = full ? std::max(kKsSmem, ks_full_smem(max_l)) : kKsSmem;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kKrThreads);
+  cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -491,19 +867,63 @@ void kn_step_grouped(const KnStep *steps, int count, int max_l, int cluster, cud
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  CK(cudaLaunchKernelEx(&cfg, kn_cluster_grouped_kernel, steps, series, full));
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  CK(cudaLaunchKernelEx(&cfg, kern, a, series, blocks));
   KLAUNCHED();
+}
+
+// Whether the device can run a 16-CTA cluster of the row-cut step at its largest shared memory.
+bool kr_usable() {
+  static const bool ok = [] {
+    const size_t bytes = kr_bytes(kKrMaxL, 16, kr_blocks(kKrMaxL, 16));
+    CK(cudaFuncSetAttribute(kn_rows_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    CK(cudaFuncSetAttribute(kn_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(kKrThreads);
+    cfg.dynamicSmemBytes = bytes;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 16;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kn_rows_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return n >= 1;
+  }();
+  return ok;
+}
+
+}  // namespace
+
+void kn_step_grouped(const KnStep *steps, int count, int max_l, int cluster, cudaStream_t st) {
+  if (count <= 0) return;
+  if (max_l > kKrMaxL) fail(kErrUnsupported, "grouped Kolmogorov-Nagumo step: l = %d > %d", max_l, kKrMaxL);
+  const int cs = kr_usable() ? kr_cluster(max_l, cluster > 0 ? cluster : 8) : 0;
+  if (cs == 0) fail(kErrUnsupported, "grouped Kolmogorov-Nagumo step: no thread-block cluster launch on this device");
+  static const KnSeries series = make_series();
+  kr_launch(kn_rows_grouped_kernel, cs, count * cs, max_l, st, steps, series);
 }
 
 void kn_step(const KnStep &a, cudaStream_t st) {
   if (a.l > kKsMaxL) fail(kErrUnsupported, "Kolmogorov-Nagumo step: l = %d > %d", a.l, kKsMaxL);
+  static const KnSeries series = make_series();
+  if (const int rc = kr_usable() ? kr_cluster(a.l, 16) : 0) {
+    kr_launch(kn_rows_kernel, rc, rc, a.l, st, a, series);
+    return;
+  }
   const int cs = choose_cluster_size(a, st);
   if (cs == 0) {  // no cluster launch on this device: the grid-barrier kernel (work 8 l^2 + 64 fits)
     CK(cudaMemsetAsync(a.bar, 0, 8, st));  // its barrier counters
     kn_step_fixed(a, Runtime::get().num_sms, st);
     return;
   }
-  static const KnSeries series = make_series();
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs);
   cfg.blockDim = dim3(kKsThreads);

@@ -134,15 +134,14 @@ struct KnStep {
   double fstack_scale = 1.0;
 };
 constexpr int kKnWorkMatrices = 29;
-constexpr int kSeriesLen = 64;
+constexpr int kSeriesLen = 128;
 struct KnSeries {  // power-series coefficients of C(Z) and C(Z)^-1 (k_small.cu)
   double c[kSeriesLen], d[kSeriesLen];
 };
 void kn_step(const KnStep &a, cudaStream_t st);
 // count independent steps (steps in device memory, each with its own buffers; max_l >= every l),
-// one thread-block cluster of `cluster` CTAs per step (<= 0: eight; at most what the device
-// allows).  A step's 32 x 32 product tiles are spread over its cluster: ceil(l / 32)^2 CTAs keep
-// every CTA busy.
+// one thread-block cluster per step of at most `cluster` CTAs (raised to the smallest cluster whose
+// shared memory holds a step of size max_l); max_l <= 128.
 void kn_step_grouped(const KnStep *steps, int count, int max_l, int cluster, cudaStream_t st);
 
 // ---------------------------------------------------------------- k_chol.cu

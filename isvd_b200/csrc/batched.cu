@@ -505,7 +505,7 @@ void build_lists(Plan<T> &P, cudaStream_t st) {
     P.qbar_l.host.push_back(prod(m, l, Nl, M.qs.p, Nl, 1, M.mt.p, l, 1, M.qbar.p, l, 1));
     P.proj.host.push_back(prod(n, l, m, P.a[b], 1, P.lda[b], M.qbar.p, l, 1, M.z.p, l, 1));
     P.wzl.host.push_back(prod(l, l, n, M.z.p, 1, l, M.z.p, l, 1, M.wz.p, l, 1));
-    e2.push_back(EigDesc{l, M.wz.p, M.vz.p, M.lz.p});
+    e2.push_back(EigDesc{l, M.wz.p, M.vz.p, M.lz.p, M.work.p});  // the KN step's work, free by then
     P.m_s.host.push_back(gm(M.lz.p, 1, 0, P.s[b], 1, 0, l, 1, kMapSqrt));
     P.m_wk.host.push_back(gm(M.vz.p, l, 1, M.wk.p, k, 1, l, k, kMapCopy));
     P.m_vk.host.push_back(gm(M.vz.p, l, 1, M.vk.p, k, 1, l, k, kMapInvSqrt, M.lz.p));

@@ -71,10 +71,14 @@ constexpr int eig_max_mine(int nt) {
 template <bool VS, int NT = kEigThreads>
 __global__ void __launch_bounds__(NT)
     sym_eig_kernel(int n_uniform, const double *__restrict__ Ag, double *__restrict__ Vg, double *__restrict__ wg,
-                   int order, bool absval, double *__restrict__ scratch, int *status, const EigDesc *desc) {
+                   int order, bool absval, double *__restrict__ scratch, int *status, const EigDesc *desc,
+                   const double *refined, size_t refined_stride) {
   extern __shared__ double sm[];
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int n = desc ? desc[b].n : n_uniform;
+  // after eig_refined: only the matrices it did not settle
+  const double *rw = desc ? desc[b].work : refined ? refined + (size_t)b * refined_stride : nullptr;
+  if (rw && !*(const int *)(rw + eig_need_at(n))) return;
   const double *A0 = desc ? desc[b].A : Ag + (size_t)b * n * n;
   double *V = desc ? desc[b].V : Vg + (size_t)b * n * n;
   double *w = desc ? desc[b].w : wg + (size_t)b * n;
@@ -821,26 +825,24 @@ size_t svd_smem(int n) { return (size_t)n * n * 8 + (size_t)n * 8 + 16; }
 
 namespace {
 
-// Cluster size for the one-matrix eigensolver (0: use the one-CTA kernel): the largest of 16, 8,
-// 4, 2 that the device can co-schedule, for 112 <= n <= 160.  A round costs about 2.5 us on the
-// cluster whatever n (barrier and exchange), against shared-memory bandwidth on one CTA, which
-// grows as n^2: measured per solve on B200, 3.45 against 4.18 ms at n = 128 and 5.7 against
-// 10.8 ms at n = 160, but 2.49 against 2.19 ms at n = 96.
+// Cluster size for the one-matrix eigensolver of 128 < n <= 160 (0: use the one-CTA kernel): the
+// largest of 16, 8, 4, 2 that the device can co-schedule.  A round costs about 2.5 us on the cluster
+// whatever n (barrier and exchange), against shared-memory bandwidth on one CTA, which grows as n^2:
+// measured per solve on B200, 5.7 against 10.8 ms at n = 160.  (n <= 128: eig_refined.)
 int eig_cluster_size(int n, cudaStream_t st) {
-  static int decided[2] = {-1, -1};  // per size class: n <= 128, n <= 160
-  if (n < 112 || n > 160) return 0;
+  static int d = -1;
+  if (n <= 128 || n > 160) return 0;
   // ISVD_GPU_EIG_CLUSTER: 0 off, 2..16 the largest size tried
   static const int top = [] {
     const char *e = getenv("ISVD_GPU_EIG_CLUSTER");
     return e ? std::max(0, std::min(16, atoi(e))) : 16;
   }();
   if (top < 2) return 0;
-  int &d = decided[n > 128 ? 1 : 0];
   if (d >= 0) return d;
   CK(cudaFuncSetAttribute(sym_eig_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   d = 0;
   for (int cs = top; cs >= 2; cs /= 2) {
-    const size_t smem = eig_cluster_smem(n > 128 ? 160 : 128, cs);
+    const size_t smem = eig_cluster_smem(160, cs);
     if (cudaFuncSetAttribute(sym_eig_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess) {
       cudaGetLastError();
@@ -900,7 +902,12 @@ void sym_eig_batched(int n, int batch, const double *A, double *V, double *w, in
   if (n <= 0 || batch <= 0) return;
   ProfileScope prof("sym_eig", st);
   Runtime &rt = Runtime::get();
-  if (batch == 1) {
+  DBuf<double> work;
+  const size_t stride = eig_work_doubles(n);
+  if (eig_refined_usable(n)) {
+    work.alloc(batch * stride);
+    eig_refined(n, batch, A, work.p, V, w, order, absval, nullptr, st);
+  } else if (batch == 1) {
     const int cs = eig_cluster_size(n, st);
     if (cs > 0) {
       const size_t smem = eig_cluster_smem(n, cs);
@@ -925,7 +932,8 @@ void sym_eig_batched(int n, int batch, const double *A, double *V, double *w, in
   const size_t smem_vs = eig_smem(n, true);
   if (smem_vs <= rt.smem_optin) {
     CK(cudaFuncSetAttribute(sym_eig_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_vs));
-    sym_eig_kernel<true><<<batch, kEigThreads, smem_vs, st>>>(n, A, V, w, order, absval, nullptr, status, nullptr);
+    sym_eig_kernel<true><<<batch, kEigThreads, smem_vs, st>>>(n, A, V, w, order, absval, nullptr, status, nullptr,
+                                                              work.p, stride);
     KLAUNCHED();
     return;
   }
@@ -934,7 +942,7 @@ void sym_eig_batched(int n, int batch, const double *A, double *V, double *w, in
   DBuf<double> scratch((size_t)batch * n * n);
   CK(cudaFuncSetAttribute(sym_eig_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   sym_eig_kernel<false><<<batch, kEigThreads, smem, st>>>(n, A, V, w, order, absval, scratch.p, status,
-                                                            nullptr);
+                                                            nullptr, work.p, stride);
   KLAUNCHED();
 }
 
@@ -944,10 +952,12 @@ void sym_eig_grouped(const EigDesc *desc, int count, int max_n, int order, bool 
   const size_t smem = eig_smem(max_n, true);
   if (smem > Runtime::get().smem_optin)
     fail(kErrUnsupported, "symmetric eigensolver: l = %d exceeds on-chip capacity", max_n);
-  // the smallest CTA that holds the largest matrix: small matrices leave room for many CTAs per SM
+  if (!eig_refined_usable(max_n)) fail(kErrUnsupported, "grouped eigensolver: no thread-block cluster launch");
+  eig_refined(max_n, count, nullptr, nullptr, nullptr, nullptr, order, absval, desc, st);
+  // the matrices that did not settle; the smallest CTA that holds the largest matrix: small matrices leave room for many CTAs per SM
   auto go = [&](auto kernel, int nt) {
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<count, nt, smem, st>>>(0, nullptr, nullptr, nullptr, order, absval, nullptr, status, desc);
+    kernel<<<count, nt, smem, st>>>(0, nullptr, nullptr, nullptr, order, absval, nullptr, status, desc, nullptr, 0);
     KLAUNCHED();
   };
   if (max_n <= eig_max_n(128)) go(sym_eig_kernel<true, 128>, 128);

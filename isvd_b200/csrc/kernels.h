@@ -98,7 +98,8 @@ void scale_cols_batched(const Ts *src, long long lds, Td *dst, long long ldd, lo
                         long long rows_per_batch, const double *s, int mode, cudaStream_t st);
 
 // ------------------------------------------------------------------ small dense FP64 (l x l)
-// Batched symmetric eigendecomposition by parallel cyclic Jacobi, one CTA per matrix.
+// Batched symmetric eigendecomposition: eig_refined for n <= 128, parallel cyclic two-sided Jacobi
+// (one CTA per matrix) for larger n and for the matrices that eig_refined does not settle.
 // A: batch x (n x n) row-major (only read), V: batch x (n x n) row-major eigenvectors (columns),
 // w: batch x n eigenvalues.  order > 0: sort by |lambda| descending (gesvd of a PSD matrix);
 // order < 0: ascending lambda (syev).  absval: return |lambda| in w.
@@ -106,7 +107,16 @@ struct EigDesc {  // one matrix of a grouped eigensolve: n x n row-major A -> V 
   int n;
   const double *A;
   double *V, *w;
+  double *work;  // eig_work_doubles(n) doubles
 };
+// FP32 Jacobi with FP64 refinement (k_eig.cu) of count matrices, n <= 128 (desc: of sizes up to n, each
+// with its own buffers; else count x n x n with `work` of count x eig_work_doubles(n)).  A matrix it
+// does not settle has the int at work + eig_need_at(n) set, its V and w unwritten.
+size_t eig_work_doubles(int n);
+__host__ __device__ constexpr size_t eig_need_at(int n) { return 4 * (size_t)n * n + n + 49; }
+bool eig_refined_usable(int n);
+void eig_refined(int n, int count, const double *A, double *work, double *V, double *w, int order, bool absval,
+                 const EigDesc *desc, cudaStream_t st);
 // As sym_eig_batched for count matrices of different sizes (desc in device memory; max_n >= every n).
 void sym_eig_grouped(const EigDesc *desc, int count, int max_n, int order, bool absval, int *status,
                      cudaStream_t st);

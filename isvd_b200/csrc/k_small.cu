@@ -227,10 +227,17 @@ __global__ void __launch_bounds__(NT)
 }
 
 // One-sided Jacobi SVD: B (row-major n x n) -> U diag(s) V'.
-// Columns of B are held column-major in shared memory; V in global memory (this CTA only).
-__global__ void __launch_bounds__(kEigThreads)
+// Columns of B and of V are held column-major, B's in shared memory, V's too when both fit (VS), else in
+// global scratch.  Sixteen lanes per column pair (their 8-byte accesses are one 128-byte wavefront), EPL
+// elements of a column each, read once per round.  A round is bound by latency: the reduction, the
+// root-and-division chain of the rotation, the barrier; with V's columns strided in global memory (as the
+// output stores them) it was bound by those accesses instead: 1.8 ms against 0.4 ms for n = 48.
+constexpr int kSvdLanes = 16;
+
+template <bool VS, int EPL>
+__global__ void __launch_bounds__(1024)
     svd_jacobi_kernel(int n, const double *__restrict__ Bg, double *__restrict__ Ug, double *__restrict__ sg,
-                      double *__restrict__ Vg, int *status) {
+                      double *__restrict__ Vg, double *__restrict__ scratch, int *status) {
   extern __shared__ double sm[];
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
@@ -239,66 +246,77 @@ __global__ void __launch_bounds__(kEigThreads)
   double *V = Vg + (size_t)b * n * n;
   double *s = sg + (size_t)b * n;
   const int ne = n + (n & 1), np = ne / 2;
-  double *X = sm;                  // column-major: X[j * n + i] = B(i, j)
-  double *nrm = X + n * n;         // n
-  int *flag = (int *)(nrm + n);
+  double *X = sm;                                                       // X[j * n + i] = B(i, j)
+  double *Vt = VS ? X + (size_t)n * n : scratch + (size_t)b * n * n;    // Vt[j * n + i] = V(i, j)
+  double *nrm = X + (VS ? 2 : 1) * (size_t)n * n;                       // n
+  int *rnk = (int *)(nrm + n);                                          // n
 
-  __shared__ double red[kEigThreads];
+  __shared__ double red[32];
   double fr = 0.0;
   for (int e = tid; e < n * n; e += nt) {
     const int i = e / n, j = e - i * n;
-    X[j * n + i] = B0[e];
-    fr += B0[e] * B0[e];
-    V[e] = (i == j) ? 1.0 : 0.0;
+    const double v = B0[e];
+    X[j * n + i] = v;
+    fr += v * v;
+    Vt[e] = (i == j) ? 1.0 : 0.0;
   }
-  red[tid] = fr;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) fr += __shfl_xor_sync(0xffffffffu, fr, o);
+  if (lane == 0) red[warp] = fr;
   __syncthreads();
-  for (int h = nt / 2; h > 0; h >>= 1) {
-    if (tid < h) red[tid] += red[tid + h];
-    __syncthreads();
-  }
+  fr = 0.0;
+  for (int i = 0; i < nwarp; ++i) fr += red[i];
   const double tol = kEps * fmax(1.0, sqrt((double)n));
-  const double floor2 = kEps * kEps * red[0];  // ||B||_F^2 eps^2
-  __syncthreads();
+  const double floor2 = kEps * kEps * fr;  // ||B||_F^2 eps^2
+  const int grp = tid / kSvdLanes, sub = tid % kSvdLanes, ngrp = nt / kSvdLanes;
+  const int passes = (np + ngrp - 1) / ngrp;
   int sweep = 0;
   for (; sweep < kMaxSweeps; ++sweep) {
-    if (tid == 0) *flag = 0;
-    __syncthreads();
+    int rotated = 0;
     for (int r = 0; r < ne - 1; ++r) {
-      for (int k = warp; k < np; k += nwarp) {
-        int p = rr_player(k, r, ne), q = rr_player(ne - 1 - k, r, ne);
-        if (p > q) { const int t = p; p = q; q = t; }
-        if (q >= n) continue;
-        double al = 0.0, be = 0.0, ga = 0.0;
-        for (int i = lane; i < n; i += 32) {
-          const double xp = X[p * n + i], xq = X[q * n + i];
-          al += xp * xp; be += xq * xq; ga += xp * xq;
+      for (int w = 0; w < passes; ++w) {  // every lane runs every pass: the shuffles need whole warps
+        const int k = grp + w * ngrp;
+        int p = 0, q = n;
+        if (k < np) {
+          p = rr_player(k, r, ne);
+          q = rr_player(ne - 1 - k, r, ne);
+          if (p > q) { const int t = p; p = q; q = t; }
+        }
+        const bool live = q < n;
+        double xp[EPL], xq[EPL], al = 0.0, be = 0.0, ga = 0.0;
+#pragma unroll
+        for (int u = 0; u < EPL; ++u) {
+          const int i = sub + u * kSvdLanes;
+          xp[u] = live && i < n ? X[p * n + i] : 0.0;
+          xq[u] = live && i < n ? X[q * n + i] : 0.0;
+          al += xp[u] * xp[u]; be += xq[u] * xq[u]; ga += xp[u] * xq[u];
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int o = kSvdLanes / 2; o > 0; o >>= 1) {
           al += __shfl_xor_sync(0xffffffffu, al, o);
           be += __shfl_xor_sync(0xffffffffu, be, o);
           ga += __shfl_xor_sync(0xffffffffu, ga, o);
         }
-        if (fabs(ga) <= tol * fmax(sqrt(al * be), floor2)) continue;
-        if (lane == 0) *flag = 1;
-        const double zeta = (be - al) / (2.0 * ga);
-        const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-        const double c = 1.0 / sqrt(1.0 + t * t), sn = t * c;
-        for (int i = lane; i < n; i += 32) {
-          const double xp = X[p * n + i], xq = X[q * n + i];
-          X[p * n + i] = c * xp - sn * xq;
-          X[q * n + i] = sn * xp + c * xq;
-          const double vp = V[i * n + p], vq = V[i * n + q];
-          V[i * n + p] = c * vp - sn * vq;
-          V[i * n + q] = sn * vp + c * vq;
+        if (!live || fabs(ga) <= tol * fmax(sqrt(al * be), floor2)) continue;
+        rotated = 1;
+        // t = tan(theta), as in jacobi_rot
+        const double d = be - al, e = 2.0 * ga;
+        const double t = (d >= 0.0 ? e : -e) / (fabs(d) + sqrt(d * d + e * e));
+        const double c = rsqrt(1.0 + t * t), sn = t * c;
+#pragma unroll
+        for (int u = 0; u < EPL; ++u) {
+          const int i = sub + u * kSvdLanes;
+          if (i >= n) continue;
+          X[p * n + i] = c * xp[u] - sn * xq[u];
+          X[q * n + i] = sn * xp[u] + c * xq[u];
+          const double vp = Vt[p * n + i], vq = Vt[q * n + i];
+          Vt[p * n + i] = c * vp - sn * vq;
+          Vt[q * n + i] = sn * vp + c * vq;
         }
       }
       __syncthreads();
     }
-    const int f = *flag;
-    __syncthreads();
-    if (!f) break;
+    if (!__syncthreads_or(rotated)) break;
   }
   if (sweep == kMaxSweeps && tid == 0) atomicExch(status, kErrNumerical);
   for (int j = warp; j < n; j += nwarp) {
@@ -309,25 +327,21 @@ __global__ void __launch_bounds__(kEigThreads)
     if (lane == 0) nrm[j] = sqrt(a);
   }
   __syncthreads();
-  // sort by singular value descending; write U = X / s (row-major) and permuted V.
+  // sort by singular value descending; write U = X / s and V (row-major)
   for (int j = tid; j < n; j += nt) {
     const double sj = nrm[j];
     int rank = 0;
     for (int k = 0; k < n; ++k) rank += (nrm[k] > sj) || (nrm[k] == sj && k < j);
     s[rank] = sj;
-    const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-    for (int i = 0; i < n; ++i) U[i * n + rank] = X[j * n + i] * inv;
+    rnk[rank] = j;
   }
   __syncthreads();
-  // permute V columns through shared memory (X no longer needed)
-  for (int j = tid; j < n; j += nt) {
+  for (int e = tid; e < n * n; e += nt) {
+    const int i = e / n, j = rnk[e - i * n];
     const double sj = nrm[j];
-    int rank = 0;
-    for (int k = 0; k < n; ++k) rank += (nrm[k] > sj) || (nrm[k] == sj && k < j);
-    for (int i = 0; i < n; ++i) X[i * n + rank] = V[i * n + j];
+    U[e] = X[j * n + i] * (sj > 0.0 ? 1.0 / sj : 0.0);
+    V[e] = Vt[j * n + i];
   }
-  __syncthreads();
-  for (int e = tid; e < n * n; e += nt) V[e] = X[e];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -819,7 +833,7 @@ size_t eig_smem(int n, bool vs) {
   const size_t npk = ((size_t)n * (n + 1) / 2 + 1) & ~(size_t)1;
   return npk * 8 + (vs ? (size_t)n * n * 8 : 0) + (size_t)np * 16 + (size_t)n * 8 + (size_t)np * 8 + 16;
 }
-size_t svd_smem(int n) { return (size_t)n * n * 8 + (size_t)n * 8 + 16; }
+size_t svd_smem(int n, bool vs) { return (vs ? 2 : 1) * (size_t)n * n * 8 + (size_t)n * 12 + 16; }
 
 }  // namespace
 
@@ -970,11 +984,21 @@ void svd_jacobi_batched(int n, int batch, const double *B, double *U, double *s,
                         cudaStream_t st) {
   if (n <= 0 || batch <= 0) return;
   Runtime &rt = Runtime::get();
-  const size_t smem = svd_smem(n);
-  if (smem > rt.smem_optin) fail(kErrUnsupported, "Jacobi SVD: l = %d exceeds on-chip capacity", n);
-  CK(cudaFuncSetAttribute(svd_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  svd_jacobi_kernel<<<batch, kEigThreads, smem, st>>>(n, B, U, s, V, status);
-  KLAUNCHED();
+  const bool vs = svd_smem(n, true) + 1024 <= rt.smem_optin;
+  const size_t smem = svd_smem(n, vs);
+  if (smem + 1024 > rt.smem_optin) fail(kErrUnsupported, "Jacobi SVD: l = %d exceeds on-chip capacity", n);
+  const int threads = std::max(64, std::min(1024, ((n + 1) / 2 * kSvdLanes + 31) / 32 * 32));
+  DBuf<double> scratch;
+  if (!vs) scratch.alloc((size_t)batch * n * n);
+  auto go = [&](auto kernel) {
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<batch, threads, smem, st>>>(n, B, U, s, V, scratch.p, status);
+    KLAUNCHED();
+  };
+  if (!vs) go(svd_jacobi_kernel<false, 11>);
+  else if (n <= 32) go(svd_jacobi_kernel<true, 2>);
+  else if (n <= 64) go(svd_jacobi_kernel<true, 4>);
+  else go(svd_jacobi_kernel<true, 8>);
 }
 
 void kn_step_fixed_preload() {

@@ -32,7 +32,9 @@ const char *isvd_gpu_get_error_string( void );
 void isvd_gpu_clear_error( void );
 
 /* ---------------------------------------------------------------- precision */
-#define ISVD_GPU_PRECISION_NATIVE   0  /* products in the routine's own type (FP64 for isvd_d*, FP32 for isvd_s*) */
+#define ISVD_GPU_PRECISION_NATIVE   0  /* products in the routine's own type (FP64 for isvd_d*, FP32 for isvd_s*); large
+                                          FP32 products on tcgen05 from operands split exactly into three bf16
+                                          planes, with less rounding than an FP32 multiply-add chain */
 #define ISVD_GPU_PRECISION_MIXED    1  /* bf16 split products (2 or 3 planes per operand) on tcgen05 tensor
                                           cores, FP32 accumulation; l x l steps (eigensolves, inverse square
                                           roots, small SVDs) in FP64 */
@@ -154,7 +156,8 @@ void isvd_gpu_batch_destroy( isvd_gpu_batch *batch );
  * *iterations (may be NULL) receives the CG iterations used (both systems together).  Buffers may
  * be host or device memory.  In MIXED precision (isvd_gpu_set_precision) isvd_sSvdAdjoint runs the
  * products by A and A' on the tensor cores (A in two bf16 planes, the other operand in three);
- * NATIVE keeps them in FP32 on CUDA cores.  Returns an ISVD_GPU_* status. */
+ * NATIVE takes A in three planes, exact to FP32, or on CUDA cores when the products are too small for
+ * planes.  Returns an ISVD_GPU_* status. */
 int isvd_sSvdAdjoint(
     const isvd_int_t m, const isvd_int_t n, const isvd_int_t k, const char ordera,
     const isvd_s_val_t *a, const isvd_int_t lda, const isvd_s_val_t *s,

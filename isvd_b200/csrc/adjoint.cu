@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -194,7 +195,8 @@ void coldot(cudaStream_t st, const T *x, const T *y, long long rows, int k, doub
 }
 
 // Products by A (m x n, stored per ordera) and A' with k-column operands (contiguous).  MIXED with
-// FP32 operands: A's two bf16 planes (made once) on the tcgen05 engine; otherwise the strided GEMM.
+// FP32 operands: A's two bf16 planes (made once) on the tcgen05 engine; NATIVE FP32: A's three planes
+// (A itself, to its last bit) when the products are large enough for them; otherwise the strided GEMM.
 template <class T>
 struct AProducts {
   const StageCtx &c;
@@ -203,18 +205,27 @@ struct AProducts {
   const T *a;
   long long lda;
   bool mixed;
+  int np = 0;  // planes of A (0: strided GEMM)
   PlaneBuf ap;
   PlaneBuf xpn, xpm;  // the other operand's planes (n or m rows), kept across products
-  AProducts(const StageCtx &c_, int m_, int n_, char ordera_, const T *a_, long long lda_)
+  AProducts(const StageCtx &c_, int m_, int n_, int k, char ordera_, const T *a_, long long lda_)
       : c(c_), m(m_), n(n_), ordera(ordera_), a(a_), lda(lda_),
         mixed(c_.precision == kMixed && sizeof(T) == sizeof(float)) {
-    if (!mixed) return;
-    if (ordera == 'R') make_planes<T>(ap, a, lda, m, n, 2, false, c.st);  // m x n, n contiguous
-    else make_planes<T>(ap, a, lda, n, m, 2, true, c.st);
+    np = mixed ? 2 : 0;
+    if constexpr (std::is_same<T, float>::value)
+      if (!mixed && f32_operator_pays(m, n, k)) np = 3;
+    if (!np) return;
+    try {
+      if (ordera == 'R') make_planes<T>(ap, a, lda, m, n, np, false, c.st);  // m x n, n contiguous
+      else make_planes<T>(ap, a, lda, n, m, np, true, c.st);
+    } catch (const Error &e) {
+      if (mixed || e.code != kErrMemory) throw;
+      np = 0;
+    }
   }
   // Y = A X (m x k) or, transpose, A' X (n x k)
   void mul(bool transpose, int k, const T *X, T *Y) {
-    if (!mixed) {
+    if (!np) {
       mul_a<T>(c.st, ordera, m, n, a, lda, transpose, k, X, Y);
       return;
     }
@@ -235,17 +246,18 @@ struct AProducts {
     }
     g.nprod = 0;
     for (int s = 0; s < 3; ++s)  // plane pairs (p of A, q of X) with p + q < 3
-      for (int p = 0; p <= s && p < 2; ++p) {
+      for (int p = 0; p <= s && p < np; ++p) {
         const int q = s - p;
         if (transpose) { g.pa[g.nprod] = q; g.pb[g.nprod] = p; } else { g.pa[g.nprod] = p; g.pb[g.nprod] = q; }
         ++g.nprod;
       }
     g.c_double = false;
+    g.chunk_k = mixed ? 0 : f32_chunk();
     g.status = c.status;
     g.tag = "adjoint_a";
     umma_gemm(g, c.st);
   }
-  // MIXED only: one pass over A for two k-column operands side by side,
+  // On the planes: one pass over A for two k-column operands side by side,
   //   Y = A [X1 | X2] (m x 2k; X1, X2: n x k)   or, transpose,   Y = A' [X1 | X2] (n x 2k; X1, X2: m x k),
   // with X1, X2 of row strides ld1, ld2 and Y of row stride ldy.  Each output column depends on its
   // own operand column only, so the two halves are the products mul() would give (to the rounding
@@ -275,12 +287,13 @@ struct AProducts {
     }
     g.nprod = 0;
     for (int sum = 0; sum < 3; ++sum)  // plane pairs (p of A, q of X) with p + q < 3
-      for (int p = 0; p <= sum && p < 2; ++p) {
+      for (int p = 0; p <= sum && p < np; ++p) {
         const int q = sum - p;
         if (transpose) { g.pa[g.nprod] = q; g.pb[g.nprod] = p; } else { g.pa[g.nprod] = p; g.pb[g.nprod] = q; }
         ++g.nprod;
       }
     g.c_double = false;
+    g.chunk_k = mixed ? 0 : f32_chunk();
     g.status = c.status;
     g.tag = "adjoint_a2";
     umma_gemm(g, c.st);
@@ -398,7 +411,7 @@ int complement_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, long lo
   };
   int it = 0;
   const char *sep = getenv("ISVD_GPU_ADJOINT_SEPARATE");  // diagnostic: one pass over A per product
-  if (A.mixed && sys[0].active && sys[1].active && !(sep && atoi(sep) != 0)) {
+  if (A.np && sys[0].active && sys[1].active && !(sep && atoi(sep) != 0)) {
     // Both systems in one pass over A per product: the left operator applies A' then A, the right
     // one A then A', so with the right system half an iteration behind, every product by A' takes
     // [p_L | w_R] and every product by A takes [w_L | p_R] (2k columns, one read of A's planes):
@@ -608,7 +621,7 @@ int svd_adjoint_dev(const StageCtx &c, int m, int n, int k, char ordera, const T
   }
   adj_core_kernel<T><<<egrid((long long)kk), 256, 0, st>>>(k, s, ds, K1.p, K2.p, J.p);
   KLAUNCHED();
-  AProducts<T> A(c, m, n, ordera, a, lda);
+  AProducts<T> A(c, m, n, k, ordera, a, lda);
   if (!du) CK(cudaMemsetAsync(lam.p, 0, mk * sizeof(T), st));
   if (!dv) CK(cudaMemsetAsync(gam.p, 0, nk * sizeof(T), st));
   // MIXED, n <= m: the systems in the n-dimensional coordinates of B'B (ISVD_GPU_ADJOINT_CG_A=1 keeps

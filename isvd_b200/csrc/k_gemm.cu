@@ -1,5 +1,5 @@
-// General strided matrix product on CUDA cores (FP64 / FP32), used by the NATIVE precision path
-// and for the small (Nl x l, l x l) products of the integration loop.
+// General strided matrix product on CUDA cores (FP64 / FP32), used by the NATIVE precision path (its
+// smaller FP32 products; the larger ones go to k_f32x3.cu) and for the small (Nl x l, l x l) products of the integration loop.
 //
 // Tiling: BM x BN output tile per 256-thread CTA, BK-deep K slices staged in shared memory
 // with register prefetch of the next slice; each thread owns a (BM/16) x (BN/16) register
@@ -274,6 +274,9 @@ void gemm(const Gemm<T, Tout> &g, cudaStream_t st) {
       dmma_gemm(g, a_kc, b_nc, st);
       return;
     }
+  }
+  if constexpr (std::is_same<T, float>::value) {
+    if (gemm_f32_planes(g, a_kc, b_nc, st)) return;  // large FP32 products: bf16 planes on the tensor cores
   }
   if (g.pl_t) fail(kErrArgument, "gemm: plane output only on the FP64 tensor-core path");
   // 128 x 128 tiles when they fill the GPU, or when a long inner dimension lets split-K fill it

@@ -50,6 +50,7 @@ struct KParams {
   int upper;  // only tiles intersecting the upper triangle (symmetric output)
   int *status;
   int chunk_kb;   // k-blocks per tensor-memory accumulation chunk
+  int unbias;     // chunks of one k-block, the leading plane pair last: see UmmaGemm::unbias
   int stage_out;  // epilogue stages its rows through shared memory (C rows contiguous)
   int bloop;      // one CTA runs every batch of its tile in turn (grid z = 1, no split-K)
   int vec_out;    // direct epilogue stores as 16-byte vectors (C rows contiguous and aligned)
@@ -436,6 +437,15 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t v[16];
         tmem_ld16(tbase + (uint32_t)j, v);
         tmem_wait();
+        if (p.unbias) {
+          // half a unit in the last place for a 32-deep chunk, three quarters for a 64-deep one, on
+          // average over the values with an odd last place (UmmaGemm::unbias)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const uint32_t odd = v[i] & 1u;
+            v[i] += BK == 64 ? odd + (odd & (v[i] >> 1)) : odd;
+          }
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[j + i] += __uint_as_float(v[i]);
       }
@@ -917,18 +927,6 @@ __global__ void mirror_upper_kernel(T *C, long long n, long long ld) {
 
 // ------------------------------------------------------------------------------ splits
 
-// Pieces of an FP32 value in FP32 arithmetic: x - bf16(x) is exact in FP32 (the rounding error of
-// an 8-bit rounding of a 24-bit significand), and so is the next remainder.
-__device__ __forceinline__ void split3f(float x, __nv_bfloat16 *o) {
-  const __nv_bfloat16 h0 = __float2bfloat16_rn(x);
-  const float r1 = x - __bfloat162float(h0);
-  const __nv_bfloat16 h1 = __float2bfloat16_rn(r1);
-  const float r2 = r1 - __bfloat162float(h1);
-  o[0] = h0;
-  o[1] = h1;
-  o[2] = __float2bfloat16_rn(r2);
-}
-
 // Non-transposed: plane(r, c) for r < rows_pad, c < ld (zero outside rows x cols).  Grid: x over
 // 8-column groups of a row (one 16-byte vector per plane per thread), y striding over rows; rows
 // with unit column stride and 16-byte aligned starts are read as vectors.
@@ -1164,7 +1162,8 @@ void launch_t(const UmmaGemm &g, cudaStream_t st, int *status) {
   const int stage_bytes = g.A.np * C::A_TILE + g.B.np * C::B_TILE;
   const int budget = (int)rt.smem_optin - 1024 - 256;
   int stages = std::min(8, budget / stage_bytes);
-  p.chunk_kb = chunk_kblocks(BK, g.chunk_k);
+  p.chunk_kb = g.unbias ? 1 : chunk_kblocks(BK, g.chunk_k);
+  p.unbias = g.unbias ? 1 : 0;
   // rows of C contiguous (or a split-K partial): stage the epilogue through shared memory when the
   // pipeline buffers can hold the 8 warps' 32 x (BN/2 + 1) blocks
   // many short batches (e.g. N block products of K = l): one CTA per tile runs all of them in turn,
@@ -1357,7 +1356,7 @@ static bool pair_mn_ok(const UmmaGemm &g) {
   const char *e = getenv("ISVD_UMMA_PAIR_MN");
   if (e && atoi(e) == 0) return false;
   const long long tiles = (long long)((g.N + 255) / 256) * ((g.M + 255) / 256);
-  return tiles >= Runtime::get().num_sms / 2 && g.K >= 1024 && g.A.np + g.B.np <= 4;
+  return tiles >= Runtime::get().num_sms / 2 && g.K >= 1024 && !g.unbias && g.A.np + g.B.np <= 4;
 }
 // ISVD_UMMA_WIDE_MN=0: MN-major B products keep 128-wide tiles (for comparison)
 static bool wide_mn_off() {
@@ -1413,7 +1412,7 @@ void umma_gemm(const UmmaGemm &g, cudaStream_t st) {
     const int sbk = smalln_bk();
     if (g.A.np + g.B.np >= 5 && (sbk == 32 || (sbk != 64 && !few_tiles))) launch_t<128, 32, false, false>(g, st, status);
     else launch_t<128, 64, false, false>(g, st, status);
-  } else if (g.batch == 1 && g.splits <= 0 && !g.upper && !g.planes && pair_ok(g)) {
+  } else if (g.batch == 1 && g.splits <= 0 && !g.upper && !g.planes && !g.unbias && pair_ok(g)) {
     if (pair_bk() == 32) launch_pair<32, false>(g, st, status);
     else launch_pair<64, false>(g, st, status);
   } else if (3 * stage64 <= (int)rt.smem_optin - 2048 && !bk32_forced()) {

@@ -40,6 +40,12 @@ struct Gemm {
 template <class T, class Tout>
 void gemm(const Gemm<T, Tout> &g, cudaStream_t st);
 
+// FP32 operands as three bf16 planes on the tensor cores (k_f32x3.cu): true when the product was
+// enqueued there, false when it has to run on the CUDA cores (too small, a layout the planes do not
+// take, beta != 0, or no memory for the planes).
+template <class Tout>
+bool gemm_f32_planes(const Gemm<float, Tout> &g, bool a_kc, bool b_nc, cudaStream_t st);
+
 // FP64 operands and result on the FP64 tensor-core path (mma.sync m8n8k4, k_dmma.cu); gemm()
 // routes Gemm<double, double> here unless ISVD_GPU_DMMA=0.  a_kc: A has unit K stride; b_nc: B
 // has unit N stride.

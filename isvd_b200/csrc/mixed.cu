@@ -86,7 +86,7 @@ int sketch_planes() {
 // less, eight lose 5 %, and the L2 evict-last policy on Omega' gains nothing.
 // ISVD_GPU_SKETCH_NGROUP overrides the group width (0: row-major order), ISVD_GPU_SKETCH_L2HINT=1
 // adds the evict-last / evict-first policies.
-static void sketch_tile_order(UmmaGemm &g, long long n, long long Nl, int bn) {
+void sketch_tile_order(UmmaGemm &g, long long n, long long Nl, int bn) {
   static const long long l2 = [] {
     int dev = 0, v = 0;
     CK(cudaGetDevice(&dev));

@@ -69,6 +69,35 @@ template <class T>
 void mixed_sketch(const StageCtx &c, int m, int n, int Nl, char ordera, const T *a, long long lda, const T *omega,
                   long long ldom, uint64_t seed, T *y, long long ldy, PlaneHandoff *hand = nullptr);
 
+// Tile order of a sketch product whose Omega' (B planes set) is larger than L2.
+void sketch_tile_order(UmmaGemm &g, long long n, long long Nl, int bn);
+
+// NATIVE FP32 on the bf16 tensor cores (k_f32x3.cu): operands in three planes, exact to FP32.
+// The sketch: A's planes against the one exact plane of an Omega drawn here (offset: the value offset of
+// its first row).  keep: the planes of all rows stay there for f32_project when memory allows.
+bool f32_sketch_pays(long long m, long long n, long long Nl, long long offset);
+void f32_sketch_rows(const Planes &omega_t, long long rows, int n, int Nl, char ordera, const float *a, long long ld,
+                     float *y, long long ldy, MixedCache *keep, cudaStream_t st);
+// Z = A' Qbar from the sketch's planes of A; false when mc does not hold them.
+bool f32_project(const MixedCache *mc, int m, int n, int l, char ordera, const float *a, const float *qt, long long ldqt,
+                 float *z, cudaStream_t st);
+// Accumulation chunk of FP32-exact plane products; whether repeated products of an m x n A with
+// k columns are faster from A's three planes.
+int f32_chunk();
+bool f32_operator_pays(long long m, long long n, int k);
+// Planes of the N column blocks (l columns, each block padded to a multiple of 8) of a tall matrix, and
+// W_i = Y_i' Y_i and out_i = Y_i Wp_i from them (out may be the matrix itself).  f32_block_planes: false
+// when the products are too small for planes or there is no memory for them.
+bool f32_block_planes(PlaneBuf &pb, const float *y, long long ldy, long long rows, int l, int N, cudaStream_t st);
+void f32_block_gram(const PlaneBuf &yp, int rows, int l, int N, double *W, cudaStream_t st);
+void f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp, float *out, long long ldo,
+                     cudaStream_t st);
+// Planes of a tall rows x Nl matrix, G = Qs'Qs (whole) and out = Qs M from them.
+bool f32_tall_planes(PlaneBuf &pb, const float *qs, long long ldq, long long rows, int Nl, cudaStream_t st);
+void f32_tall_gram(const PlaneBuf &qp, int rows, int Nl, double *G, cudaStream_t st);
+void f32_tall_apply(const PlaneBuf &qp, int rows, int Nl, int l, const float *M, long long ldm, float *out, long long ldo,
+                    cudaStream_t st);
+
 // The next four take bf16 planes `yp` of an m x Nl row-major matrix (split without transpose,
 // make_planes(.., false)) and the matrix itself (`y`, used when the block width rules out the
 // plane path: l % 8 != 0 for MN-major operands, l % 64 != 0 for per-block K offsets).

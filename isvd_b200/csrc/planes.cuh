@@ -21,6 +21,24 @@ __device__ __forceinline__ void split3(T x, __nv_bfloat16 *o, int np) {
   }
 }
 
+// Pieces of an FP32 value in FP32 arithmetic: x - bf16(x) is exact in FP32 (the rounding error of
+// an 8-bit rounding of a 24-bit significand), and so is the next remainder.  Infinities and NaN stay
+// whole in the first piece; a value that would round up to infinity is truncated there instead.
+__device__ __forceinline__ void split3f(float x, __nv_bfloat16 *o) {
+  __nv_bfloat16 h0 = __float2bfloat16_rn(x);
+  float f0 = __bfloat162float(h0), r1 = x - f0;
+  if (!(fabsf(f0) <= 3.4028235e38f)) {
+    const bool finite = fabsf(x) <= 3.4028235e38f;
+    f0 = finite ? __uint_as_float(__float_as_uint(x) & 0xffff0000u) : x;
+    h0 = __float2bfloat16_rn(f0);
+    r1 = finite ? x - f0 : 0.f;
+  }
+  const __nv_bfloat16 h1 = __float2bfloat16_rn(r1);
+  o[0] = h0;
+  o[1] = h1;
+  o[2] = __float2bfloat16_rn(r1 - __bfloat162float(h1));
+}
+
 __device__ __forceinline__ uint4 pack8(const __nv_bfloat16 *v) {
   uint4 u;
   u.x = (uint32_t)__bfloat16_as_ushort(v[0]) | ((uint32_t)__bfloat16_as_ushort(v[1]) << 16);

@@ -1,8 +1,9 @@
-// Device-level iSVD stages (one MPI rank).  NATIVE precision: products in the stage's type on
-// CUDA cores; l x l steps in FP64.  MIXED precision routes the large products to the tcgen05
+// Device-level iSVD stages (one MPI rank).  NATIVE precision: products in the stage's type (FP64 on
+// mma.sync, large FP32 products on bf16 planes, k_f32x3.cu); l x l steps in FP64.  MIXED precision routes the large products to the tcgen05
 // bf16 split-product engine (mixed.cu).
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.h"
@@ -50,13 +51,30 @@ void sketch_dev(const StageCtx &c, int m, int n, int Nl, char ordera, const T *a
     return;
   }
   DBuf<T> om;
-  if (!omega) {
+  PlaneBuf om_t;  // FP32: Omega' as one exact bf16 plane, for the tensor-core sketch
+  if constexpr (std::is_same<T, float>::value) {
+    const long long off = c.col_begin * (long long)Nl;
+    if (!omega && f32_sketch_pays(m, n, Nl, off)) {
+      const long long old = plane_ld(n), orp = plane_rows(Nl);
+      om_t.buf.alloc((size_t)orp * old);
+      rng_gaussian_bf16_t(om_t.buf.p, n, Nl, old, orp, seed, c.st, off);
+      Planes &P = om_t.P;
+      P.ptr = om_t.buf.p; P.np = 1; P.rows = Nl; P.cols = n; P.ld = old; P.plane_stride = orp * old;
+    }
+  }
+  if (!omega && !om_t.P.ptr) {
     om.alloc((size_t)n * Nl);
     rng_gaussian<T>(om.p, n, Nl, Nl, seed, (uint64_t)c.col_begin * Nl, c.st);  // column blocks: own rows
     omega = om.p;
     ldom = Nl;
   }
   auto rows_times_omega = [&](long long r0, long long rows, const T *ap, long long ld) {
+    if constexpr (std::is_same<T, float>::value) {
+      if (om_t.P.ptr) {
+        f32_sketch_rows(om_t.P, rows, n, Nl, ordera, ap, ld, y + r0 * ldy, ldy, ap == a ? c.cache : nullptr, c.st);
+        return;
+      }
+    }
     Gemm<T, T> g = gm<T>((int)rows, Nl, n);
     g.A = ap; set_a(g, ordera, ld, false);
     g.B = omega; g.b_rs = ldom; g.b_cs = 1;
@@ -86,8 +104,13 @@ void gramian_pass(const StageCtx &c, int m, int l, int N, T *y, long long ldy, b
   const bool from_hand = c.precision == kMixed && c.handoff && c.handoff->holds(y, ldy);
   if (from_hand) yp.P = c.handoff->pb.P;
   else if (c.precision == kMixed) make_planes<T>(yp, y, ldy, m, Nl, 3, false, c.st);
+  bool fp = false;  // FP32: yp holds the planes of Y's blocks
+  if constexpr (std::is_same<T, float>::value)
+    if (c.precision != kMixed) fp = f32_block_planes(yp, y, ldy, m, l, N, c.st);
   // W_i = Y_i' Y_i   (reference :82-84)
-  if (c.precision == kMixed) {
+  if (fp) {
+    f32_block_gram(yp, m, l, N, W.p, c.st);
+  } else if (c.precision == kMixed) {
     mixed_block_gram<T>(c, yp.P, m, l, N, y, ldy, W.p);
   } else {
     Gemm<T, double> g;
@@ -140,6 +163,11 @@ void gramian_pass(const StageCtx &c, int m, int l, int N, T *y, long long ldy, b
     if (!out_planes && c.handoff && c.handoff->holds(y, ldy)) c.handoff->of = nullptr;  // y's values changed
     return;
   }
+  if constexpr (std::is_same<T, float>::value)
+    if (fp) {
+      f32_block_apply(yp, m, l, N, Wp.p, y, ldy, c.st);
+      return;
+    }
   if (from_hand) fail(kErrUnsupported, "plane hand-off into the Gramian orthogonalization needs l %% 64 == 0");
   DBuf<T> tmp((size_t)m * Nl);
   if (c.precision == kMixed) {
@@ -237,7 +265,11 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
   PlaneBuf qp;  // MIXED: bf16 planes of Qs, shared by G and the final Qbar = Qs M
   if (c.precision == kMixed && c.handoff && c.handoff->holds(qs, ldq)) qp.P = c.handoff->pb.P;  // the apply's
   else if (c.precision == kMixed) make_planes<T>(qp, qs, ldq, m, Nl, 3, false, c.st);
-  if (c.precision == kMixed) {
+  bool fp = false;  // FP32: qp holds the planes of Qs
+  if constexpr (std::is_same<T, float>::value)
+    if (c.precision != kMixed && (fp = f32_tall_planes(qp, qs, ldq, m, Nl, c.st))) f32_tall_gram(qp, m, Nl, G.p, c.st);
+  if (fp) {
+  } else if (c.precision == kMixed) {
     mixed_gram_full<T>(c, qp.P, m, Nl, qs, ldq, G.p);
   } else {
     Gemm<T, double> g;
@@ -371,6 +403,11 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
   } else {
     DBuf<T> Mt(nl);
     copy2d<double, T>(Wp, lw, 1, Mt.p, l, 1, Nl, l, c.st);
+    if constexpr (std::is_same<T, float>::value)
+      if (fp) {
+        f32_tall_apply(qp, m, Nl, l, Mt.p, l, qt, ldqt, c.st);
+        return res;
+      }
     Gemm<T, T> g = gm<T>(m, l, Nl);
     g.A = qs; g.a_rs = ldq; g.a_cs = 1;
     g.B = Mt.p; g.b_rs = l; g.b_cs = 1;
@@ -428,6 +465,8 @@ void project(const StageCtx &c, int m, int n, int l, char ordera, const T *a, lo
     mixed_project<T>(c, m, n, l, ordera, a, lda, qt, ldqt, z);
     return;
   }
+  if constexpr (std::is_same<T, float>::value)
+    if (f32_project(c.cache, m, n, l, ordera, a, qt, ldqt, z, c.st)) return;
   auto add_rows = [&](long long r0, long long rows, const T *ap, long long ld) {  // Z += A_p' Qbar_p
     Gemm<T, T> g = gm<T>(n, l, (int)rows);
     g.A = ap; set_a(g, ordera, ld, true);
@@ -473,7 +512,18 @@ void post_gramian_dev(const StageCtx &c, int m, int n, int k, int l, char ordera
   DBuf<T> Z((size_t)n * l);
   project_sum<T>(c, m, n, l, ordera, a, lda, qt, ldqt, Z.p);  // several ranks: the whole Z on each
   DBuf<double> W(ll), V(ll), w(l);
-  {  // W = Z' Z  (reference @x@_postprocess_gramian.c:145)
+  // W = Z' Z  (reference @x@_postprocess_gramian.c:145).  FP32: in FP64 on mma.sync -- 2 n l^2 operations are
+  // few (8 us at n = 2003, l = 65), and rounding of W is what close singular values amplify in U and V
+  DBuf<double> Zd;
+  if (std::is_same<T, float>::value && c.precision != kMixed && dmma_enabled()) {
+    Zd.alloc((size_t)n * l);
+    copy2d<T, double>(Z.p, l, 1, Zd.p, l, 1, n, l, c.st);
+    Gemm<double, double> g = gm<double>(l, l, n);
+    g.A = Zd.p; g.a_rs = 1; g.a_cs = l;
+    g.B = Zd.p; g.b_rs = l; g.b_cs = 1;
+    g.C = W.p; g.c_rs = l; g.c_cs = 1;
+    gemm(g, c.st);
+  } else {
     Gemm<T, double> g;
     g.M = l; g.N = l; g.K = n;
     g.A = Z.p; g.a_rs = 1; g.a_cs = l;

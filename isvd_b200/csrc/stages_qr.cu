@@ -115,7 +115,12 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
   long long lds = ldy, ldd = Nl;
   for (int pass = 0; pass < 3; ++pass) {
     PlaneBuf yp;
-    if (mixed) {
+    bool fp = false;  // FP32: yp holds the planes of the blocks, the product may overwrite them
+    if constexpr (std::is_same<T, float>::value)
+      if (!mixed && (fp = f32_block_planes(yp, src, lds, rows, l, N, c.st)))
+        f32_block_gram(yp, (int)rows, l, N, W.p, c.st);
+    if (fp) {
+    } else if (mixed) {
       make_planes<T>(yp, src, lds, rows, Nl, 3, false, c.st);
       mixed_block_gram<T>(c, yp.P, (int)rows, l, N, src, lds, W.p);
     } else {
@@ -151,6 +156,11 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
       }
     }
     copy2d<double, T>(X.p, l, 1, Xt.p, l, 1, (long long)N * l, l, c.st);
+    if constexpr (std::is_same<T, float>::value)
+      if (fp) {
+        f32_block_apply(yp, (int)rows, l, N, Xt.p, src, lds, c.st);
+        continue;
+      }
     if (mixed) {
       mixed_block_apply<T>(c, yp.P, (int)rows, l, N, src, lds, Xt.p, dst, ldd);
     } else {
@@ -168,8 +178,8 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
   CK(cudaMemcpyAsync(&nulls, nmask.p + Nl, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
   if (nulls > 0) complete_null_columns<T>(c, rows, l, N, src, lds, dst, ldd, nmask.p);
-  // three passes: y -> tmp -> y -> tmp (two more for a completion: -> y -> tmp)
-  CK(cudaMemcpy2DAsync(y, ldy * sizeof(T), src, lds * sizeof(T), (size_t)Nl * sizeof(T), rows,
+  // three passes: y -> tmp -> y -> tmp (two more for a completion: -> y -> tmp), or in place
+  if (src != y) CK(cudaMemcpy2DAsync(y, ldy * sizeof(T), src, lds * sizeof(T), (size_t)Nl * sizeof(T), rows,
                        cudaMemcpyDeviceToDevice, c.st));
 }
 
@@ -204,7 +214,11 @@ IterResult integrate_wy_dev(const StageCtx &c, int m, int l, int N, const T *qs,
   cudaStream_t st = c.st;
   DBuf<double> G((size_t)Nl * Nl);
   PlaneBuf qp;  // MIXED: bf16 planes of Qs, shared by G and the final Qbar = Qs M
-  if (mixed) {
+  bool fp = false;  // FP32: qp holds the planes of Qs
+  if constexpr (std::is_same<T, float>::value)
+    if (!mixed && (fp = f32_tall_planes(qp, qs, ldq, m, Nl, st))) f32_tall_gram(qp, m, Nl, G.p, st);
+  if (fp) {
+  } else if (mixed) {
     if (c.handoff && c.handoff->holds(qs, ldq)) qp.P = c.handoff->pb.P;  // the Gramian apply's planes
     else make_planes<T>(qp, qs, ldq, m, Nl, 3, false, st);
     mixed_gram_full<T>(c, qp.P, m, Nl, qs, ldq, G.p);
@@ -353,6 +367,11 @@ IterResult integrate_wy_dev(const StageCtx &c, int m, int l, int N, const T *qs,
   } else {
     DBuf<T> Mt(nl);
     copy2d<double, T>(Mp, l, 1, Mt.p, l, 1, Nl, l, st);
+    if constexpr (std::is_same<T, float>::value)
+      if (fp) {
+        f32_tall_apply(qp, m, Nl, l, Mt.p, l, qt, ldqt, st);
+        return res;
+      }
     Gemm<T, T> g;
     g.M = m; g.N = l; g.K = Nl;
     g.A = qs; g.a_rs = ldq; g.a_cs = 1;

@@ -117,6 +117,8 @@ size_t device_budget() {
 
 long long host_panel_rows(long long m, long long n, size_t resident_bytes, size_t row_bytes, size_t work_bytes,
                           size_t elem) {
+  // without a limit, what fits in any device needs no look at the free memory (100 us)
+  if (isvd_gpu_memory_limit == 0 && resident_bytes + work_bytes <= ((size_t)128 << 20)) return 0;
   const size_t budget = device_budget();
   if (resident_bytes + work_bytes <= budget) return 0;
   const size_t avail = budget > work_bytes ? budget - work_bytes : 0;

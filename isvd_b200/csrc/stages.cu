@@ -1,6 +1,6 @@
 // Device-level iSVD stages (one MPI rank).  NATIVE precision: products in the stage's type (FP64 on
-// mma.sync, large FP32 products on bf16 planes, k_f32x3.cu); l x l steps in FP64.  MIXED precision routes the large products to the tcgen05
-// bf16 split-product engine (mixed.cu).
+// mma.sync, large FP32 products on bf16 planes, k_f32x3.cu); l x l steps in FP64.  MIXED precision
+// routes the large products to the tcgen05 bf16 split-product engine (mixed.cu).
 #include <cmath>
 #include <cstdlib>
 #include <type_traits>
@@ -307,9 +307,13 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
     return !(e && atoi(e) == 0);
   }();
   bool split_bc = true;  // the first iteration's Bc = G[:, 0:l] is split by the G product
-  // One iteration: W(next) from W(cur).  After two eager iterations (which size every buffer and
-  // set every kernel attribute) the iteration is captured as one CUDA graph per parity of the
-  // ping-pong buffers, so that an iteration costs one graph launch plus the host read of err.
+  // One iteration: W(next) from W(cur).  Iterations are enqueued one ahead of the GPU (below), and the six
+  // launches of one take the host about 35 us against 50 us and more on the GPU; only after
+  // kGraphFrom of them is the iteration captured as one CUDA graph per parity of the ping-pong
+  // buffers.  Capturing, instantiating and destroying the two graphs costs about 400 us, more than all of
+  // a short loop's launches: a 2000 x 1000 solve of 11 iterations takes 1657 us with graphs from the
+  // third iteration on and 1290 us without; from the 33rd on they pay for themselves in host time.
+  constexpr int kGraphFrom = 32;
   auto iteration = [&](double *Wcur, double *Wnext, double *errp) {
     double *Bc = Wcur + l, *Bgc = Wcur + 2 * l;
     if (c.precision == kMixed) {  // Bgc = G Bc / N   (:174-177)
@@ -370,7 +374,7 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
   for (int e = 0; e < 2; ++e) CK(cudaEventCreateWithFlags(&ev[e], cudaEventDisableTiming));
   auto launch = [&](int it, double *cur, double *next) {
     const int par = it & 1;
-    if (graphs.usable && it > 2) graphs.run(par, [&] { iteration(cur, next, hpin + par); });
+    if (graphs.usable && it > kGraphFrom) graphs.run(par, [&] { iteration(cur, next, hpin + par); });
     else iteration(cur, next, hpin + par);
     CK(cudaEventRecord(ev[par], c.st));
   };

@@ -30,6 +30,7 @@
 
 #include "kernels.h"
 #include "mixed.h"
+#include "planes.cuh"
 #include "runtime.h"
 #include "stages.h"
 
@@ -126,6 +127,189 @@ __global__ void cg_step2_kernel(T *p, const T *__restrict__ r, long long rows, i
     const int c = (int)(e % k);
     const double b = rr[c] > 0.0 ? rn[c] / rr[c] : 0.0;
     p[e] = (T)((double)r[e] + b * (double)p[e]);
+  }
+}
+
+// The conjugate-gradient iteration of complement_gram_cg in three launches behind the operator's product z:
+//   cg_apply_kernel   q = s^2 p - z and pq_c = p_c' q_c
+//   cg_update_kernel  x += a p, r -= a q (a_c = rr_c / pq_c), rn_c = r_c' r_c, b_c = rn_c / rr_c, rr = rn
+//   cg_next_kernel    p = r + b p, and the planes of p' for the next product
+// A dot product is finished by the last CTA of its own launch (arrival counter; the slices are added in
+// order, so the result does not depend on which CTA is last).  `ctl` holds [0] the arrival counter and
+// [1] the done word: set by the update that brings every column below tol, after which the launches
+// that the host has already enqueued return at once.  Bound by latency (the loads, two reductions and the
+// arrival counter; 2 to 4 MB moved): at n = 4096, 2 k = 128 the three take 15, 18 and 6 us, where two
+// dot products of two launches each, the scaling, both steps, a copy and the split took 52.
+constexpr int kCgThreads = 512;
+constexpr int kCgBlocks = 128;
+
+// acc: this thread's sums of columns c0 + t % cw over its rows; adds the CTA's slices and, in the last CTA,
+// all of them (fin: column, sum).
+template <class F>
+__device__ __forceinline__ void cg_dot_finish(double *sh, int kc, double *partial, unsigned *ctl, F fin) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ctl, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) ctl[0] = 0;
+  // four columns per warp at a time, lanes over the slices: sixteen loads in flight
+  constexpr int kSl = (kCgBlocks + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  for (int c0 = 4 * (threadIdx.x >> 5); c0 < kc; c0 += 4 * (kCgThreads / 32)) {
+    double v[4][kSl];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int w = 0; w < kSl; ++w) {
+        const int b = lane + 32 * w;
+        v[u][w] = (c0 + u < kc && b < (int)gridDim.x) ? __ldcg(partial + (size_t)b * kc + c0 + u) : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      double s = v[u][0];
+#pragma unroll
+      for (int w = 1; w < kSl; ++w) s += v[u][w];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0 && c0 + u < kc) sh[c0 + u] = s;
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < kc; c += kCgThreads) fin(c, sh[c]);
+}
+
+// Rows of this CTA; prep(column) returns f with f.load(element) and f.apply(element, loaded), which stores
+// the element's results and returns its term of the column's dot product.  Eight elements are loaded
+// before the first is stored.
+template <class F>
+__device__ __forceinline__ void cg_dot_rows(double *sh, long long rows, int kc, double *partial, F prep) {
+  const long long per = (rows + gridDim.x - 1) / gridDim.x;
+  const long long r0 = blockIdx.x * per, r1 = min(rows, r0 + per);
+  for (int c0 = 0; c0 < kc; c0 += kCgThreads) {
+    const int cw = min(kCgThreads, kc - c0), lanes = kCgThreads / cw, t = threadIdx.x;
+    double v = 0.0;
+    if (t < lanes * cw) {
+      const int c = c0 + t % cw;
+      const auto f = prep(c);
+      for (long long r = r0 + t / cw; r < r1; r += 8LL * lanes) {
+        float4 in[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (r + u * lanes < r1) in[u] = f.load((r + u * lanes) * kc + c);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (r + u * lanes < r1) v += f.apply((r + u * lanes) * kc + c, in[u]);
+      }
+    }
+    __syncthreads();
+    sh[t] = v;
+    __syncthreads();
+    if (t < cw) {
+      double sum = 0.0;
+      for (int j = 0; j < lanes; ++j) sum += sh[j * cw + t];
+      partial[(size_t)blockIdx.x * kc + c0 + t] = sum;
+    }
+  }
+}
+
+struct CgApply {
+  const float *p, *z;
+  float *q;
+  double s2;
+  __device__ float4 load(long long e) const { return make_float4(p[e], z[e], 0.f, 0.f); }
+  __device__ double apply(long long e, float4 v) const {
+    const float qe = (float)((double)v.x * s2 - (double)v.y);
+    q[e] = qe;
+    return (double)v.x * (double)qe;
+  }
+};
+
+struct CgUpdate {
+  float *x, *r;
+  const float *p, *q;
+  double a;
+  __device__ float4 load(long long e) const { return make_float4(x[e], r[e], p[e], q[e]); }
+  __device__ double apply(long long e, float4 v) const {
+    x[e] = (float)((double)v.x + a * (double)v.z);
+    const float re = (float)((double)v.y - a * (double)v.w);
+    r[e] = re;
+    return (double)re * (double)re;
+  }
+};
+
+__global__ void __launch_bounds__(kCgThreads)
+    cg_apply_kernel(const float *__restrict__ p, const float *__restrict__ z, const float *__restrict__ s,
+                    float *__restrict__ q,
+                    long long rows, int kc, double *partial, unsigned *ctl, double *pq) {
+  extern __shared__ double sh[];
+  if (((volatile unsigned *)ctl)[1]) return;
+  cg_dot_rows(sh, rows, kc, partial, [=](int c) {
+    const double sc = s[c];
+    return CgApply{p, z, q, sc * sc};
+  });
+  cg_dot_finish(sh, kc, partial, ctl, [&](int c, double v) { pq[c] = v; });
+}
+
+__global__ void __launch_bounds__(kCgThreads)
+    cg_update_kernel(float *__restrict__ x, float *__restrict__ r, const float *__restrict__ p, const float *__restrict__ q, long long rows, int kc,
+                     double *rr, const double *__restrict__ bb, const double *__restrict__ pq, double *beta, double tol2,
+                     double *partial, unsigned *ctl, double *host_done) {
+  extern __shared__ double sh[];
+  __shared__ int above;
+  if (((volatile unsigned *)ctl)[1]) return;
+  cg_dot_rows(sh, rows, kc, partial, [=](int c) {
+    return CgUpdate{x, r, p, q, (rr[c] > 0.0 && pq[c] != 0.0) ? rr[c] / pq[c] : 0.0};
+  });
+  if (threadIdx.x == 0) above = 0;
+  bool mine = false;  // this CTA is the last one
+  cg_dot_finish(sh, kc, partial, ctl, [&](int c, double v) {
+    beta[c] = rr[c] > 0.0 ? v / rr[c] : 0.0;
+    rr[c] = v;
+    if (v > tol2 * bb[c]) above = 1;
+    mine = true;
+  });
+  if (!__syncthreads_or(mine)) return;
+  if (threadIdx.x == 0) {
+    ctl[1] = above ? 0u : 1u;
+    *host_done = above ? 0.0 : 1.0;
+  }
+}
+
+// 64 rows x 32 columns of p per CTA; planes: kc x rows, row stride ld, plane stride ps.
+__global__ void __launch_bounds__(256)
+    cg_next_kernel(float *p, const float *__restrict__ r, const double *__restrict__ beta, long long rows, int kc,
+                   const unsigned *ctl, __nv_bfloat16 *__restrict__ planes, long long ld, long long ps) {
+  __shared__ float tile[64][33];
+  if (((const volatile unsigned *)ctl)[1]) return;
+  const long long r0 = (long long)blockIdx.x * 64;
+  const int c0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int j = ty; j < 64; j += 8) {
+    const long long row = r0 + j;
+    const int c = c0 + tx;
+    float v = 0.f;
+    if (row < rows && c < kc) {
+      const long long e = row * kc + c;
+      v = (float)((double)r[e] + beta[c] * (double)p[e]);
+      p[e] = v;
+    }
+    tile[j][tx] = v;
+  }
+  __syncthreads();
+  const int cl = threadIdx.x >> 3, seg = threadIdx.x & 7;
+  const long long rr0 = r0 + 8 * seg;
+  if (c0 + cl < kc && rr0 < ld) {
+    __nv_bfloat16 o[3][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      __nv_bfloat16 t[3];
+      split3f(tile[8 * seg + i][cl], t);
+      o[0][i] = t[0]; o[1][i] = t[1]; o[2][i] = t[2];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) *(uint4 *)(planes + k * ps + (long long)(c0 + cl) * ld + rr0) = pack8(o[k]);
   }
 }
 
@@ -502,12 +686,32 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
     g.alpha = alpha; g.beta = beta;
     gemm(g, st);
   };
-  dprod(n, n, k, b1d.p, k, 1, b1d.p, 1, k, G.p, n, -1.0, 1.0);  // H = G - B1' B1
-  dprod(n, k, n, G.p, n, 1, vd.p, k, 1, hv.p, k, 1.0, 0.0);     // H V
-  dprod(k, k, n, vd.p, 1, k, hv.p, k, 1, cm.p, k, 1.0, 0.0);    // C = V' H V
-  dprod(n, k, k, vd.p, k, 1, cm.p, k, 1, hv.p, k, -0.5, 1.0);   // Z = H V - V C / 2
-  dprod(n, n, k, vd.p, k, 1, hv.p, 1, k, G.p, n, -1.0, 1.0);    // H - V Z'
-  dprod(n, n, k, hv.p, k, 1, vd.p, 1, k, G.p, n, -1.0, 1.0);    //   - Z V'  = Gp
+  // with H = G - B1' B1 and Z = H V - V (V' H V) / 2:  Gp = H - V Z' - Z V', one rank-3k update of the upper
+  // triangle (each pass over the n x n FP64 matrix costs more than its rank-k product)
+  dprod(n, k, n, G.p, n, 1, vd.p, k, 1, hv.p, k, 1.0, 0.0);         // G V
+  dprod(k, k, n, b1d.p, 1, k, vd.p, k, 1, cm.p, k, 1.0, 0.0);       // B1 V  (k x k; b1d = B1')
+  dprod(n, k, k, b1d.p, k, 1, cm.p, k, 1, hv.p, k, -1.0, 1.0);      // H V = G V - B1' (B1 V)
+  dprod(k, k, n, vd.p, 1, k, hv.p, k, 1, cm.p, k, 1.0, 0.0);        // C = V' H V
+  dprod(n, k, k, vd.p, k, 1, cm.p, k, 1, hv.p, k, -0.5, 1.0);       // Z = H V - V C / 2
+  {
+    const long long k3 = 3LL * k;
+    DBuf<double> lhs((size_t)n * k3), rhs((size_t)n * k3);           // [B1' | V | Z], [B1' | Z | V]
+    const double *parts[3] = {b1d.p, vd.p, hv.p};
+    for (int i = 0; i < 3; ++i) {
+      copy2d<double, double>(parts[i], k, 1, lhs.p + i * k, k3, 1, n, k, st);
+      copy2d<double, double>(parts[i == 0 ? 0 : 3 - i], k, 1, rhs.p + i * k, k3, 1, n, k, st);
+    }
+    Gemm<double, double> g;
+    g.M = n; g.N = n; g.K = (int)k3;
+    g.A = lhs.p; g.a_rs = k3; g.a_cs = 1;
+    g.B = rhs.p; g.b_rs = 1; g.b_cs = k3;
+    g.C = G.p; g.c_rs = n; g.c_cs = 1;
+    g.alpha = -1.0; g.beta = 1.0;
+    g.upper = true;
+    g.splits = 1;
+    gemm(g, st);
+    mirror_upper(G.p, n, n, st);
+  }
   PlaneBuf gp;
   make_planes<double>(gp, G.p, n, n, n, 3, false, st);
   // right-hand sides [B' bu | bv] (n x kc) and s repeated per system
@@ -527,8 +731,7 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
   }
   for (int i = 0; i < ns; ++i) CK(cudaMemcpyAsync(s2.p + (size_t)i * k, s, k * sizeof(T), cudaMemcpyDeviceToDevice, st));
   PlaneBuf xp;
-  auto op = [&](const T *X, T *Y) {  // Y = X S^2 - Gp X
-    make_planes<T>(xp, X, kc, n, kc, 3, true, st);  // X' planes (kc x n)
+  auto product = [&]() {  // z = Gp X from X's planes
     UmmaGemm g;
     g.M = n; g.N = kc; g.K = n;
     g.A = gp.P; g.B = xp.P;
@@ -539,39 +742,64 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
     g.status = c.status;
     g.tag = "adjoint_gram_op";
     umma_gemm(g, st);
-    colscale_add<T>(st, Y, X, s2.p, 2, -1.0, z.p, n, kc);
   };
-  DBuf<double> scal((size_t)2 * kc), rn(kc), pq(kc), part((size_t)kColdotBlocks * kc);
+  DBuf<double> scal((size_t)2 * kc), beta(kc), pq(kc), part((size_t)kCgBlocks * kc);
+  DBuf<unsigned> ctl(2);
+  CK(cudaMemsetAsync(ctl.p, 0, 2 * sizeof(unsigned), st));
   double *rr = scal.p, *bb = scal.p + kc;
   colscale_add<T>(st, x.p, b.p, s2.p, -2, 0.0, nullptr, n, kc);  // x = b S^-2
-  op(x.p, q.p);
+  make_planes<T>(xp, x.p, kc, n, kc, 3, true, st);               // X' planes (kc x n)
+  product();
+  colscale_add<T>(st, q.p, x.p, s2.p, 2, -1.0, z.p, n, kc);      // q = op(x) = x S^2 - Gp x
   colscale_add<T>(st, r.p, b.p, s2.p, 0, -1.0, q.p, n, kc);      // r = b - op(x)
   CK(cudaMemcpyAsync(pv.p, r.p, nc * sizeof(T), cudaMemcpyDeviceToDevice, st));
   coldot<T>(st, b.p, b.p, n, kc, part.p, bb);
   coldot<T>(st, r.p, r.p, n, kc, part.p, rr);
-  auto body = [&]() {
-    op(pv.p, q.p);
-    coldot<T>(st, pv.p, q.p, n, kc, part.p, pq.p);
-    cg_step1_kernel<T><<<egrid((long long)nc), 256, 0, st>>>(x.p, r.p, pv.p, q.p, n, kc, rr, pq.p);
-    KLAUNCHED();
-    coldot<T>(st, r.p, r.p, n, kc, part.p, rn.p);
-    cg_step2_kernel<T><<<egrid((long long)nc), 256, 0, st>>>(pv.p, r.p, n, kc, rr, rn.p);
-    KLAUNCHED();
-    CK(cudaMemcpyAsync(rr, rn.p, kc * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  };
-  GraphPair graphs(st);
+  make_planes<T>(xp, pv.p, kc, n, kc, 3, true, st);
   std::vector<double> h((size_t)2 * kc);
+  CK(cudaMemcpyAsync(h.data(), scal.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  bool done = true;
+  for (int j = 0; j < kc; ++j)
+    if (h[j] > tol * tol * h[kc + j]) done = false;
+  // Iteration i + 1 is enqueued before the host reads whether iteration i has converged; when it has,
+  // the launches of i + 1 find the done word set and leave x as it is.
+  double *hpin = Runtime::get().host_pin;
+  const int nb = (int)std::max<long long>(1, std::min<long long>(kCgBlocks, (n + 15) / 16));
+  const size_t dsm = (size_t)std::max(kCgThreads, kc) * sizeof(double);
+  auto body = [&](int par) {
+    product();
+    cg_apply_kernel<<<nb, kCgThreads, dsm, st>>>(pv.p, z.p, s2.p, q.p, n, kc, part.p, ctl.p, pq.p);
+    KLAUNCHED();
+    cg_update_kernel<<<nb, kCgThreads, dsm, st>>>(x.p, r.p, pv.p, q.p, n, kc, rr, bb, pq.p, beta.p, tol * tol, part.p,
+                                                  ctl.p, hpin + par);
+    KLAUNCHED();
+    cg_next_kernel<<<dim3((unsigned)((n + 63) / 64), (unsigned)((kc + 31) / 32)), 256, 0, st>>>(
+        pv.p, r.p, beta.p, n, kc, ctl.p, xp.buf.p, xp.P.ld, xp.P.plane_stride);
+    KLAUNCHED();
+  };
   int its = 0;
-  for (int it = 0; it < maxit; ++it) {
-    CK(cudaMemcpyAsync(h.data(), scal.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    bool done = true;
-    for (int j = 0; j < kc; ++j)
-      if (h[j] > tol * tol * h[kc + j]) done = false;
-    if (done) break;
-    ++its;
-    if (graphs.usable && it >= 2) graphs.run(0, body);
-    else body();
+  if (!done && maxit > 0) {
+    cudaEvent_t ev[2];
+    for (int e = 0; e < 2; ++e) CK(cudaEventCreateWithFlags(&ev[e], cudaEventDisableTiming));
+    try {
+      hpin[0] = hpin[1] = 0.0;
+      body(1);
+      CK(cudaEventRecord(ev[1], st));
+      for (its = 1;; ++its) {
+        if (its < maxit) {
+          hpin[(its + 1) & 1] = 0.0;
+          body((its + 1) & 1);
+          CK(cudaEventRecord(ev[(its + 1) & 1], st));
+        }
+        CK(cudaEventSynchronize(ev[its & 1]));
+        if (((volatile double *)hpin)[its & 1] != 0.0 || its >= maxit) break;
+      }
+    } catch (...) {
+      for (int e = 0; e < 2; ++e) cudaEventDestroy(ev[e]);
+      throw;
+    }
+    for (int e = 0; e < 2; ++e) cudaEventDestroy(ev[e]);
   }
   if (bv) copy2d<T, T>(x.p + off_r, kc, 1, xv, k, 1, n, k, st);  // gam
   if (bu) {  // lam = (bu + (I - UU') A mu) S^-2
@@ -630,10 +858,17 @@ int svd_adjoint_dev(const StageCtx &c, int m, int n, int k, char ordera, const T
   const char *in_a = getenv("ISVD_GPU_ADJOINT_CG_A");
   const bool gram = A.mixed && n <= m && n % 8 == 0 && (long long)n <= 128LL * k && cg_iters > 0 && (du || dv) &&
                     !(in_a && atoi(in_a) != 0);
-  const int iters = gram ? complement_gram_cg<T>(c, A, k, u, ldu, v, ldv, s, du ? ru.p : nullptr, lam.p,
-                                                 dv ? rv.p : nullptr, gam.p, cg_iters, tol)
-                         : complement_cg<T>(c, A, k, u, ldu, v, ldv, s, du ? ru.p : nullptr, lam.p,
-                                            dv ? rv.p : nullptr, gam.p, cg_iters, tol);
+  int iters = 0;
+  bool solved = false;
+  if constexpr (std::is_same<T, float>::value)
+    if (gram) {
+      iters = complement_gram_cg<T>(c, A, k, u, ldu, v, ldv, s, du ? ru.p : nullptr, lam.p, dv ? rv.p : nullptr,
+                                    gam.p, cg_iters, tol);
+      solved = true;
+    }
+  if (!solved)
+    iters = complement_cg<T>(c, A, k, u, ldu, v, ldv, s, du ? ru.p : nullptr, lam.p, dv ? rv.p : nullptr, gam.p,
+                             cg_iters, tol);
   // w1 = (I - VV') A' Lam  ->  Q1 = V J' + Gam S + w1 ;  w2 = (I - UU') A Gam  ->  P2 = Lam S + w2
   A.mul(true, k, lam.p, w1.p);
   project_out<T>(st, n, k, v, ldv, w1.p, tk.p);
@@ -644,16 +879,18 @@ int svd_adjoint_dev(const StageCtx &c, int m, int n, int k, char ordera, const T
   colscale_add<T>(st, w2.p, lam.p, s, 1, 1.0, w2.p, m, k);
   // dA = U Q1' + P2 V'  (stored per ordera)
   const long long crs = (ordera == 'R') ? ldda : 1, ccs = (ordera == 'R') ? 1 : ldda;
-  {
+  {  // one product [U | P2] [Q1 | V]': dA is written once
+    const long long k2 = 2LL * k;
+    DBuf<T> lhs((size_t)m * k2), rhs((size_t)n * k2);
+    copy2d<T, T>(u, ldu, 1, lhs.p, k2, 1, m, k, st);
+    copy2d<T, T>(w2.p, k, 1, lhs.p + k, k2, 1, m, k, st);
+    copy2d<T, T>(w1.p, k, 1, rhs.p, k2, 1, n, k, st);
+    copy2d<T, T>(v, ldv, 1, rhs.p + k, k2, 1, n, k, st);
     Gemm<T, T> g;
-    g.M = m; g.N = n; g.K = k;
-    g.A = u; g.a_rs = ldu; g.a_cs = 1;
-    g.B = w1.p; g.b_rs = 1; g.b_cs = k;
+    g.M = m; g.N = n; g.K = (int)k2;
+    g.A = lhs.p; g.a_rs = k2; g.a_cs = 1;
+    g.B = rhs.p; g.b_rs = 1; g.b_cs = k2;
     g.C = da; g.c_rs = crs; g.c_cs = ccs;
-    gemm(g, st);
-    g.A = w2.p; g.a_rs = k; g.a_cs = 1;
-    g.B = v; g.b_rs = 1; g.b_cs = ldv;
-    g.beta = 1.0;
     gemm(g, st);
   }
   return iters;

@@ -190,9 +190,7 @@ struct View {
     host = const_cast<T *>(p);
     own.alloc((size_t)((outer - 1) * ld + inner));
     d = own.p;
-    if (copy_in)
-      CK(cudaMemcpy2DAsync(d, ld * sizeof(T), p, ld * sizeof(T), inner * sizeof(T), outer, cudaMemcpyHostToDevice,
-                           st));
+    if (copy_in) copy_to_device(d, ld * sizeof(T), p, ld * sizeof(T), inner * sizeof(T), outer, st);
   }
   // Copy `cols` leading elements of each line back to the host buffer.
   void back(cudaStream_t st, long long cols = -1) {

@@ -59,11 +59,9 @@ void for_each_host_panel(const StageCtx &c, const T *a, long long lda, char orde
       const int b = p & 1;
       if (p >= 2) CK(cudaStreamWaitEvent(rt.copy_stream, consumed[b], 0));
       if (ordera == 'R') {
-        CK(cudaMemcpy2DAsync(stage[b].p, n * sizeof(T), a + r0 * lda, lda * sizeof(T), n * sizeof(T), rows,
-                             cudaMemcpyHostToDevice, rt.copy_stream));
+        copy_to_device(stage[b].p, n * sizeof(T), a + r0 * lda, lda * sizeof(T), n * sizeof(T), rows, rt.copy_stream);
       } else {
-        CK(cudaMemcpy2DAsync(stage[b].p, rows * sizeof(T), a + r0, lda * sizeof(T), rows * sizeof(T), n,
-                             cudaMemcpyHostToDevice, rt.copy_stream));
+        copy_to_device(stage[b].p, rows * sizeof(T), a + r0, lda * sizeof(T), rows * sizeof(T), n, rt.copy_stream);
       }
       CK(cudaEventRecord(copied[b], rt.copy_stream));
       CK(cudaStreamWaitEvent(c.st, copied[b], 0));

@@ -9,6 +9,8 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 extern "C" size_t isvd_gpu_memory_limit;  // include/isvd/gpu/env.h
@@ -73,6 +75,11 @@ void Runtime::reset() {
   cudaStreamSynchronize(g_rt.stream);
   cudaFree(g_rt.ctl);
   cudaFreeHost(g_rt.host_pin);
+  if (g_rt.stage) {
+    cudaStreamSynchronize(g_rt.copy_stream);
+    cudaFreeHost(g_rt.stage);
+    for (cudaEvent_t e : g_rt.stage_ev) cudaEventDestroy(e);
+  }
   cudaStreamDestroy(g_rt.own_stream);
   cudaStreamDestroy(g_rt.copy_stream);
   g_rt = Runtime();
@@ -147,6 +154,92 @@ bool is_device_pointer(const void *p) {
     return false;
   }
   return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+}
+
+namespace {
+
+bool pageable(const void *p) {
+  cudaPointerAttributes attr;
+  if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return attr.type == cudaMemoryTypeUnregistered;
+}
+
+bool stage_ready(Runtime &rt) {
+  if (rt.stage) return true;
+  void *p = nullptr;
+  if (cudaMallocHost(&p, Runtime::kStageSlots * Runtime::kStageBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  for (cudaEvent_t &e : rt.stage_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  rt.stage = static_cast<unsigned char *>(p);
+  return true;
+}
+
+}  // namespace
+
+// The driver copies pageable memory through its own pinned buffer with one thread, about 9 GB/s of the link's
+// 55.  Here each of up to eight threads takes 2 MB pieces in turn: waits until its buffer's last copy is
+// done, fills it, enqueues the copy: a 12007 x 3001 FP32 solve with A in host memory (144 MB) 22.2 -> 9.9 ms.
+// Below 4 MB the threads' start outweighs it.
+void copy_to_device(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, size_t rows,
+                    cudaStream_t st) {
+  if (width == 0 || rows == 0) return;
+  constexpr size_t kBytes = Runtime::kStageBytes;
+  Runtime &rt = Runtime::get();
+  const int threads = std::min<int>(Runtime::kStageSlots / 2, (int)std::thread::hardware_concurrency() / 2);
+  // (cudaStreamPerThread names another stream in each of the threads)
+  if (width * rows < (4u << 20) || threads < 2 || st == cudaStreamPerThread || !pageable(src) || !stage_ready(rt)) {
+    CK(cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, cudaMemcpyHostToDevice, st));
+    return;
+  }
+  if (width == spitch && width == dpitch) {  // contiguous: one long line
+    width *= rows;
+    spitch = dpitch = width;
+    rows = 1;
+  }
+  // pieces: whole lines, or stretches of one line when a line is longer than a buffer
+  const size_t lines = std::max<size_t>(1, kBytes / width);
+  const size_t cut = width > kBytes ? (width + kBytes - 1) / kBytes : 1;
+  const size_t pieces = cut > 1 ? rows * cut : (rows + lines - 1) / lines;
+  std::atomic<size_t> next{0};
+  std::atomic<int> error{(int)cudaSuccess};
+  auto work = [&](int t) {
+    cudaError_t e = cudaSetDevice(rt.device);
+    int turn = 0;
+    for (size_t i; e == cudaSuccess && (i = next.fetch_add(1)) < pieces; turn ^= 1) {
+      const int slot = 2 * t + turn;
+      unsigned char *buf = rt.stage + slot * kBytes;
+      if ((e = cudaEventSynchronize(rt.stage_ev[slot])) != cudaSuccess) break;
+      size_t r0, n, off = 0, w = width;
+      if (cut > 1) {
+        r0 = i / cut; n = 1;
+        off = (i % cut) * kBytes;
+        w = std::min(kBytes, width - off);
+      } else {
+        r0 = i * lines;
+        n = std::min(lines, rows - r0);
+      }
+      const unsigned char *from = static_cast<const unsigned char *>(src) + r0 * spitch + off;
+      for (size_t r = 0; r < n; ++r) memcpy(buf + r * w, from + r * spitch, w);
+      e = cudaMemcpy2DAsync(static_cast<unsigned char *>(dst) + r0 * dpitch + off, dpitch, buf, w, w, n,
+                            cudaMemcpyHostToDevice, st);
+      if (e == cudaSuccess) e = cudaEventRecord(rt.stage_ev[slot], st);
+    }
+    if (e != cudaSuccess) error.store((int)e);
+  };
+  std::vector<std::thread> pool;
+  const int count = (int)std::min<size_t>(threads, pieces);
+  try {
+    for (int t = 1; t < count; ++t) pool.emplace_back(work, t);
+  } catch (const std::system_error &) {  // no more threads: the ones that run take all pieces
+  }
+  work(0);
+  for (std::thread &t : pool) t.join();
+  CK((cudaError_t)error.load());
 }
 
 void sync() { CK(cudaStreamSynchronize(Runtime::get().stream)); }

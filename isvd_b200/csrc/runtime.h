@@ -54,6 +54,12 @@ struct Runtime {
   unsigned int *ctl = nullptr;
   // Pinned host block (64 doubles) for small asynchronous read-backs (iteration errors).
   double *host_pin = nullptr;
+  // Pinned buffers of copy_to_device (kStageSlots x kStageBytes, made on first use) and the event of each
+  // buffer's last copy.  The API lock keeps calls from sharing them.
+  static constexpr int kStageSlots = 16;
+  static constexpr size_t kStageBytes = (size_t)2 << 20;
+  unsigned char *stage = nullptr;
+  cudaEvent_t stage_ev[kStageSlots] = {};
   static Runtime &get();  // initialises on first use (device = current device)
   static bool initialised();
   static void reset();    // releases stream and control block (isvd_Finalize_gpu)
@@ -104,6 +110,12 @@ void DBuf<T>::release() {
 
 // Pointer classification: true when the GPU can dereference `p` directly.
 bool is_device_pointer(const void *p);
+
+// Copy of `rows` lines of `width` bytes from host memory (line stride spitch) to device memory (dpitch),
+// ordered on st; the host memory has been read when it returns.  Pageable memory of several MB goes
+// through pinned buffers filled by several host threads (runtime.cu).
+void copy_to_device(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, size_t rows,
+                    cudaStream_t st);
 
 void sync();  // synchronise the library stream, converting errors into Error
 

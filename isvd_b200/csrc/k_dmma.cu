@@ -124,6 +124,8 @@ __global__ void __launch_bounds__(WM * WN * 32)
   const int wm0 = (warp / WN) * (BM / WM), wn0 = (warp % WN) * (BN / WN);
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   if (g.upper && n0 + BN <= m0) return;  // tile strictly below the diagonal: mirrored by the caller
+  // (128 x 128 tiles) computed on the int8 tensor cores already (k_i8.cu)
+  if (g.done_a && g.done_a[blockIdx.x] * g.done_b[blockIdx.y] <= g.done_lim) return;
   const int b = blockIdx.z / splits, sp = blockIdx.z % splits;
   const int kb = sp * kchunk, ke = min(g.K, kb + kchunk);
 
@@ -338,6 +340,14 @@ void dmma_gemm(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream_t
     dmma_launch<64, 64, 2, 2>(g, a_kc, b_nc, st);
   else
     dmma_launch<128, 128, 2, 4>(g, a_kc, b_nc, st);
+}
+
+void dmma_gemm_rest(const Gemm<double, double> &g, bool a_kc, bool b_nc, const float *done_a, const float *done_b,
+                    float lim, cudaStream_t st) {
+  Gemm<double, double> f = g;
+  f.done_a = done_a; f.done_b = done_b; f.done_lim = lim;
+  f.splits = 1;
+  dmma_launch<128, 128, 2, 4>(f, a_kc, b_nc, st);
 }
 
 int dmma_grouped_bm(int shape) { return shape == 2 ? 128 : shape == 4 ? 32 : 64; }

@@ -270,7 +270,8 @@ void gemm(const Gemm<T, Tout> &g, cudaStream_t st) {
   if (!a_kc && g.a_rs != 1) fail(kErrArgument, "gemm: operand A has no unit stride");
   if (!b_nc && g.b_rs != 1) fail(kErrArgument, "gemm: operand B has no unit stride");
   if constexpr (std::is_same<T, double>::value && std::is_same<Tout, double>::value) {
-    if (dmma_enabled()) {  // FP64 operands: the FP64 tensor-core path (k_dmma.cu)
+    if (dmma_enabled()) {  // FP64 operands: large products on the int8 tensor cores (k_i8.cu), else mma.sync f64
+      if (gemm_f64_int8(g, a_kc, b_nc, st)) return;
       dmma_gemm(g, a_kc, b_nc, st);
       return;
     }

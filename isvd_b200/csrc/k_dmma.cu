@@ -10,6 +10,8 @@
 // staged in the orientation of its unit stride (K-contiguous rows of BK + 4, or MN-contiguous
 // rows of BM + 4 / BN + 4 doubles), which makes both the copies and the fragment reads free of
 // shared-memory bank conflicts.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstdlib>
 
@@ -198,6 +200,73 @@ __global__ void __launch_bounds__(WM * WN * 32)
   }
 }
 
+// Small products: the CTAs of a cluster compute one output tile from a K chunk each, and add their partial
+// tiles through distributed shared memory, CTA `rank` the rows rank, rank + splits, ... in the order of the
+// ranks.  Against partial sums in global memory this saves their round trip and the reduction's launch.
+template <int BM, int BN, int WM, int WN, bool A_KC, bool B_NC>
+__global__ void __launch_bounds__(WM * WN * 32)
+    dmma_cluster_kernel(const Gemm<double, double> g, const int splits, const int kchunk) {
+  constexpr int TM = BM / WM / 8, TN = BN / WN / 8, NT = WM * WN * 32, LD = BN + 2;
+  static_assert(BM * LD <= kStages * DmmaLayout<BM, BN, A_KC, B_NC>::stage, "the tile fits the ring");
+  extern __shared__ double smem[];
+  namespace cg = cooperative_groups;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm0 = (warp / WN) * (BM / WM), wn0 = (warp % WN) * (BN / WN);
+  const int fr = lane >> 2, fc = lane & 3;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+  const int b = blockIdx.z / splits, sp = blockIdx.z % splits;
+  const int kb = min(g.K, sp * kchunk), ke = min(g.K, kb + kchunk);
+  double acc[TM][TN][2];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  dmma_tile<BM, BN, WM, WN, A_KC, B_NC>(smem, g.A + (long long)b * g.a_bs, g.a_rs, g.a_cs, g.B + (long long)b * g.b_bs,
+                                        g.b_rs, g.b_cs, g.M, g.N, kb, ke, m0, n0, acc);
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) smem[(wm0 + 8 * i + fr) * LD + wn0 + 8 * j + 2 * fc + h] = acc[i][j][h];
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  double *__restrict__ C = g.C + (long long)b * g.c_bs;
+  const int mine = (BM - sp + splits - 1) / splits;  // rows sp, sp + splits, ...
+  for (int t = tid; t < mine * BN; t += NT) {
+    const int r = sp + (t / BN) * splits, c = t % BN, gm = m0 + r, gn = n0 + c;
+    if (gm >= g.M || gn >= g.N) continue;
+    double v = 0.0;
+#pragma unroll 8
+    for (int q = 0; q < splits; ++q) v += cl.map_shared_rank(smem, q)[r * LD + c];
+    double *o = C + (long long)gm * g.c_rs + (long long)gn * g.c_cs;
+    v *= g.alpha;
+    if (g.beta != 0.0) v += g.beta * *o;
+    *o = v;
+  }
+  if (g.pl_t && b == g.pl_batch) {  // splits == 1: planes of this tile's transpose, as dmma_gemm_kernel writes them
+    for (int t = tid; t < BN * (BM / 8); t += NT) {
+      const int c = t / (BM / 8), seg = t - c * (BM / 8), gn = n0 + c;
+      if (gn >= g.N) continue;
+      __nv_bfloat16 o[3][8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int r = 8 * seg + e;
+        double v = g.alpha * smem[r * LD + c];
+        __nv_bfloat16 pc[3];
+        split3<double>(v, pc, 3);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) o[q][e] = pc[q];
+      }
+      const long long po = (long long)gn * g.pl_ld + m0 + 8 * seg;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) *(uint4 *)(g.pl_t + q * g.pl_ps + po) = pack8(o[q]);
+    }
+  }
+  cl.sync();  // the peers' reads of this CTA's tile are done
+}
+
 // Grouped products (dmma_grouped): each CTA walks the work items blockIdx.x, blockIdx.x + gridDim.x,
 // ...; a work item is one BM x BN output tile of the product that owns it (binary search on tile0).
 template <int BM, int BN, int WM, int WN, bool A_KC, bool B_NC>
@@ -263,35 +332,34 @@ void dmma_grouped_launch(const GroupedProd *prods, int nprod, int total, cudaStr
   KLAUNCHED();
 }
 
+// K splits of dmma_launch, by a time model: the busiest SM runs ceil(tiles s / SMs) CTAs of BM BN (K / s)
+// FMAs (about 0.23 TFLOP/s per SM on mma.sync f64) plus a fixed 2 us each, and s > 1 adds the partial
+// sums' round trip (s + 1) M N 8 bytes at about 4 TB/s; the smallest s within 3 % of the best, with at
+// least 64 of K per split and at most 512 MB of partials.
+int dmma_splits(const Gemm<double, double> &g, int BM, int BN) {
+  if (g.splits > 0) return g.splits;
+  const int sms = Runtime::get().num_sms;
+  const long long tiles = (long long)((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) * g.batch;
+  const double rate = 0.23e12, fixed = 2e-6, bw = 4e12;
+  const long long mnb = (long long)g.M * g.N * g.batch;
+  auto model = [&](long long s) {
+    const long long per_sm = (tiles * s + sms - 1) / sms;
+    const double kc = (double)((g.K + s - 1) / s);
+    return per_sm * (2.0 * BM * BN * kc / rate + fixed) + (s > 1 ? (double)(s + 1) * mnb * 8.0 / bw : 0.0);
+  };
+  const long long smax = std::max<long long>(
+      1, std::min<long long>({64, (long long)g.K / 64, (512LL << 20) / std::max<long long>(1, mnb * 8)}));
+  double best = model(1);
+  for (long long s = 2; s <= smax; ++s) best = std::min(best, model(s));
+  for (long long s = 1; s <= smax; ++s)
+    if (model(s) <= 1.03 * best) return (int)s;
+  return 1;
+}
+
 template <int BM, int BN, int WM, int WN>
 void dmma_launch(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream_t st) {
-  Runtime &rt = Runtime::get();
   const int gx = (g.M + BM - 1) / BM, gy = (g.N + BN - 1) / BN;
-  const long long tiles = (long long)gx * gy * g.batch;
-  int splits = g.splits;
-  if (splits <= 0) {
-    // split-K by a time model: the busiest SM runs ceil(tiles s / SMs) CTAs of BM BN (K / s) FMAs
-    // (about 0.23 TFLOP/s per SM on mma.sync f64) plus a fixed 2 us each, and s > 1 adds the
-    // partial sums' round trip (s + 1) M N 8 bytes at about 4 TB/s; the smallest s within 3 % of
-    // the best, with at least 64 of K per split and at most 512 MB of partials
-    const double rate = 0.23e12, fixed = 2e-6, bw = 4e12;
-    const long long mnb = (long long)g.M * g.N * g.batch;
-    auto model = [&](long long s) {
-      const long long per_sm = (tiles * s + rt.num_sms - 1) / rt.num_sms;
-      const double kc = (double)((g.K + s - 1) / s);
-      return per_sm * (2.0 * BM * BN * kc / rate + fixed) + (s > 1 ? (double)(s + 1) * mnb * 8.0 / bw : 0.0);
-    };
-    const long long smax = std::max<long long>(
-        1, std::min<long long>({64, (long long)g.K / 64, (512LL << 20) / std::max<long long>(1, mnb * 8)}));
-    double best = model(1);
-    for (long long s = 2; s <= smax; ++s) best = std::min(best, model(s));
-    splits = 1;
-    for (long long s = 1; s <= smax; ++s)
-      if (model(s) <= 1.03 * best) {
-        splits = (int)s;
-        break;
-      }
-  }
+  int splits = dmma_splits(g, BM, BN);
   int kchunk = (g.K + splits - 1) / splits;
   kchunk = ((kchunk + kBK - 1) / kBK) * kBK;
   if (kchunk <= 0) kchunk = kBK;
@@ -316,6 +384,65 @@ void dmma_launch(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream
   if (splits > 1) splitk_reduce(g, splits, part.p, st);
 }
 
+template <int BM, int BN, int WM, int WN>
+void dmma_cluster_launch(const Gemm<double, double> &g, int splits, bool a_kc, bool b_nc, cudaStream_t st) {
+  const int kchunk = ((g.K + splits - 1) / splits + 3) / 4 * 4;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((g.M + BM - 1) / BM, (g.N + BN - 1) / BN, g.batch * splits);
+  cfg.blockDim = dim3(WM * WN * 32);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = splits;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+#define ISVD_DMMA_CASE(AK, BNC)                                                                        \
+  if (a_kc == AK && b_nc == BNC) {                                                                     \
+    auto *k = dmma_cluster_kernel<BM, BN, WM, WN, AK, BNC>;                                            \
+    cfg.dynamicSmemBytes = kStages * DmmaLayout<BM, BN, AK, BNC>::stage * sizeof(double);              \
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes)); \
+    CK(cudaLaunchKernelEx(&cfg, k, g, splits, kchunk));                                                \
+    KLAUNCHED();                                                                                       \
+  }
+  ISVD_DMMA_CASE(true, true)
+  ISVD_DMMA_CASE(true, false)
+  ISVD_DMMA_CASE(false, true)
+  ISVD_DMMA_CASE(false, false)
+#undef ISVD_DMMA_CASE
+}
+
+// Shape of a small product's clusters.  Modelled time of a launch: 5 us, and per 16-deep K slice of a CTA
+// the slice's latency for a CTA alone or, when the busiest SM's CTAs together take longer, their sum
+// (measured: 64 x 64 tiles 1.2 and 0.75 us, 32 x 32 tiles 0.57 and 0.265 us).  The partial tiles' sum costs
+// 0.5 us and their bytes at about 3 TB/s; partials through global memory, 5 us of a second launch and their
+// round trip at about 1 TB/s.  Measured, launches
+// back to back, before and after: 2048 x 128 x 2048 100 -> 55 us, 1536 x 96 x 1536 57 -> 33, 1040 x 65 x
+// 1040 35 -> 19, 256 x 32 x 256 14.4 -> 6.3; 2 x 65 x 65 x 1040 15.7 -> 10.4; 2 x 1536 x 96 x 192 19.6 -> 12.4.
+struct ClusterPlan {
+  int bm = 0, splits = 1;  // bm 0: not by clusters
+};
+ClusterPlan cluster_plan(const Gemm<double, double> &g) {
+  ClusterPlan p;
+  const int sms = Runtime::get().num_sms;
+  const double mb = (double)g.M * g.N * g.batch * 8.0 / 1e6;
+  auto time = [&](int bm, int s) {
+    const double ctas = std::ceil(g.M / (double)bm) * std::ceil(g.N / (double)bm) * g.batch * s;
+    const double slices = std::ceil(g.K / (double)s / kBK);
+    return 5.0 + slices * std::max(bm == 64 ? 1.2 : 0.57, std::ceil(ctas / sms) * (bm == 64 ? 0.75 : 0.265));
+  };
+  const int s0 = dmma_splits(g, 64, 64);
+  double best = time(64, s0) + (s0 > 1 ? 5.0 + (s0 + 1.0) * mb : 0.0);
+  for (int bm = 64; bm >= 32; bm /= 2)
+    for (int s = 1; s <= (g.pl_t ? 1 : 8) && (s == 1 || g.K / s >= kBK); s *= 2)
+      if (const double t = time(bm, s) + (s > 1 ? 0.5 + s * mb / 3 : 0.0); t < 0.97 * best) {
+        best = t;
+        p.bm = bm;
+        p.splits = s;
+      }
+  return p;
+}
+
 }  // namespace
 
 bool dmma_enabled() {
@@ -334,6 +461,11 @@ void dmma_gemm(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream_t
   if (g.pl_t && (g.splits != 1 || g.M % 64 || g.pl_ld % 8 || ((uintptr_t)g.pl_t & 15) || g.pl_ps % 8 ||
                  g.pl_batch < 0 || g.pl_batch >= g.batch))
     fail(kErrArgument, "dmma_gemm: plane output needs splits = 1, M %% 64 == 0 and 16-byte aligned plane rows");
+  if (!g.upper && tiles128 < 2LL * sms && !long_k) {  // few output tiles and a short K: clusters of splits
+    const ClusterPlan p = cluster_plan(g);
+    if (p.bm == 64) return dmma_cluster_launch<64, 64, 2, 2>(g, p.splits, a_kc, b_nc, st);
+    if (p.bm == 32) return dmma_cluster_launch<32, 32, 2, 2>(g, p.splits, a_kc, b_nc, st);
+  }
   // plane output: 64 x 64 tiles (their epilogue stages a tile's transpose through the cp.async
   // ring; without split-K the tile shape does not change the results)
   if (g.pl_t || g.M <= 64 || g.N <= 64 || (tiles128 < 2LL * sms && !long_k))

@@ -307,8 +307,9 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
     return !(e && atoi(e) == 0);
   }();
   bool split_bc = true;  // the first iteration's Bc = G[:, 0:l] is split by the G product
-  // One iteration: W(next) from W(cur).  Iterations are enqueued one ahead of the GPU (below), and the six
-  // launches of one take the host about 35 us against 50 us and more on the GPU; only after
+  // One iteration: W(next) from W(cur).  Iterations are enqueued one ahead of the GPU (below), and the four
+  // launches of one (the products of few tiles by clusters, without reduction launches) take the host about
+  // 25 us against 35 us and more on the GPU; only after
   // kGraphFrom of them is the iteration captured as one CUDA graph per parity of the ping-pong
   // buffers.  Capturing, instantiating and destroying the two graphs costs about 400 us, more than all of
   // a short loop's launches: a 2000 x 1000 solve of 11 iterations takes 1657 us with graphs from the
@@ -330,8 +331,8 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
     {  // [Dc, Dgc] = Bc' [Bc, Bgc] / N   (:181-184), one batched product
       Gemm<double, double> g = gm<double>(l, l, Nl);
       g.batch = 2;
-      // long K (N l >= 2048): 128-deep K chunks per CTA, more splits than the generic split-K
-      // model picks (measured at N l = 4096: 32 splits 157.7 us per iteration against 161.2 with
+      // long K (N l >= 2048) where clusters of at most 8 splits are not faster: 128-deep K chunks
+      // per CTA, more splits than the generic split-K model picks (measured at N l = 4096: 32 splits 157.7 us per iteration against 161.2 with
       // the model's 18; 24: 161.8, 12: 167.6, 6: 187.5); ISVD_GPU_KN_DD_KCHUNK overrides the depth
       if (Nl >= kn_dd_from() && kn_dd_kchunk() > 0) g.splits = std::max(1, Nl / kn_dd_kchunk());
       g.alpha = invN;

@@ -16,6 +16,7 @@
 #include <cstdlib>
 
 #include "kernels.h"
+#include "pdl.cuh"
 #include "planes.cuh"
 #include "runtime.h"
 
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(WM * WN * 32)
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  pdl_wait();
   dmma_tile<BM, BN, WM, WN, A_KC, B_NC>(smem, g.A + (long long)b * g.a_bs, g.a_rs, g.a_cs, g.B + (long long)b * g.b_bs,
                                         g.b_rs, g.b_cs, g.M, g.N, kb, ke, m0, n0, acc);
   __syncthreads();
@@ -230,6 +232,7 @@ __global__ void __launch_bounds__(WM * WN * 32)
     for (int j = 0; j < TN; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) smem[(wm0 + 8 * i + fr) * LD + wn0 + 8 * j + 2 * fc + h] = acc[i][j][h];
+  pdl_trigger();  // not earlier: CTAs of the next kernel placed around this one's would be spread unevenly
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
   double *__restrict__ C = g.C + (long long)b * g.c_bs;
@@ -391,12 +394,17 @@ void dmma_cluster_launch(const Gemm<double, double> &g, int splits, bool a_kc, b
   cfg.gridDim = dim3((g.M + BM - 1) / BM, (g.N + BN - 1) / BN, g.batch * splits);
   cfg.blockDim = dim3(WM * WN * 32);
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1] = pdl_attribute();
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = splits;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  // CTAs that start beside those of the kernel before are spread unevenly over the SMs, so only launches
+  // that leave SMs idle anyway, of the small tiles, whose time is latency (2048 x 128 x 2048, 256 CTAs of
+  // 64 x 64: 52 us after the kernel before, 102 us beside its end)
+  const bool pdl = BM <= 32 && (long long)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z <= Runtime::get().num_sms;
+  cfg.numAttrs = pdl ? 2 : 1;
 #define ISVD_DMMA_CASE(AK, BNC)                                                                        \
   if (a_kc == AK && b_nc == BNC) {                                                                     \
     auto *k = dmma_cluster_kernel<BM, BN, WM, WN, AK, BNC>;                                            \

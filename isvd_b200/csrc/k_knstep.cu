@@ -37,6 +37,7 @@
 
 #include "kernels.h"
 #include "kn_common.cuh"
+#include "pdl.cuh"
 #include "rows.cuh"
 #include "runtime.h"
 
@@ -614,6 +615,7 @@ __device__ __forceinline__ void kn_rows_body(const KnStep &a, const KnSeries &se
       }
     }
   });
+  pdl_trigger();  // the next product is placed on the SMs now
   const double err = sqrt(kr_cluster_sum(k, cluster, e2, slots + 32, red));
   if (k.rank == 0 && tid == 0) {
     *a.err = err;
@@ -622,6 +624,7 @@ __device__ __forceinline__ void kn_rows_body(const KnStep &a, const KnSeries &se
 }
 
 __global__ void __launch_bounds__(kKrThreads, 1) kn_rows_kernel(KnStep a, KnSeries ser, int blocks) {
+  pdl_wait();
   kn_rows_body(a, ser, blocks);
 }
 
@@ -712,7 +715,7 @@ int kr_cluster(int l, int want) {
 }
 
 template <class Kern, class Arg>
-void kr_launch(Kern kern, int cs, int grid, int l, cudaStream_t st, Arg a, const KnSeries &series) {
+void kr_launch(Kern kern, int cs, int grid, int l, bool pdl, cudaStream_t st, Arg a, const KnSeries &series) {
   const int blocks = kr_blocks(l, cs);
   const int bytes = (int)kr_bytes(l, cs, blocks);
   cudaLaunchConfig_t cfg = {};
@@ -720,13 +723,14 @@ void kr_launch(Kern kern, int cs, int grid, int l, cudaStream_t st, Arg a, const
   cfg.blockDim = dim3(kKrThreads);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1] = pdl_attribute();
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = cs;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl ? 2 : 1;  // pdl: the kernel calls pdl_wait()
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   CK(cudaLaunchKernelEx(&cfg, kern, a, series, blocks));
@@ -768,14 +772,14 @@ void kn_step_grouped(const KnStep *steps, int count, int max_l, int cluster, cud
   const int cs = kr_usable() ? kr_cluster(max_l, cluster > 0 ? cluster : 8) : 0;
   if (cs == 0) fail(kErrUnsupported, "grouped Kolmogorov-Nagumo step: no thread-block cluster launch on this device");
   static const KnSeries series = make_series();
-  kr_launch(kn_rows_grouped_kernel, cs, count * cs, max_l, st, steps, series);
+  kr_launch(kn_rows_grouped_kernel, cs, count * cs, max_l, false, st, steps, series);
 }
 
 void kn_step(const KnStep &a, cudaStream_t st) {
   if (a.l > kKsMaxL) fail(kErrUnsupported, "Kolmogorov-Nagumo step: l = %d > %d", a.l, kKsMaxL);
   static const KnSeries series = make_series();
   if (const int rc = kr_usable() ? kr_cluster(a.l, 16) : 0) {
-    kr_launch(kn_rows_kernel, rc, rc, a.l, st, a, series);
+    kr_launch(kn_rows_kernel, rc, rc, a.l, true, st, a, series);
     return;
   }
   const int cs = choose_cluster_size(a, st);

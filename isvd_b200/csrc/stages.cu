@@ -331,9 +331,10 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
     {  // [Dc, Dgc] = Bc' [Bc, Bgc] / N   (:181-184), one batched product
       Gemm<double, double> g = gm<double>(l, l, Nl);
       g.batch = 2;
-      // long K (N l >= 2048) where clusters of at most 8 splits are not faster: 128-deep K chunks
-      // per CTA, more splits than the generic split-K model picks (measured at N l = 4096: 32 splits 157.7 us per iteration against 161.2 with
-      // the model's 18; 24: 161.8, 12: 167.6, 6: 187.5); ISVD_GPU_KN_DD_KCHUNK overrides the depth
+      // long K (N l >= 2048) where clusters of at most 8 splits are not faster: 128-deep K chunks per
+      // CTA, more splits than the generic split-K model picks (measured at N l = 4096: 32 splits
+      // 157.7 us per iteration against 161.2 with the model's 18; 24: 161.8, 12: 167.6, 6: 187.5);
+      // ISVD_GPU_KN_DD_KCHUNK overrides the depth
       if (Nl >= kn_dd_from() && kn_dd_kchunk() > 0) g.splits = std::max(1, Nl / kn_dd_kchunk());
       g.alpha = invN;
       g.A = Bc; g.a_rs = 1; g.a_cs = lw; g.a_bs = 0;

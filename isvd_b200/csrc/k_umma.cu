@@ -30,6 +30,7 @@ namespace {
 constexpr int BM = 128;
 constexpr int kThreads = 320;
 constexpr int kEpiWarps = 8;
+constexpr int kStage32 = 32 * 33;  // floats of an epilogue warp's staging area (KParams::stage32)
 constexpr int kChunkK = 128;  // K depth of one tensor-memory accumulation chunk
 
 struct KParams {
@@ -51,6 +52,7 @@ struct KParams {
   int unbias;     // chunks of one k-block, the leading plane pair last: see UmmaGemm::unbias
   int stage_out;  // epilogue stages its rows through shared memory (C rows contiguous)
   int bloop;      // one CTA runs every batch of its tile in turn (grid z = 1, no split-K)
+  int stage32;    // batch loop, value output: rows through a staging area of its own, 32 columns at a time
   int vec_out;    // direct epilogue stores as 16-byte vectors (C rows contiguous and aligned)
   __nv_bfloat16 *pl;  // optional bf16 planes of the output (UmmaGemm::planes)
   long long pl_ld, pl_ps;
@@ -364,6 +366,26 @@ __global__ void __launch_bounds__(kThreads, 1)
             p.partial[(((long long)b * p.splits + split) * p.M + gr) * p.N + gn] = v;
           }
         }
+      }
+    } else if (BN <= 128 && ok && p.stage32) {
+      // the pipeline buffers already take the next batch's loads, so whole rows go through an area behind
+      // them (30011 x 65 blocks, whose odd rows take no vector stores: 432 -> 238 us for 16 of them)
+      float *stg = (float *)(smem + (size_t)stages * stage_bytes + 256) + (warp - 2) * kStage32;
+#pragma unroll
+      for (int t = 0; t < C::HALF / 32; ++t) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) stg[lane * 33 + j] = acc[t * 32 + j];
+        __syncwarp();
+        const int gn = n0 + h * C::HALF + t * 32 + lane;
+        const int nr = gn < p.N ? min(32, p.M - (m0 + q * 32)) : 0;
+        const long long off = (long long)b * p.c_step + (long long)(m0 + q * 32) * p.c_rs + gn;
+#pragma unroll 8
+        for (int r = 0; r < nr; ++r) {
+          const double v = p.alpha * (double)stg[r * 33 + lane];
+          if (p.c_double) ((double *)p.C)[off + r * p.c_rs] = v;
+          else ((float *)p.C)[off + r * p.c_rs] = (float)v;
+        }
+        __syncwarp();
       }
     } else if (BN <= 128 && ok && gm < p.M && p.vec_out && p.splits == 1) {
       // this thread's row: 16-byte stores of 4 (FP32) or 2 (FP64) consecutive columns
@@ -1026,21 +1048,25 @@ void launch_t(const UmmaGemm &g, cudaStream_t st, int *status) {
   CUtensorMap mb = BMN ? make_map(g.B, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B) : make_map(g.B, BK, BN, swa);
   const int stage_bytes = g.A.np * C::A_TILE + g.B.np * C::B_TILE;
   const int budget = (int)rt.smem_optin - 1024 - 256;
-  int stages = std::min(8, budget / stage_bytes);
+  // many short batches (e.g. N block products of K = l): one CTA per tile runs all of them in turn,
+  // each one accumulation segment, instead of one CTA per (tile, batch) that would mostly set up
+  p.bloop = (BN <= 128 && g.batch > 1 && p.splits == 1 && p.total_kb <= 16) ? 1 : 0;
+  p.vec_out = (BN <= 128 && g.c_cs == 1 && !g.upper && g.N % 4 == 0 && g.c_rs % 4 == 0 && g.c_step % 4 == 0 &&
+               (!g.planes || (g.N % 8 == 0 && g.p_ld % 8 == 0 && g.c_step % 8 == 0 && ((uintptr_t)g.planes % 16) == 0)) &&
+               ((uintptr_t)g.C % 16) == 0) ? 1 : 0;
+  constexpr int stage32_bytes = kEpiWarps * kStage32 * (int)sizeof(float);
+  p.stage32 = (p.bloop && !p.vec_out && g.C && !g.planes && g.c_cs == 1 && !g.upper && C::HALF >= 32 &&
+               (budget - stage32_bytes) / stage_bytes >= 2) ? 1 : 0;
+  const int staging = p.stage32 ? stage32_bytes : 0;
+  int stages = std::min(8, (budget - staging) / stage_bytes);
   p.chunk_kb = g.unbias ? 1 : chunk_kblocks(BK, g.chunk_k);
   p.unbias = g.unbias ? 1 : 0;
   // rows of C contiguous (or a split-K partial): stage the epilogue through shared memory when the
   // pipeline buffers can hold the 8 warps' 32 x (BN/2 + 1) blocks
-  // many short batches (e.g. N block products of K = l): one CTA per tile runs all of them in turn,
-  // each one accumulation segment, instead of one CTA per (tile, batch) that would mostly set up
-  p.bloop = (BN <= 128 && g.batch > 1 && p.splits == 1 && p.total_kb <= 16) ? 1 : 0;
   p.stage_out = (!p.bloop && (p.splits > 1 || g.c_cs == 1) && stages * stage_bytes >= 8 * 32 * (C::HALF + 1) * 4) ? 1 : 0;
   if (g.planes_in_place && !p.bloop) fail(kErrUnsupported, "tcgen05 GEMM: in-place plane output needs the batch loop");
-  p.vec_out = (BN <= 128 && g.c_cs == 1 && !g.upper && g.N % 4 == 0 && g.c_rs % 4 == 0 && g.c_step % 4 == 0 &&
-               (!g.planes || (g.N % 8 == 0 && g.p_ld % 8 == 0 && g.c_step % 8 == 0 && ((uintptr_t)g.planes % 16) == 0)) &&
-               ((uintptr_t)g.C % 16) == 0) ? 1 : 0;
   if (stages < 2) fail(kErrUnsupported, "tcgen05 GEMM: %d planes do not fit in shared memory", g.A.np + g.B.np);
-  const size_t smem = (size_t)stages * stage_bytes + 1024 + 256;
+  const size_t smem = (size_t)stages * stage_bytes + 1024 + 256 + staging;
   static_assert(kThreads == 64 + 32 * kEpiWarps, "warp roles");
   auto kern = umma_gemm_kernel<BN, BK, AMN, BMN>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -856,8 +856,71 @@ __global__ void split_kernel(const T *__restrict__ src, long long s_rs, long lon
 #pragma unroll
       for (int q = 0; q < 3; ++q) o[q][i] = t[q];
     }
-    for (int q = 0; q < np; ++q) *(uint4 *)(dst + q * ps + r * ld + c0) = pack8(o[q]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)  // unrolled: a loop to np would index the pieces in local memory
+      if (q < np) *(uint4 *)(dst + q * ps + r * ld + c0) = pack8(o[q]);
   }
+}
+
+// The same for FP32 rows with unit column stride and 16-byte aligned starts, two rows per step: without the
+// general form's strides and scalar path it needs half the registers, and twice the threads are in flight.
+// 13334 x 20000 values to two planes: 763 -> 314 us (6.8 TB/s); to three planes 5.6 -> 6.8 TB/s.
+template <int NP>
+__global__ void __launch_bounds__(256, 6)
+    split_vec_kernel(const float *__restrict__ src, long long s_rs, int rows, int cols, int rows_pad,
+                     __nv_bfloat16 *__restrict__ dst, int ld, long long ps) {
+  const int c0 = 8 * (blockIdx.x * 256 + threadIdx.x);
+  if (c0 >= ld) return;
+  for (int r0 = 2 * blockIdx.y; r0 < rows_pad; r0 += 2 * gridDim.y) {
+    float4 x[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      x[i][0] = x[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float *row = src + (r0 + i) * s_rs;
+      if (r0 + i < rows && c0 + 8 <= cols) {
+        x[i][0] = __ldg((const float4 *)(row + c0));
+        x[i][1] = __ldg((const float4 *)(row + c0) + 1);
+      } else if (r0 + i < rows && c0 < cols) {
+        float t[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) t[e] = c0 + e < cols ? row[c0 + e] : 0.f;
+        x[i][0] = make_float4(t[0], t[1], t[2], t[3]);
+        x[i][1] = make_float4(t[4], t[5], t[6], t[7]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (r0 + i >= rows_pad) break;
+      const float t[8] = {x[i][0].x, x[i][0].y, x[i][0].z, x[i][0].w, x[i][1].x, x[i][1].y, x[i][1].z, x[i][1].w};
+      __nv_bfloat16 o[3][8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        __nv_bfloat16 pc[3];
+        split3f(t[e], pc);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) o[q][e] = pc[q];
+      }
+#pragma unroll
+      for (int q = 0; q < NP; ++q) *(uint4 *)(dst + q * ps + (long long)(r0 + i) * ld + c0) = pack8(o[q]);
+    }
+  }
+}
+
+template <class T>
+void launch_split(const T *src, long long s_rs, long long s_cs, long long rows, long long cols, long long rows_pad, int np,
+                  __nv_bfloat16 *dst, long long ld, long long ps, cudaStream_t st) {
+  const unsigned gx = (unsigned)((ld / 8 + 255) / 256);
+  if constexpr (std::is_same<T, float>::value)
+    if (s_cs == 1 && s_rs % 4 == 0 && ((uintptr_t)src & 15) == 0 && rows_pad < (1LL << 31) && ld < (1LL << 31) && np <= 3) {
+      const dim3 grid(gx, (unsigned)std::max<long long>(1, std::min<long long>((rows_pad + 1) / 2, 65535)));
+      auto *k = np == 1 ? split_vec_kernel<1> : np == 2 ? split_vec_kernel<2> : split_vec_kernel<3>;
+      k<<<grid, 256, 0, st>>>(src, s_rs, (int)rows, (int)cols, (int)rows_pad, dst, (int)ld, ps);
+      KLAUNCHED();
+      return;
+    }
+  const dim3 grid(gx, (unsigned)std::min<long long>(std::max(rows_pad, 1LL), 65535));
+  split_kernel<T><<<grid, 256, 0, st>>>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, ps);
+  KLAUNCHED();
 }
 
 // Transposed: plane(c, r) = piece(src(r, c)) through a 64 (r) x 32 (c) shared tile; each thread
@@ -882,11 +945,14 @@ __global__ void split_t_kernel(const T *__restrict__ src, long long s_rs, long l
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       __nv_bfloat16 t[3];
-      split3<T>(tile[8 * seg + i][cl], t, 3);
+      if (sizeof(T) == 4) split3f((float)tile[8 * seg + i][cl], t);
+      else split3<T>(tile[8 * seg + i][cl], t, 3);
 #pragma unroll
       for (int q = 0; q < 3; ++q) o[q][i] = t[q];
     }
-    for (int q = 0; q < np; ++q) *(uint4 *)(dst + q * ps + c * ld + rr) = pack8(o[q]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (q < np) *(uint4 *)(dst + q * ps + c * ld + rr) = pack8(o[q]);
   }
 }
 
@@ -1173,9 +1239,7 @@ void split_planes(const T *src, long long s_rs, long long s_cs, long long rows, 
   if (rows_pad < out_rows || ld < (transpose ? rows : cols)) fail(kErrArgument, "split_planes: plane too small");
   if (!transpose) {
     if (ld % 8) fail(kErrArgument, "split_planes: ld must be a multiple of 8");
-    const dim3 grid((unsigned)((ld / 8 + 255) / 256), (unsigned)std::min<long long>(rows_pad, 65535));
-    split_kernel<T><<<grid, 256, 0, st>>>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, plane_stride);
-    KLAUNCHED();
+    launch_split<T>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, plane_stride, st);
   } else {
     // zero the padding (rows beyond cols, columns beyond rows), then transpose-split
     for (int q = 0; q < np; ++q) {
@@ -1199,9 +1263,7 @@ void split_rows(const T *src, long long s_rs, long long s_cs, long long rows, lo
   if (ld % 8) fail(kErrArgument, "split_rows: ld must be a multiple of 8");
   if (!transpose) {
     if (ld < cols) fail(kErrArgument, "split_rows: plane too narrow");
-    const dim3 grid((unsigned)((ld / 8 + 255) / 256), (unsigned)std::min<long long>(std::max(rows, 1LL), 65535));
-    split_kernel<T><<<grid, 256, 0, st>>>(src, s_rs, s_cs, rows, cols, rows, np, dst, ld, plane_stride);
-    KLAUNCHED();
+    launch_split<T>(src, s_rs, s_cs, rows, cols, rows, np, dst, ld, plane_stride, st);
   } else {
     // output rows = cols of src, output columns = rows of src; the grid covers ld when
     // ld == roundup(rows, 64)

@@ -358,10 +358,11 @@ __global__ void __launch_bounds__(256) osj_kernel(int n_uniform, const double *_
 }
 
 // One cluster per matrix: the FP64 refinement on the rows of X' (row i = eigenvector i), then the
-// eigenpairs in order (as sym_eig_batched).
+// eigenpairs in order (as sym_eig_batched).  loose: eigenvectors that are not separated stay mixed, as
+// orthonormal as the others.
 __global__ void __launch_bounds__(kKrThreads, 1)
     eig_refine_kernel(int n_uniform, double *workg, size_t work_stride, double *__restrict__ Vg,
-                      double *__restrict__ wg, int order, bool absval, const EigDesc *desc) {
+                      double *__restrict__ wg, int order, bool absval, bool loose, const EigDesc *desc) {
   extern __shared__ double sm[];
   __shared__ double red[kKrWarps], lam[kMaxN];
   __shared__ int sbad;
@@ -430,7 +431,7 @@ __global__ void __launch_bounds__(kKrThreads, 1)
           v = q;
           m = fabs(q);
         } else {
-          bad = 1;  // not separated, and coupled above rounding (or not a number)
+          bad = !loose;  // not separated, and coupled above rounding (or not a number)
         }
       }
       R[e] = v;
@@ -541,7 +542,7 @@ bool eig_refined_usable(int n) {
 }
 
 void eig_refined(int n, int count, const double *A, double *work, double *V, double *w, int order, bool absval,
-                 const EigDesc *desc, cudaStream_t st) {
+                 const EigDesc *desc, cudaStream_t st, bool loose) {
   const size_t stride = eig_work_doubles(n);
   const size_t osm = osj_smem(n);
   with_epl(n, [&](auto kern) {
@@ -565,7 +566,7 @@ void eig_refined(int n, int count, const double *A, double *work, double *V, dou
   cfg.numAttrs = 1;
   CK(cudaFuncSetAttribute(eig_refine_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   CK(cudaFuncSetAttribute(eig_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  CK(cudaLaunchKernelEx(&cfg, eig_refine_kernel, n, work, stride, V, w, order, absval, desc));
+  CK(cudaLaunchKernelEx(&cfg, eig_refine_kernel, n, work, stride, V, w, order, absval, loose, desc));
   KLAUNCHED();
 }
 

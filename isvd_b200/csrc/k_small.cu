@@ -234,10 +234,18 @@ __global__ void __launch_bounds__(NT)
 // output stores them) it was bound by those accesses instead: 1.8 ms against 0.4 ms for n = 48.
 constexpr int kSvdLanes = 16;
 
+// Start of the rotations: orthogonal V0 (row-major) and X0 = B V0, the identity and B where matrix b's word
+// need[b stride] is set.
+struct SvdStart {
+  const double *V0 = nullptr, *X0 = nullptr;
+  const double *need = nullptr;
+  size_t stride = 0;
+};
+
 template <bool VS, int EPL>
 __global__ void __launch_bounds__(1024)
     svd_jacobi_kernel(int n, const double *__restrict__ Bg, double *__restrict__ Ug, double *__restrict__ sg,
-                      double *__restrict__ Vg, double *__restrict__ scratch, int *status) {
+                      double *__restrict__ Vg, double *__restrict__ scratch, SvdStart start, int *status) {
   extern __shared__ double sm[];
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
@@ -253,12 +261,14 @@ __global__ void __launch_bounds__(1024)
 
   __shared__ double red[32];
   double fr = 0.0;
+  const bool warm = start.V0 && *(const int *)(start.need + b * start.stride) == 0;
+  const double *X0 = warm ? start.X0 + (size_t)b * n * n : B0, *V0 = warm ? start.V0 + (size_t)b * n * n : nullptr;
   for (int e = tid; e < n * n; e += nt) {
     const int i = e / n, j = e - i * n;
-    const double v = B0[e];
+    const double v = X0[e];
     X[j * n + i] = v;
     fr += v * v;
-    Vt[e] = (i == j) ? 1.0 : 0.0;
+    Vt[j * n + i] = V0 ? V0[e] : (i == j) ? 1.0 : 0.0;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) fr += __shfl_xor_sync(0xffffffffu, fr, o);
@@ -341,6 +351,40 @@ __global__ void __launch_bounds__(1024)
     const double sj = nrm[j];
     U[e] = X[j * n + i] * (sj > 0.0 ? 1.0 / sj : 0.0);
     V[e] = Vt[j * n + i];
+  }
+}
+
+// W = 4^-e B'B with 2^e the largest entry's exponent, the identity for a zero or non-finite B.  One CTA per
+// matrix.
+__global__ void __launch_bounds__(1024) svd_gram_kernel(int n, const double *__restrict__ Bg, double *__restrict__ Wg) {
+  extern __shared__ double sm[];  // n rows of n + 1
+  __shared__ double red[32];
+  const double *B = Bg + (size_t)blockIdx.x * n * n;
+  double *W = Wg + (size_t)blockIdx.x * n * n;
+  const int tid = threadIdx.x, nt = blockDim.x, ld = n + 1;
+  double mx = 0.0;
+  bool bad = false;
+  for (int e = tid; e < n * n; e += nt) {
+    const double v = B[e];
+    sm[e / n * ld + e % n] = v;
+    mx = fmax(mx, fabs(v));
+    bad |= !(fabs(v) <= 1.7976931348623157e308);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) red[tid >> 5] = mx;
+  bad = __syncthreads_or(bad);
+  mx = 0.0;
+  for (int i = 0; i < nt / 32; ++i) mx = fmax(mx, red[i]);
+  bad = bad || mx == 0.0;
+  int e = 0;
+  if (!bad) frexp(mx, &e);
+  const double h = ldexp(1.0, -(e / 2)), h2 = ldexp(1.0, -(e - e / 2));
+  for (int t = tid; t < n * n; t += nt) {
+    const int i = t / n, j = t - i * n;
+    double v = 0.0;
+    for (int k = 0; k < n; ++k) v = fma(sm[k * ld + i] * h * h2, sm[k * ld + j] * h * h2, v);
+    W[t] = bad ? (i == j ? 1.0 : 0.0) : v;
   }
 }
 
@@ -980,7 +1024,7 @@ void sym_eig_grouped(const EigDesc *desc, int count, int max_n, int order, bool 
   else go(sym_eig_kernel<true, kEigThreads>, kEigThreads);
 }
 
-void svd_jacobi_batched(int n, int batch, const double *B, double *U, double *s, double *V, int *status,
+void svd_jacobi_batched(int n, int batch, const double *B, double *U, double *s, double *V, bool from_gram, int *status,
                         cudaStream_t st) {
   if (n <= 0 || batch <= 0) return;
   Runtime &rt = Runtime::get();
@@ -990,9 +1034,31 @@ void svd_jacobi_batched(int n, int batch, const double *B, double *U, double *s,
   const int threads = std::max(64, std::min(1024, ((n + 1) / 2 * kSvdLanes + 31) / 32 * 32));
   DBuf<double> scratch;
   if (!vs) scratch.alloc((size_t)batch * n * n);
+  // Start from the eigenvectors of B'B (FP32 Jacobi with FP64 refinement, k_eig.cu): B V0 has orthogonal
+  // columns up to rounding relative to ||B||, so that one or two sweeps of the seven to nine are left.  From
+  // n = 32 on, where a sweep costs more than the launches (n = 48: 450 -> 190 us in all).
+  SvdStart start;
+  DBuf<double> W, V0, X0, w0, work;
+  if (from_gram && n >= 32 && n <= 128 && eig_refined_usable(n)) {
+    const size_t nn = (size_t)n * n, gsm = (size_t)n * (n + 1) * sizeof(double);
+    W.alloc(batch * nn); V0.alloc(batch * nn); X0.alloc(batch * nn); w0.alloc((size_t)batch * n);
+    work.alloc(batch * eig_work_doubles(n));
+    CK(cudaFuncSetAttribute(svd_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm));
+    svd_gram_kernel<<<batch, 1024, gsm, st>>>(n, B, W.p);
+    KLAUNCHED();
+    eig_refined(n, batch, W.p, work.p, V0.p, w0.p, +1, true, nullptr, st, true);
+    Gemm<double, double> g;
+    g.M = g.N = g.K = n; g.batch = batch;
+    g.A = B; g.a_rs = n; g.a_cs = 1; g.a_bs = (long long)nn;
+    g.B = V0.p; g.b_rs = n; g.b_cs = 1; g.b_bs = (long long)nn;
+    g.C = X0.p; g.c_rs = n; g.c_cs = 1; g.c_bs = (long long)nn;
+    gemm(g, st);
+    start.V0 = V0.p; start.X0 = X0.p;
+    start.need = work.p + eig_need_at(n); start.stride = eig_work_doubles(n);
+  }
   auto go = [&](auto kernel) {
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<batch, threads, smem, st>>>(n, B, U, s, V, scratch.p, status);
+    kernel<<<batch, threads, smem, st>>>(n, B, U, s, V, scratch.p, start, status);
     KLAUNCHED();
   };
   if (!vs) go(svd_jacobi_kernel<false, 11>);

@@ -130,8 +130,9 @@ struct EigDesc {  // one matrix of a grouped eigensolve: n x n row-major A -> V 
 size_t eig_work_doubles(int n);
 __host__ __device__ constexpr size_t eig_need_at(int n) { return 4 * (size_t)n * n + n + 49; }
 bool eig_refined_usable(int n);
+// loose: an orthogonal V that diagonalises A up to FP32 rounding within clusters will do.
 void eig_refined(int n, int count, const double *A, double *work, double *V, double *w, int order, bool absval,
-                 const EigDesc *desc, cudaStream_t st);
+                 const EigDesc *desc, cudaStream_t st, bool loose = false);
 // As sym_eig_batched for count matrices of different sizes (desc in device memory; max_n >= every n).
 void sym_eig_grouped(const EigDesc *desc, int count, int max_n, int order, bool absval, int *status,
                      cudaStream_t st);
@@ -139,8 +140,9 @@ void sym_eig_batched(int n, int batch, const double *A, double *V, double *w, in
                      int *status, cudaStream_t st);
 
 // Batched general SVD B = U diag(s) V' by one-sided Jacobi, one CTA per matrix.
-// B, U, V: batch x (n x n) row-major; s descending.
-void svd_jacobi_batched(int n, int batch, const double *B, double *U, double *s, double *V, int *status,
+// B, U, V: batch x (n x n) row-major; s descending.  from_gram: start from the eigenvectors of B'B, for
+// callers to whom singular values are exact to rounding relative to ||B||.
+void svd_jacobi_batched(int n, int batch, const double *B, double *U, double *s, double *V, bool from_gram, int *status,
                         cudaStream_t st);
 
 // Kolmogorov-Nagumo l x l step (reference core/stage/@x@_integrate_kolmogorov_nagumo.c:180-234):

@@ -442,7 +442,7 @@ void integrate_hr_dev(const StageCtx &c, int m, int l, int N, T *qs, long long l
     }
     allreduce_sum(Bs.p, (size_t)h * ll, c.st);  // row blocks on several ranks: a sum (:100)
     // svd(B(i)) = W S T' (the same B on every rank: the same factors)
-    svd_jacobi_batched(l, h, Bs.p, W.p, s.p, Vv.p, c.status, c.st);
+    svd_jacobi_batched(l, h, Bs.p, W.p, s.p, Vv.p, true, c.status, c.st);
     // Q(i) := (Q(i) W + Q(i+h) T) / sqrt(2 (1 + s))
     scale_cols_batched<double, T>(W.p, l, Wt.p, l, (long long)h * l, l, l, s.p, kScaleHr, c.st);
     scale_cols_batched<double, T>(Vv.p, l, Tt.p, l, (long long)h * l, l, l, s.p, kScaleHr, c.st);

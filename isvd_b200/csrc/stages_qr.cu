@@ -411,7 +411,7 @@ void post_tsqr_dev(const StageCtx &c, int m, int n, int k, int l, char ordera, c
     gemm(g, c.st);
   }
   copy2d<double, double>(R.p, 1, l, L.p, l, 1, l, l, c.st);  // L = R'
-  svd_jacobi_batched(l, 1, L.p, Ul.p, sv.p, Vl.p, c.status, c.st);
+  svd_jacobi_batched(l, 1, L.p, Ul.p, sv.p, Vl.p, false, c.status, c.st);
   copy2d<double, T>(sv.p, 1, 1, s, 1, 1, l, 1, c.st);
   if (wu) {  // U = Qbar V_L[:, 0:k]
     DBuf<T> Vt(ll);

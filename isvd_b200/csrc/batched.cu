@@ -436,6 +436,7 @@ struct Plan : BatchPlan {
   bool bound = false;
   int solves = 0;
   // work lists
+  std::vector<int> own_sketch, own_gfull;  // matrices whose sketch / Qs'Qs are products of their own
   GemmList<T, T> sketch, apply, qbar_l, proj, ul, vl;
   GemmList<T, double> gram, gfull, wzl;
   GemmList<double, double> l1, l2, l4;
@@ -476,27 +477,46 @@ struct Plan : BatchPlan {
   }
 };
 
+// Whether a matrix's sketch, or its Qs'Qs (gram), is large enough for a product of its own on the tensor
+// cores (bf16 planes for FP32, int8 digits for FP64) in place of a share of the grouped product: there the
+// CUDA cores make about 33 TFLOP/s of FP32 sketches and 14 of Grams.  A product of its own costs two or
+// three launches of 5 to 20 us, which fewer than 2 GFLOP of a sketch or 0.8 of a Gram do not repay.  Measured
+// for 64 matrices of 512 to 8192 by 256 to 4096, l 12 to 96, N = 8: 19.3 -> 18.7 ms.
+template <class T>
+bool own_product(double M, double N, double K, bool gram) {
+  const double flops = (gram ? 1.1 : 2.0) * M * N * K;
+  if (std::is_same<T, float>::value) return flops >= (gram ? 0.8e9 : 2e9) && f32_planes_pay(M, N, K, gram);
+  return flops >= 2e9 && f64_int8_pays(M, N, K, gram);
+}
+
 template <class T>
 void build_lists(Plan<T> &P, cudaStream_t st) {
   const int B = P.count, N = P.N;
   P.sketch.clear(); P.apply.clear(); P.qbar_l.clear(); P.proj.clear(); P.ul.clear(); P.vl.clear();
   P.gram.clear(); P.gfull.clear(); P.wzl.clear();
   P.m_x.host.clear(); P.m_s.host.clear(); P.m_mirror.host.clear(); P.m_wk.host.clear(); P.m_vk.host.clear(); P.m_init.host.clear();
+  P.own_sketch.clear(); P.own_gfull.clear();
   std::vector<CholDesc> c1;
   std::vector<EigDesc> e2;
   for (int b = 0; b < B; ++b) {
     auto &M = *P.mats[b];
     const int m = P.m[b], n = P.n[b], k = P.k[b], l = P.l[b], Nl = P.Nl[b];
     const size_t ll = (size_t)l * l;
-    P.sketch.host.push_back(prod(m, Nl, n, P.a[b], P.lda[b], 1, M.om.p, Nl, 1, M.y.p, Nl, 1));
+    if (own_product<T>(m, Nl, n, false)) P.own_sketch.push_back(b);
+    else P.sketch.host.push_back(prod(m, Nl, n, P.a[b], P.lda[b], 1, M.om.p, Nl, 1, M.y.p, Nl, 1));
     for (int i = 0; i < N; ++i) {
       P.gram.host.push_back(prod(l, l, m, M.y.p + i * l, 1, Nl, M.y.p + i * l, Nl, 1, M.wg.p + i * ll, l, 1));
       c1.push_back(CholDesc{l, M.wg.p + i * ll, M.xr.p + i * ll});
       P.m_x.host.push_back(gm(M.xr.p + i * ll, l, 1, M.wp.p + i * ll, l, 1, l, l, kMapCopy));
       P.apply.host.push_back(prod(m, l, l, M.y.p + i * l, Nl, 1, M.wp.p + i * ll, l, 1, M.qs.p + i * l, Nl, 1));
     }
-    P.gfull.host.push_back(prod(Nl, Nl, m, M.qs.p, 1, Nl, M.qs.p, Nl, 1, M.G.p, Nl, 1));
-    P.gfull.host.back().upper = 1;  // G = Qs'Qs symmetric: the upper triangle's tiles, then mirrored
+    if (own_product<T>(Nl, Nl, m, true)) {
+      P.own_gfull.push_back(b);
+    } else {
+      P.gfull.host.push_back(prod(Nl, Nl, m, M.qs.p, 1, Nl, M.qs.p, Nl, 1, M.G.p, Nl, 1));
+      P.gfull.host.back().upper = 1;
+    }
+    // G = Qs'Qs symmetric: the upper triangle's tiles, then mirrored
     P.m_mirror.host.push_back(gm(M.G.p, Nl, 1, M.G.p, Nl, 1, Nl, Nl, kMapMirror));
     // iterate [M | B | Bgc] in W[0]: Bc = G[:, 0:l], M = [I; 0]
     P.m_init.host.push_back(gm(M.G.p, Nl, 1, M.W.p + l, 3 * l, 1, Nl, l, kMapCopy));
@@ -538,13 +558,48 @@ inline void eig_classes(const DevList<EigDesc> &d, const std::vector<std::pair<i
 
 template <class T>
 void run_pre(Plan<T> &P, cudaStream_t st, bool measure) {
-  for (int b = 0; b < P.count; ++b)
+  for (int b = 0, o = 0; b < P.count; ++b) {
+    if (o < (int)P.own_sketch.size() && P.own_sketch[o] == b) {
+      ++o;
+      continue;
+    }
     rng_gaussian<T>(P.mats[b]->om.p, P.n[b], P.Nl[b], P.Nl[b], P.seeds[b], 0, st);
+  }
   P.sketch.run(st, measure);
   P.gram.run(st, measure);
   chol_inv_grouped(P.chol.d.p, P.chol.count, P.max_l, P.status.p, st);
   P.m_x.launch(st);
   P.apply.run(st, measure);
+}
+
+// The products of their own, whose workspaces live for the call only: outside the graphs, before run_pre and
+// after it.
+template <class T>
+void run_own_sketches(Plan<T> &P, cudaStream_t st) {
+  for (int b : P.own_sketch) {
+    auto &M = *P.mats[b];
+    rng_gaussian<T>(M.om.p, P.n[b], P.Nl[b], P.Nl[b], P.seeds[b], 0, st);
+    Gemm<T, T> g;
+    g.M = P.m[b]; g.N = P.Nl[b]; g.K = P.n[b];
+    g.A = P.a[b]; g.a_rs = P.lda[b]; g.a_cs = 1;
+    g.B = M.om.p; g.b_rs = P.Nl[b]; g.b_cs = 1;
+    g.C = M.y.p; g.c_rs = P.Nl[b]; g.c_cs = 1;
+    gemm(g, st);
+  }
+}
+
+template <class T>
+void run_gfull(Plan<T> &P, cudaStream_t st, bool measure) {
+  for (int b : P.own_gfull) {
+    auto &M = *P.mats[b];
+    Gemm<T, double> g;
+    g.M = g.N = P.Nl[b]; g.K = P.m[b];
+    g.A = M.qs.p; g.a_rs = 1; g.a_cs = P.Nl[b];
+    g.B = M.qs.p; g.b_rs = P.Nl[b]; g.b_cs = 1;
+    g.C = M.G.p; g.c_rs = P.Nl[b]; g.c_cs = 1;
+    g.upper = true;
+    gemm(g, st);
+  }
   P.gfull.run(st, measure);
   P.m_mirror.launch(st);
   P.m_init.launch(st);
@@ -669,7 +724,9 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
   }
   const bool capture = P.solves > 0 && st != nullptr && !profiling();
   CK(cudaMemsetAsync(P.status.p, 0, sizeof(int), st));
+  run_own_sketches(P, st);
   graphed(P.pre, P.pre_k, capture, st, [&] { run_pre(P, st, !capture); });
+  run_gfull(P, st, !capture);
 
   // ---- Kolmogorov-Nagumo iterations of the active matrices (reference :153-266)
   const double invN = 1.0 / N;

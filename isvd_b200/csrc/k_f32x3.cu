@@ -131,6 +131,10 @@ static bool plane_product_pays(double M, double N, double K, double batch, doubl
   return planes < 0.8 * cuda;
 }
 
+bool f32_planes_pay(double M, double N, double K, bool gram) {
+  return !planes_off() && Runtime::get().cc_major == 10 && plane_product_pays(M, N, K, 1, M * K, gram ? 0.0 : N * K);
+}
+
 template <class Tout>
 bool gemm_f32_planes(const Gemm<float, Tout> &g, bool a_kc, bool b_nc, cudaStream_t st) {
   if (planes_off() || Runtime::get().cc_major != 10 || g.beta != 0.0 || g.pl_t) return false;

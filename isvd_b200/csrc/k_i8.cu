@@ -581,6 +581,10 @@ bool i8_pays(double M, double N, double K, bool same, bool upper) {
 
 }  // namespace
 
+bool f64_int8_pays(double M, double N, double K, bool gram) {
+  return !i8_off() && Runtime::get().cc_major == 10 && K >= 640 && M >= 64 && N >= 64 && i8_pays(M, N, K, gram, gram);
+}
+
 bool gemm_f64_int8(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream_t st) {
   if (g.batch != 1 || g.beta != 0.0 || g.pl_t || g.splits > 1 || i8_off() || Runtime::get().cc_major != 10) return false;
   if (g.K < 640 || g.M < 64 || g.N < 64 || g.N > (1 << 20)) return false;

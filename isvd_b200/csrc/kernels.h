@@ -49,6 +49,10 @@ void gemm(const Gemm<T, Tout> &g, cudaStream_t st);
 template <class Tout>
 bool gemm_f32_planes(const Gemm<float, Tout> &g, bool a_kc, bool b_nc, cudaStream_t st);
 
+// Whether an M x N x K product (gram: C = A'A, M == N) is faster by planes (FP32) or digits (FP64).
+bool f32_planes_pay(double M, double N, double K, bool gram);
+bool f64_int8_pays(double M, double N, double K, bool gram);
+
 // FP64 operands and result on the FP64 tensor-core path (mma.sync m8n8k4, k_dmma.cu); gemm()
 // routes Gemm<double, double> here unless ISVD_GPU_DMMA=0.  a_kc: A has unit K stride; b_nc: B
 // has unit N stride.

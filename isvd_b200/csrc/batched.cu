@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "batched.h"
+#include "grouped_next.cuh"
 #include "kernels.h"
 #include "runtime.h"
 
@@ -82,15 +83,16 @@ constexpr int ggemm_smem() {  // bytes of the kGStages ring of A (BK x BM) and B
   return kGStages * kGBK * (BM + BN + 2 * (16 / (int)sizeof(T))) * (int)sizeof(T);
 }
 
-// Grouped products on CUDA cores: each CTA walks the work items blockIdx.x, blockIdx.x + gridDim.x,
-// ...; a work item is one BM x BN output tile of the product that owns it.  K slices of 16 flow
+// Grouped products on CUDA cores: each CTA takes the work item blockIdx.x and then the next one that no
+// CTA has (GroupedNext; the list has its longest products first); a work item is one BM x BN output tile of the product that owns it.  K slices of 16 flow
 // through a kGStages-deep cp.async ring in shared memory (A stored k-major as As[k][m], B as
 // Bs[k][n]).  256 threads in a 16 x 16 grid, each accumulating TM x TN outputs: rows
 // ty * TM/2 + [0, TM/2) of both halves of the tile (and columns likewise), so that a thread's
 // operands of one k are two vector loads from shared memory per operand.  Each output is one FMA
 // chain in ascending k.
 template <class T, class Tout, int BM, int BN>
-__global__ void __launch_bounds__(kGThreads) ggemm_kernel(const GProd *__restrict__ prods, int nprod, int total) {
+__global__ void __launch_bounds__(kGThreads)
+    ggemm_kernel(const GProd *__restrict__ prods, int nprod, int total, int *next) {
   constexpr int BK = kGBK, TM = BM / 16, TN = BN / 16, HM = TM / 2, HN = TN / 2;
   constexpr int LA = BM * BK / kGThreads, LB = BK * BN / kGThreads;
   constexpr int kPad = 16 / (int)sizeof(T);  // rows stay 16-byte aligned; transposing stores spread over banks
@@ -98,7 +100,10 @@ __global__ void __launch_bounds__(kGThreads) ggemm_kernel(const GProd *__restric
   extern __shared__ __align__(16) unsigned char gsm[];
   T *ring = reinterpret_cast<T *>(gsm);
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  for (int t = blockIdx.x; t < total; t += gridDim.x) {
+  __shared__ int snext;
+  GroupedNext items(next, &snext);
+  for (int t = blockIdx.x; t < total; t = items.take()) {
+    items.fetch();
     int lo = 0, hi = nprod - 1;  // the product owning work item t
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -181,10 +186,11 @@ __global__ void __launch_bounds__(kGThreads) ggemm_kernel(const GProd *__restric
       }
     }
   }
+  items.done();
 }
 
 template <class T, class Tout, int BM, int BN>
-void ggemm_launch(const GProd *prods, int nprod, int total, cudaStream_t st) {
+void ggemm_launch(const GProd *prods, int nprod, int total, int *next, cudaStream_t st) {
   auto *k = ggemm_kernel<T, Tout, BM, BN>;
   constexpr int bytes = ggemm_smem<T, BM, BN>();
   static int per_sm = 0;  // resident CTAs per SM, resolved on first use
@@ -194,7 +200,7 @@ void ggemm_launch(const GProd *prods, int nprod, int total, cudaStream_t st) {
     per_sm = std::max(1, per_sm);
   }
   const int grid = std::max(1, std::min(total, per_sm * Runtime::get().num_sms));
-  k<<<grid, kGThreads, bytes, st>>>(prods, nprod, total);
+  k<<<grid, kGThreads, bytes, st>>>(prods, nprod, total, next);
   KLAUNCHED();
 }
 
@@ -258,6 +264,7 @@ struct GemmList {
   static constexpr bool kFp64 = std::is_same<T, double>::value && std::is_same<Tout, double>::value;
   std::vector<GProd> host;
   DevList<GProd> dev;
+  DBuf<int> next;  // GroupedNext's two words
   int config = -1, total = 0, uploaded = -1;
   bool dmma = false, a_kc = false, b_nc = false;  // orientation of the tensor-core launch
 
@@ -301,6 +308,12 @@ struct GemmList {
            std::to_string(lg(bm)) + "," + std::to_string(lg(bn)) + "," + std::to_string(lg(bk));
   }
   void finalize(int cfg, cudaStream_t st) {  // work items for tile shape cfg, uploaded
+    // the longest products first, so that the last work items of a launch are short ones
+    std::stable_sort(host.begin(), host.end(), [](const GProd &x, const GProd &y) { return x.K > y.K; });
+    if (!next.p) {
+      next.alloc(2);
+      CK(cudaMemsetAsync(next.p, 0, 2 * sizeof(int), st));
+    }
     int tot = 0;
     for (auto &g : host) {
       g.tn = (g.N + bn(cfg) - 1) / bn(cfg);
@@ -314,13 +327,13 @@ struct GemmList {
   void launch(int cfg, cudaStream_t st) {  // kernels only (capturable)
     if (host.empty() || total == 0) return;
     if (dmma) {
-      dmma_grouped(static_cast<const GroupedProd *>(dev.d.p), dev.count, total, cfg, a_kc, b_nc, st);
+      dmma_grouped(static_cast<const GroupedProd *>(dev.d.p), dev.count, total, cfg, a_kc, b_nc, next.p, st);
       return;
     }
     switch (cfg) {
-      case 0: ggemm_launch<T, Tout, 64, 64>(dev.d.p, dev.count, total, st); break;
-      case 1: ggemm_launch<T, Tout, 128, 64>(dev.d.p, dev.count, total, st); break;
-      default: ggemm_launch<T, Tout, 128, 128>(dev.d.p, dev.count, total, st); break;
+      case 0: ggemm_launch<T, Tout, 64, 64>(dev.d.p, dev.count, total, next.p, st); break;
+      case 1: ggemm_launch<T, Tout, 128, 64>(dev.d.p, dev.count, total, next.p, st); break;
+      default: ggemm_launch<T, Tout, 128, 128>(dev.d.p, dev.count, total, next.p, st); break;
     }
   }
   // Choose the tile shape (measuring every candidate on first sight of the signature when all
@@ -733,6 +746,7 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
   const int cap = maxit > 0 ? maxit : 1000000;
   std::vector<int> active(B), cur(B, 0), it_of(B, 0);
   for (int b = 0; b < B; ++b) active[b] = b;
+  std::stable_sort(active.begin(), active.end(), [&](int x, int y) { return P.l[x] > P.l[y]; });  // long products first
   std::vector<double> herr(B, 0.0);
   std::vector<KnStep> hsteps;
   for (int iter = 1; !active.empty(); ++iter) {

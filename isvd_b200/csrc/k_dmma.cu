@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "grouped_next.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "planes.cuh"
@@ -270,17 +271,20 @@ __global__ void __launch_bounds__(WM * WN * 32)
   cl.sync();  // the peers' reads of this CTA's tile are done
 }
 
-// Grouped products (dmma_grouped): each CTA walks the work items blockIdx.x, blockIdx.x + gridDim.x,
-// ...; a work item is one BM x BN output tile of the product that owns it (binary search on tile0).
+// Grouped products (dmma_grouped): each CTA takes the work item blockIdx.x and then the next one that no CTA
+// has; a work item is one BM x BN output tile of the product that owns it (binary search on tile0).
 template <int BM, int BN, int WM, int WN, bool A_KC, bool B_NC>
 __global__ void __launch_bounds__(WM * WN * 32)
-    dmma_grouped_kernel(const GroupedProd *__restrict__ prods, int nprod, int total) {
+    dmma_grouped_kernel(const GroupedProd *__restrict__ prods, int nprod, int total, int *next) {
   constexpr int TM = BM / WM / 8, TN = BN / WN / 8;
   extern __shared__ double smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm0 = (warp / WN) * (BM / WM), wn0 = (warp % WN) * (BN / WN);
   const int fr = lane >> 2, fc = lane & 3;
-  for (int t = blockIdx.x; t < total; t += gridDim.x) {
+  __shared__ int snext;
+  GroupedNext items(next, &snext);
+  for (int t = blockIdx.x; t < total; t = items.take()) {
+    items.fetch();
     int lo = 0, hi = nprod - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -317,10 +321,11 @@ __global__ void __launch_bounds__(WM * WN * 32)
         }
     }
   }
+  items.done();
 }
 
 template <int BM, int BN, int WM, int WN, bool A_KC, bool B_NC>
-void dmma_grouped_launch(const GroupedProd *prods, int nprod, int total, cudaStream_t st) {
+void dmma_grouped_launch(const GroupedProd *prods, int nprod, int total, int *next, cudaStream_t st) {
   auto *k = dmma_grouped_kernel<BM, BN, WM, WN, A_KC, B_NC>;
   constexpr int NT = WM * WN * 32;
   const int bytes = kStages * DmmaLayout<BM, BN, A_KC, B_NC>::stage * (int)sizeof(double);
@@ -331,7 +336,7 @@ void dmma_grouped_launch(const GroupedProd *prods, int nprod, int total, cudaStr
     per_sm = std::max(1, per_sm);
   }
   const int grid = std::max(1, std::min(total, per_sm * Runtime::get().num_sms));
-  k<<<grid, NT, bytes, st>>>(prods, nprod, total);
+  k<<<grid, NT, bytes, st>>>(prods, nprod, total, next);
   KLAUNCHED();
 }
 
@@ -493,13 +498,14 @@ void dmma_gemm_rest(const Gemm<double, double> &g, bool a_kc, bool b_nc, const f
 int dmma_grouped_bm(int shape) { return shape == 2 ? 128 : shape == 4 ? 32 : 64; }
 int dmma_grouped_bn(int shape) { return (shape == 0 || shape >= 3) ? 32 : 64; }
 
-void dmma_grouped(const GroupedProd *prods, int nprod, int total, int shape, bool a_kc, bool b_nc, cudaStream_t st) {
+void dmma_grouped(const GroupedProd *prods, int nprod, int total, int shape, bool a_kc, bool b_nc, int *next,
+                  cudaStream_t st) {
   if (nprod <= 0 || total <= 0) return;
 #define ISVD_DMMA_GROUPED(BM, BN, WM, WN)                                                              \
-  if (a_kc && b_nc) dmma_grouped_launch<BM, BN, WM, WN, true, true>(prods, nprod, total, st);          \
-  else if (a_kc) dmma_grouped_launch<BM, BN, WM, WN, true, false>(prods, nprod, total, st);            \
-  else if (b_nc) dmma_grouped_launch<BM, BN, WM, WN, false, true>(prods, nprod, total, st);            \
-  else dmma_grouped_launch<BM, BN, WM, WN, false, false>(prods, nprod, total, st);
+  if (a_kc && b_nc) dmma_grouped_launch<BM, BN, WM, WN, true, true>(prods, nprod, total, next, st);          \
+  else if (a_kc) dmma_grouped_launch<BM, BN, WM, WN, true, false>(prods, nprod, total, next, st);            \
+  else if (b_nc) dmma_grouped_launch<BM, BN, WM, WN, false, true>(prods, nprod, total, next, st);            \
+  else dmma_grouped_launch<BM, BN, WM, WN, false, false>(prods, nprod, total, next, st);
   switch (shape) {  // warp tiles of 32 x 32 outputs (4 x 4 mma tiles), or 32 x 16 (shape 3)
     case 0: ISVD_DMMA_GROUPED(64, 32, 2, 1) break;
     case 1: ISVD_DMMA_GROUPED(64, 64, 2, 2) break;

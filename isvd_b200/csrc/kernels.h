@@ -78,11 +78,13 @@ struct GroupedProd {
 // FP64 grouped products on the FP64 tensor-core path (k_dmma.cu): one persistent launch walks the
 // `total` work items of prods[0 .. nprod) (device memory, tile0 ascending).  Every product has the
 // same operand orientation: a_kc (a_cs == 1, else a_rs == 1) and b_nc (b_cs == 1, else b_rs == 1).
+// next: two ints, zero before the first launch (grouped_next.cuh).
 // Tile shapes: dmma_grouped_bm(shape) x dmma_grouped_bn(shape), shape < kDmmaGroupedShapes.
 constexpr int kDmmaGroupedShapes = 5;
 int dmma_grouped_bm(int shape);
 int dmma_grouped_bn(int shape);
-void dmma_grouped(const GroupedProd *prods, int nprod, int total, int shape, bool a_kc, bool b_nc, cudaStream_t st);
+void dmma_grouped(const GroupedProd *prods, int nprod, int total, int shape, bool a_kc, bool b_nc, int *next,
+                  cudaStream_t st);
 
 // A large FP64 product on the int8 tensor cores (k_i8.cu): true when it was enqueued there.
 // dmma_gemm_rest: the tiles that it leaves to k_dmma.cu.

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(kGThreads)
     const GProd g = prods[lo];
     const int tt = t - g.tile0, m0 = (tt / g.tn) * BM, n0 = (tt % g.tn) * BN;
     if (g.upper && n0 + BN <= m0) continue;  // strictly below the diagonal (uniform in the CTA)
+    if (g.gate && *g.gate <= g.gate_tol) continue;
     const T *__restrict__ A = static_cast<const T *>(g.A);
     const T *__restrict__ B = static_cast<const T *>(g.B);
     const bool akc = (g.a_cs == 1), bnc = (g.b_cs == 1);
@@ -417,6 +418,8 @@ inline GProd prod(int M, int N, int K, const void *A, long long a_rs, long long 
   g.alpha = alpha; g.beta = 0.0;
   g.tile0 = 0; g.tn = 1;
   g.upper = 0;
+  g.gate = nullptr;
+  g.gate_tol = 0.0;
   return g;
 }
 
@@ -439,7 +442,9 @@ struct Plan : BatchPlan {
     DBuf<double> wg, xr, G, W, DD, C, Ci, F, Fs, work, wz, vz, lz;
   };
   std::vector<std::unique_ptr<Mat>> mats;
-  DBuf<double> errs;
+  DBuf<double> errs;        // of the iterations of either parity
+  double *herrs = nullptr;  // pinned copies
+  cudaEvent_t read[2] = {nullptr, nullptr};
   DBuf<int> status;
   // bound user buffers
   std::vector<const T *> a;
@@ -474,11 +479,15 @@ struct Plan : BatchPlan {
       if (join[i]) cudaEventDestroy(join[i]);
     }
     if (fork) cudaEventDestroy(fork);
+    for (int i = 0; i < 2; ++i)
+      if (read[i]) cudaEventDestroy(read[i]);
+    if (herrs) cudaFreeHost(herrs);
   }
   void make_side_streams() {
     if (fork) return;
     CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     for (int i = 0; i < 2; ++i) {
+      CK(cudaEventCreateWithFlags(&read[i], cudaEventDisableTiming));
       CK(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking));
       CK(cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming));
     }
@@ -700,7 +709,8 @@ BatchPlan *batch_plan_create(int count, const int *m, const int *n, const int *k
     M->wz.alloc(ll); M->vz.alloc(ll); M->lz.alloc(l);
     P->mats[b] = std::move(M);
   }
-  P->errs.alloc(count);
+  P->errs.alloc(2 * (size_t)count);
+  CK(cudaMallocHost(&P->herrs, 2 * (size_t)count * sizeof(double)));
   P->status.alloc(1);
   return P.release();
 }
@@ -744,31 +754,43 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
   // ---- Kolmogorov-Nagumo iterations of the active matrices (reference :153-266)
   const double invN = 1.0 / N;
   const int cap = maxit > 0 ? maxit : 1000000;
-  std::vector<int> active(B), cur(B, 0), it_of(B, 0);
+  std::vector<int> active(B), it_of(B, 0);
   for (int b = 0; b < B; ++b) active[b] = b;
   std::stable_sort(active.begin(), active.end(), [&](int x, int y) { return P.l[x] > P.l[y]; });  // long products first
   std::vector<double> herr(B, 0.0);
   std::vector<KnStep> hsteps;
-  for (int iter = 1; !active.empty(); ++iter) {
+  P.make_side_streams();
+  // Iteration `it` of the matrices `act`: from iterate buffer (it - 1) & 1 to it & 1.  It is enqueued before
+  // the errors of iteration it - 1 are read, so that the GPU does not wait for the host (60 us per
+  // iteration); a matrix that has converged meanwhile is passed over on the device (the gates).
+  auto launch = [&](int it, const std::vector<int> &act) {
+    const int par = it & 1;
     P.l1.clear(); P.l2.clear(); P.l4.clear();
     hsteps.clear();
-    for (int b : active) {
+    for (int b : act) {
       auto &M = *P.mats[b];
       const int l = P.l[b], Nl = P.Nl[b];
       const size_t ll = (size_t)l * l, nl3 = (size_t)Nl * 3 * l;
-      double *Wc = M.W.p + cur[b] * nl3, *Wn = M.W.p + (1 - cur[b]) * nl3;
+      double *Wc = M.W.p + (1 - par) * nl3, *Wn = M.W.p + par * nl3;
       const long long lw = 3LL * l;
       P.l1.host.push_back(prod(Nl, l, Nl, M.G.p, Nl, 1, Wc + l, lw, 1, Wc + 2 * l, lw, 1, invN));
       P.l2.host.push_back(prod(l, l, Nl, Wc + l, 1, lw, Wc + l, lw, 1, M.DD.p, l, 1, invN));
       P.l2.host.push_back(prod(l, l, Nl, Wc + l, 1, lw, Wc + 2 * l, lw, 1, M.DD.p + ll, l, 1, invN));
       P.l4.host.push_back(prod(Nl, l, 2 * l, Wc, lw, 1, M.Fs.p, l, 1, Wn, lw, 1));
       P.l4.host.push_back(prod(Nl, l, 2 * l, Wc + l, lw, 1, M.Fs.p + 2 * ll, l, 1, Wn + l, lw, 1));
+      const double *gate = it > 1 ? P.errs.p + (size_t)(1 - par) * B + b : nullptr;
       KnStep s;
       s.l = l; s.Dc = M.DD.p; s.Dgc = M.DD.p + ll; s.C = M.C.p; s.Cinv = M.Ci.p; s.F = M.F.p;
-      s.err = P.errs.p + b; s.work = M.work.p; s.status = P.status.p; s.bar = nullptr;
+      s.err = P.errs.p + (size_t)par * B + b; s.work = M.work.p; s.status = P.status.p; s.bar = nullptr;
       s.ns_target = 1e-18;
       s.fstack = M.Fs.p; s.fstack_scale = invN;
+      s.gate = gate; s.gate_tol = tol;
       hsteps.push_back(s);
+      for (auto *list : {&P.l1.host, &P.l2.host, &P.l4.host})
+        for (size_t e = list->size() - (list == &P.l1.host ? 1 : 2); e < list->size(); ++e) {
+          (*list)[e].gate = gate;
+          (*list)[e].gate_tol = tol;
+        }
     }
     P.l1.run(st, true);
     P.l2.run(st, true);
@@ -781,7 +803,6 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
     std::stable_sort(hsteps.begin(), hsteps.end(),
                      [&](const KnStep &x, const KnStep &y) { return class_of(x) > class_of(y); });
     P.steps.upload(hsteps, st);
-    P.make_side_streams();
     CK(cudaEventRecord(P.fork, st));
     int group = 0;
     const int sms = rt.num_sms;
@@ -811,14 +832,25 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
       g0 = g1;
     }
     P.l4.run(st, true);
+    CK(cudaMemcpyAsync(P.herrs + (size_t)par * B, P.errs.p + (size_t)par * B, B * sizeof(double), cudaMemcpyDeviceToHost,
+                       st));
+    CK(cudaEventRecord(P.read[par], st));
+  };
+  auto check_status = [&] {
     int hstatus = 0;
-    CK(cudaMemcpyAsync(herr.data(), P.errs.p, B * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&hstatus, P.status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (hstatus) fail(kErrNumerical, "batched iSVD: small dense solver reported status %d", hstatus);
+  };
+  launch(1, active);
+  for (int iter = 1; !active.empty(); ++iter) {
+    if (iter < cap) launch(iter + 1, active);
+    CK(cudaEventSynchronize(P.read[iter & 1]));
     std::vector<int> next;
+    bool lost = iter % 16 == 0;
     for (int b : active) {
-      cur[b] = 1 - cur[b];  // the iterate just written
+      herr[b] = P.herrs[(size_t)(iter & 1) * B + b];
+      lost = lost || !(herr[b] == herr[b]);
       if (herr[b] <= tol) {                 // (:235-237)
         it_of[b] = iter;
       } else if (iter == cap) {             // (:238-241)
@@ -827,15 +859,18 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
         next.push_back(b);
       }
     }
+    if (lost) check_status();
     active.swap(next);
   }
+  check_status();
+  auto last_of = [&](int b) { return std::min(it_of[b], cap) & 1; };  // the iterate buffer of the result
   // M of each matrix (in its final iterate) to the element type
   {
     MapList<double, T> mt;
     for (int b = 0; b < B; ++b) {
       auto &M = *P.mats[b];
       const size_t nl3 = (size_t)P.Nl[b] * 3 * P.l[b];
-      mt.host.push_back(gm(M.W.p + cur[b] * nl3, 3LL * P.l[b], 1, M.mt.p, P.l[b], 1, P.Nl[b], P.l[b], kMapCopy));
+      mt.host.push_back(gm(M.W.p + last_of(b) * nl3, 3LL * P.l[b], 1, M.mt.p, P.l[b], 1, P.Nl[b], P.l[b], kMapCopy));
     }
     mt.prepare(st);
     mt.launch(st);

@@ -631,6 +631,7 @@ __global__ void __launch_bounds__(kKrThreads, 1) kn_rows_kernel(KnStep a, KnSeri
 // One cluster per step of steps[] (grid = count x cluster size): many independent problems.
 __global__ void __launch_bounds__(kKrThreads, 1) kn_rows_grouped_kernel(const KnStep *steps, KnSeries ser, int blocks) {
   const KnStep a = steps[blockIdx.x / cg::this_cluster().num_blocks()];
+  if (a.gate && *a.gate <= a.gate_tol) return;  // alike in every CTA of the cluster
   kn_rows_body(a, ser, blocks);
 }
 

@@ -74,6 +74,9 @@ struct GroupedProd {
   double alpha, beta;
   int tile0, tn;
   int upper;  // C symmetric (A = B'): tiles entirely below the diagonal are skipped (mirrored by the caller)
+  // when set: nothing is computed if *gate <= gate_tol (device memory, read when the launch runs)
+  const double *gate;
+  double gate_tol;
 };
 // FP64 grouped products on the FP64 tensor-core path (k_dmma.cu): one persistent launch walks the
 // `total` work items of prods[0 .. nprod) (device memory, tile0 ascending).  Every product has the
@@ -165,6 +168,8 @@ struct KnStep {
   // kn_step only: when set, also written as the 4l x l stack [F; Cinv * fstack_scale; F; Cinv]
   double *fstack = nullptr;
   double fstack_scale = 1.0;
+  const double *gate = nullptr;  // kn_step_grouped only: as GroupedProd::gate
+  double gate_tol = 0.0;
 };
 constexpr int kKnWorkMatrices = 29;
 constexpr int kSeriesLen = 128;

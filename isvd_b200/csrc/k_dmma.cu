@@ -488,6 +488,20 @@ void dmma_gemm(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream_t
     dmma_launch<128, 128, 2, 4>(g, a_kc, b_nc, st);
 }
 
+// C_b = A_b B_b over A (column blocks of a tall matrix times N x N blocks): a CTA holds its rows' whole block
+// in one tile and has read all of it (the barrier of the last K slice) before it writes.  Saves the
+// temporary and its copy back: 0.5 ms of 0.98 GB for the 16 blocks of 40000 x 96.
+bool dmma_apply_in_place(const Gemm<double, double> &g, cudaStream_t st) {
+  if (!dmma_enabled() || g.N > 128 || g.K != g.N || g.beta != 0.0) return false;
+  Gemm<double, double> f = g;
+  f.C = const_cast<double *>(g.A);
+  f.c_rs = g.a_rs; f.c_cs = g.a_cs; f.c_bs = g.a_bs;
+  f.splits = 1;
+  if (g.N <= 64) dmma_launch<64, 64, 2, 2>(f, true, true, st);
+  else dmma_launch<128, 128, 2, 4>(f, true, true, st);
+  return true;
+}
+
 void dmma_gemm_rest(const Gemm<double, double> &g, bool a_kc, bool b_nc, const float *done_a, const float *done_b,
                     float lim, cudaStream_t st) {
   Gemm<double, double> f = g;

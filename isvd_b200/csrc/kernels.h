@@ -58,6 +58,9 @@ bool f64_int8_pays(double M, double N, double K, bool gram);
 // has unit N stride.
 bool dmma_enabled();
 void dmma_gemm(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream_t st);
+// A_b := A_b B_b (A's K and B's N contiguous, K == N <= 128, g.C not read): false when it has to go through
+// a temporary.
+bool dmma_apply_in_place(const Gemm<double, double> &g, cudaStream_t st);
 // C = alpha * (sum of the `splits` partial products) + beta * C (partials: batch x splits x M x N).
 void splitk_reduce(const Gemm<double, double> &g, int splits, const double *partial, cudaStream_t st);
 // One product of a grouped launch over many independent products of their own shapes:

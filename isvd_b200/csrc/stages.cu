@@ -156,7 +156,8 @@ void gramian_pass(const StageCtx &c, int m, int l, int N, T *y, long long ldy, b
     copy2d<double, T>(P.p, l, 1, Wp.p, l, 1, (long long)N * l, l, c.st);
   }
   // Q_i = Y_i F_i  (:95-98).  MIXED with planes: the product reads only the planes, so it writes
-  // y in place; otherwise it goes to a temporary that is copied back.
+  // y in place, as does the FP64 product with one tile per block; otherwise it goes to a temporary
+  // that is copied back.
   if (c.precision == kMixed && l % 64 == 0) {
     const bool out_planes = emit && c.handoff;
     mixed_block_apply<T>(c, yp.P, m, l, N, y, ldy, Wp.p, y, ldy, out_planes ? c.handoff : nullptr);
@@ -169,14 +170,16 @@ void gramian_pass(const StageCtx &c, int m, int l, int N, T *y, long long ldy, b
       return;
     }
   if (from_hand) fail(kErrUnsupported, "plane hand-off into the Gramian orthogonalization needs l %% 64 == 0");
+  Gemm<T, T> g = gm<T>(m, l, l);
+  g.batch = N;
+  g.A = y; g.a_rs = ldy; g.a_cs = 1; g.a_bs = l;
+  g.B = Wp.p; g.b_rs = l; g.b_cs = 1; g.b_bs = (long long)ll;
+  if constexpr (std::is_same<T, double>::value)
+    if (c.precision != kMixed && dmma_apply_in_place(g, c.st)) return;
   DBuf<T> tmp((size_t)m * Nl);
   if (c.precision == kMixed) {
     mixed_block_apply<T>(c, yp.P, m, l, N, y, ldy, Wp.p, tmp.p, Nl);
   } else {
-    Gemm<T, T> g = gm<T>(m, l, l);
-    g.batch = N;
-    g.A = y; g.a_rs = ldy; g.a_cs = 1; g.a_bs = l;
-    g.B = Wp.p; g.b_rs = l; g.b_cs = 1; g.b_bs = (long long)ll;
     g.C = tmp.p; g.c_rs = Nl; g.c_cs = 1; g.c_bs = l;
     gemm(g, c.st);
   }

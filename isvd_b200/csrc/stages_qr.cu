@@ -108,10 +108,15 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
   const bool mixed = (c.precision == kMixed);
   const double u = mixed ? 0x1p-24 : unit_roundoff<T>();
   DBuf<double> W(N * ll), X(N * ll);
-  DBuf<T> Xt(N * ll), tmp((size_t)rows * Nl);
+  DBuf<T> Xt(N * ll), tmp;  // tmp: allocated by the first pass that does not work in place
   DBuf<int> nmask((size_t)Nl + 1);  // null-column flags, then their count
   CK(cudaMemsetAsync(nmask.p, 0, ((size_t)Nl + 1) * sizeof(int), c.st));
-  T *src = y, *dst = tmp.p;
+  T *src = y, *dst = nullptr;
+  auto need_tmp = [&] {
+    if (tmp.p) return;
+    tmp.alloc((size_t)rows * Nl);
+    dst = tmp.p;
+  };
   long long lds = ldy, ldd = Nl;
   for (int pass = 0; pass < 3; ++pass) {
     PlaneBuf yp;
@@ -161,13 +166,16 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
         f32_block_apply(yp, (int)rows, l, N, Xt.p, src, lds, c.st);
         continue;
       }
+    Gemm<T, T> g;
+    g.M = (int)rows; g.N = l; g.K = l; g.batch = N;
+    g.A = src; g.a_rs = lds; g.a_cs = 1; g.a_bs = l;
+    g.B = Xt.p; g.b_rs = l; g.b_cs = 1; g.b_bs = (long long)ll;
+    if constexpr (std::is_same<T, double>::value)
+      if (!mixed && dmma_apply_in_place(g, c.st)) continue;
+    need_tmp();
     if (mixed) {
       mixed_block_apply<T>(c, yp.P, (int)rows, l, N, src, lds, Xt.p, dst, ldd);
     } else {
-      Gemm<T, T> g;
-      g.M = (int)rows; g.N = l; g.K = l; g.batch = N;
-      g.A = src; g.a_rs = lds; g.a_cs = 1; g.a_bs = l;
-      g.B = Xt.p; g.b_rs = l; g.b_cs = 1; g.b_bs = (long long)ll;
       g.C = dst; g.c_rs = ldd; g.c_cs = 1; g.c_bs = l;
       gemm(g, c.st);
     }
@@ -177,8 +185,11 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
   int nulls = 0;
   CK(cudaMemcpyAsync(&nulls, nmask.p + Nl, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
-  if (nulls > 0) complete_null_columns<T>(c, rows, l, N, src, lds, dst, ldd, nmask.p);
-  // three passes: y -> tmp -> y -> tmp (two more for a completion: -> y -> tmp), or in place
+  if (nulls > 0) {
+    need_tmp();
+    complete_null_columns<T>(c, rows, l, N, src, lds, dst, ldd, nmask.p);
+  }
+  // three passes: in place, or y -> tmp -> y -> tmp (two more for a completion: the other, and back)
   if (src != y) CK(cudaMemcpy2DAsync(y, ldy * sizeof(T), src, lds * sizeof(T), (size_t)Nl * sizeof(T), rows,
                        cudaMemcpyDeviceToDevice, c.st));
 }

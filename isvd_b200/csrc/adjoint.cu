@@ -30,6 +30,7 @@
 
 #include "kernels.h"
 #include "mixed.h"
+#include "pdl.cuh"
 #include "planes.cuh"
 #include "runtime.h"
 #include "stages.h"
@@ -139,7 +140,9 @@ __global__ void cg_step2_kernel(T *p, const T *__restrict__ r, long long rows, i
 // [1] the done word: set by the update that brings every column below tol, after which the launches
 // that the host has already enqueued return at once.  Bound by latency (the loads, two reductions and the
 // arrival counter; 2 to 4 MB moved): at n = 4096, 2 k = 128 the three take 15, 18 and 6 us, where two
-// dot products of two launches each, the scaling, both steps, a copy and the split took 52.
+// dot products of two launches each, the scaling, both steps, a copy and the split took 52.  All of an
+// iteration's launches are programmatic (pdl.cuh): 38 iterations 6.23 -> 5.87 ms of a 16384 x 4096 adjoint.
+// (In the Kolmogorov-Nagumo loop, whose products fill the SMs, the same cost 4 % at N l = 1536.)
 constexpr int kCgThreads = 512;
 constexpr int kCgBlocks = 128;
 
@@ -245,6 +248,8 @@ __global__ void __launch_bounds__(kCgThreads)
                     float *__restrict__ q,
                     long long rows, int kc, double *partial, unsigned *ctl, double *pq) {
   extern __shared__ double sh[];
+  pdl_trigger();
+  pdl_wait();
   if (((volatile unsigned *)ctl)[1]) return;
   cg_dot_rows(sh, rows, kc, partial, [=](int c) {
     const double sc = s[c];
@@ -259,6 +264,8 @@ __global__ void __launch_bounds__(kCgThreads)
                      double *partial, unsigned *ctl, double *host_done) {
   extern __shared__ double sh[];
   __shared__ int above;
+  pdl_trigger();
+  pdl_wait();
   if (((volatile unsigned *)ctl)[1]) return;
   cg_dot_rows(sh, rows, kc, partial, [=](int c) {
     return CgUpdate{x, r, p, q, (rr[c] > 0.0 && pq[c] != 0.0) ? rr[c] / pq[c] : 0.0};
@@ -283,6 +290,8 @@ __global__ void __launch_bounds__(256)
     cg_next_kernel(float *p, const float *__restrict__ r, const double *__restrict__ beta, long long rows, int kc,
                    const unsigned *ctl, __nv_bfloat16 *__restrict__ planes, long long ld, long long ps) {
   __shared__ float tile[64][33];
+  pdl_trigger();
+  pdl_wait();
   if (((const volatile unsigned *)ctl)[1]) return;
   const long long r0 = (long long)blockIdx.x * 64;
   const int c0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -743,6 +752,7 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
     g.C = z.p; g.c_double = false; g.c_rs = kc; g.c_cs = 1;
     g.status = c.status;
     g.tag = "adjoint_gram_op";
+    g.pdl = true;
     umma_gemm(g, st);
   };
   DBuf<double> scal((size_t)2 * kc), beta(kc), pq(kc), part((size_t)kCgBlocks * kc);
@@ -769,15 +779,27 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
   double *hpin = Runtime::get().host_pin;
   const int nb = (int)std::max<long long>(1, std::min<long long>(kCgBlocks, (n + 15) / 16));
   const size_t dsm = (size_t)std::max(kCgThreads, kc) * sizeof(double);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at = pdl_attribute();
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
   auto body = [&](int par) {
     product();
-    cg_apply_kernel<<<nb, kCgThreads, dsm, st>>>(pv.p, z.p, s2.p, q.p, n, kc, part.p, ctl.p, pq.p);
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(kCgThreads);
+    cfg.dynamicSmemBytes = dsm;
+    CK(cudaLaunchKernelEx(&cfg, cg_apply_kernel, (const float *)pv.p, (const float *)z.p, (const float *)s2.p, q.p,
+                          (long long)n, kc, part.p, ctl.p, pq.p));
     KLAUNCHED();
-    cg_update_kernel<<<nb, kCgThreads, dsm, st>>>(x.p, r.p, pv.p, q.p, n, kc, rr, bb, pq.p, beta.p, tol * tol, part.p,
-                                                  ctl.p, hpin + par);
+    CK(cudaLaunchKernelEx(&cfg, cg_update_kernel, x.p, r.p, (const float *)pv.p, (const float *)q.p, (long long)n, kc, rr,
+                          (const double *)bb, (const double *)pq.p, beta.p, tol * tol, part.p, ctl.p, hpin + par));
     KLAUNCHED();
-    cg_next_kernel<<<dim3((unsigned)((n + 63) / 64), (unsigned)((kc + 31) / 32)), 256, 0, st>>>(
-        pv.p, r.p, beta.p, n, kc, ctl.p, xp.buf.p, xp.P.ld, xp.P.plane_stride);
+    cfg.gridDim = dim3((unsigned)((n + 63) / 64), (unsigned)((kc + 31) / 32));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = 0;
+    CK(cudaLaunchKernelEx(&cfg, cg_next_kernel, pv.p, (const float *)r.p, (const double *)beta.p, (long long)n, kc,
+                          (const unsigned *)ctl.p, xp.buf.p, (long long)xp.P.ld, (long long)xp.P.plane_stride));
     KLAUNCHED();
   };
   int its = 0;

@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "pdl.cuh"
 #include "planes.cuh"
 #include "runtime.h"
 #include "umma.h"
@@ -57,6 +58,7 @@ struct KParams {
   __nv_bfloat16 *pl;  // optional bf16 planes of the output (UmmaGemm::planes)
   long long pl_ld, pl_ps;
   int n_group;  // N tiles per column group of the tile order (0: row-major tile order)
+  int pdl;      // UmmaGemm::pdl
   int l2_hint;  // bit 0: B loads evict-last, A loads evict-first; bit 1: A loads evict-last
 };
 
@@ -156,6 +158,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tslot;
+  pdl_wait();
 
   if (warp == 0 && lane == 0) {
     // ---------------------------------------------------------------- TMA producer
@@ -443,6 +446,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     }
   }
+  if (p.pdl) pdl_trigger();
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) atomicExch(p.status, (int)kErrTimeout);
   if (warp == 1) {
@@ -753,6 +757,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // C(b, r, c) = alpha * sum_s partial(b, s, r, c) (FP64 sum); upper: only c >= r.
 __global__ void umma_reduce_kernel(const KParams p) {
+  if (p.pdl) pdl_trigger();
+  pdl_wait();
   // one thread per 4 consecutive columns of a row; the partial of split sp is added into
   // accumulator sp % 8 and the eight are summed pairwise (a fixed order)
   const int n4 = (p.N + 3) >> 2;
@@ -1137,6 +1143,7 @@ void launch_t(const UmmaGemm &g, cudaStream_t st, int *status) {
   int stages = std::min(8, (budget - staging) / stage_bytes);
   p.chunk_kb = g.unbias ? 1 : chunk_kblocks(BK, g.chunk_k);
   p.unbias = g.unbias ? 1 : 0;
+  p.pdl = g.pdl ? 1 : 0;
   // rows of C contiguous (or a split-K partial): stage the epilogue through shared memory when the
   // pipeline buffers can hold the 8 warps' 32 x (BN/2 + 1) blocks
   p.stage_out = (!p.bloop && (p.splits > 1 || g.c_cs == 1) && stages * stage_bytes >= 8 * 32 * (C::HALF + 1) * 4) ? 1 : 0;
@@ -1153,7 +1160,15 @@ void launch_t(const UmmaGemm &g, cudaStream_t st, int *status) {
     CK(cudaEventCreate(&e1));
     CK(cudaEventRecord(e0, st));
   }
-  kern<<<grid, kThreads, smem, st>>>(ma, mb, p, stages);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at = pdl_attribute();
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = g.pdl ? 1 : 0;
+  CK(cudaLaunchKernelEx(&cfg, kern, ma, mb, p, stages));
   KLAUNCHED();
   if (profiling()) {
     CK(cudaEventRecord(e1, st));
@@ -1168,7 +1183,11 @@ void launch_t(const UmmaGemm &g, cudaStream_t st, int *status) {
     const long long groups = (long long)g.M * ((g.N + 3) / 4) * g.batch;
     if (groups >= (1LL << 31)) fail(kErrUnsupported, "tcgen05 GEMM: split-K output too large");
     const int blocks = (int)std::min<long long>((groups + 255) / 256, 16LL * rt.num_sms);
-    umma_reduce_kernel<<<blocks, 256, 0, st>>>(p);
+    cudaLaunchConfig_t rc = cfg;
+    rc.gridDim = dim3(blocks);
+    rc.blockDim = dim3(256);
+    rc.dynamicSmemBytes = 0;
+    CK(cudaLaunchKernelEx(&rc, umma_reduce_kernel, p));
     KLAUNCHED();
   }
 }

@@ -50,6 +50,7 @@ struct UmmaGemm {
   // chain has 5.7e-7 and 7e-7).  A sum that is exact because its operands are short (integers) has an even
   // last place and stays exact.
   bool unbias = false;
+  bool pdl = false;  // programmatic dependent launch (pdl.cuh): between the short kernels of a loop
   const char *tag = "gemm";  // name under which launches are recorded when profiling is enabled
   int *status = nullptr;     // device status word: set, the call returns without a host synchronisation
   // Optional output as three bf16 planes: element (i, j) of batch b, in the output type (FP32, or

@@ -337,11 +337,17 @@ __global__ void __launch_bounds__(1024)
     if (lane == 0) nrm[j] = sqrt(a);
   }
   __syncthreads();
-  // sort by singular value descending; write U = X / s and V (row-major)
+  // sort by singular value descending, NaN first; write U = X / s and V (row-major).  The ranks are a
+  // permutation whatever B holds, so that every entry of rnk is written
   for (int j = tid; j < n; j += nt) {
     const double sj = nrm[j];
+    const bool nj = isnan(sj);
     int rank = 0;
-    for (int k = 0; k < n; ++k) rank += (nrm[k] > sj) || (nrm[k] == sj && k < j);
+    for (int k = 0; k < n; ++k) {
+      const double sk = nrm[k];
+      const bool nk = isnan(sk);
+      rank += nk != nj ? nk : ((!nk && sk > sj) || ((nk || sk == sj) && k < j));
+    }
     s[rank] = sj;
     rnk[rank] = j;
   }

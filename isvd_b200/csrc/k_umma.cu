@@ -309,10 +309,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         tmem_wait();
         if (p.unbias) {
           // half a unit in the last place for a 32-deep chunk, three quarters for a 64-deep one, on
-          // average over the values with an odd last place (UmmaGemm::unbias)
+          // average over the values with an odd last place (UmmaGemm::unbias).  The largest value and what
+          // lies above it (infinity; NaN, which is 0x7fffffff here) stay as they are
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const uint32_t odd = v[i] & 1u;
+            const uint32_t odd = (v[i] << 1) < 0xfefffffeu ? v[i] & 1u : 0u;
             v[i] += BK == 64 ? odd + (odd & (v[i] >> 1)) : odd;
           }
         }

@@ -151,6 +151,7 @@ bool gemm_f32_planes(const Gemm<float, Tout> &g, bool a_kc, bool b_nc, cudaStrea
   u.tag = "fp32";
   u.chunk_k = f32_chunk();
   six_products(u);
+  u.unbias = g.unbias;
   PlaneBuf pa, pb;
   try {
     if (nb > 1) {

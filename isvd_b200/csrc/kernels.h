@@ -29,6 +29,9 @@ struct Gemm {
   // C symmetric (M == N, A = B'): tiles entirely below the diagonal are not computed; the caller
   // completes C with mirror_upper
   bool upper = false;
+  // FP32 by planes: UmmaGemm::unbias.  Off for products whose common scale does not matter (sketches), which
+  // then return sums of one term to the last bit
+  bool unbias = true;
   // FP64 tensor-core path without split-K only (dmma_gemm, splits == 1, M % 64 == 0): batch
   // pl_batch's output C(i, j) is also written as three bf16 planes of its transpose, piece q at
   // pl_t[q pl_ps + j pl_ld + i] (as split_planes(.., transpose = true) splits it)

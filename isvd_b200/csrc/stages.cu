@@ -79,6 +79,7 @@ void sketch_dev(const StageCtx &c, int m, int n, int Nl, char ordera, const T *a
     g.A = ap; set_a(g, ordera, ld, false);
     g.B = omega; g.b_rs = ldom; g.b_cs = 1;
     g.C = y + r0 * ldy; g.c_rs = ldy; g.c_cs = 1;
+    g.unbias = false;
     gemm(g, c.st);
   };
   if (c.a_panel_rows > 0 && !is_device_pointer(a))  // out-of-core A: Y's rows panel by panel

@@ -48,7 +48,8 @@ struct UmmaGemm {
   // quarters of a unit in the last place, back to the chunks whose last place is odd: measured bias
   // below 8e-9, rms error unchanged (1.2e-7 to 1.5e-7 at K = 2048 and 20000, where a round-to-nearest FP32
   // chain has 5.7e-7 and 7e-7).  A sum that is exact because its operands are short (integers) has an even
-  // last place and stays exact.
+  // last place and stays exact; one that is exact with all 24 bits (a single term) moves by one or two units in
+  // the last place when that is odd.  NaN, infinities and the largest value are left alone.
   bool unbias = false;
   bool pdl = false;  // programmatic dependent launch (pdl.cuh): between the short kernels of a loop
   const char *tag = "gemm";  // name under which launches are recorded when profiling is enabled

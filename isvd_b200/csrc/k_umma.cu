@@ -57,6 +57,7 @@ struct KParams {
   int vec_out;    // direct epilogue stores as 16-byte vectors (C rows contiguous and aligned)
   __nv_bfloat16 *pl;  // optional bf16 planes of the output (UmmaGemm::planes)
   long long pl_ld, pl_ps;
+  int gx;       // N tiles
   int n_group;  // N tiles per column group of the tile order (0: row-major tile order)
   int pdl;      // UmmaGemm::pdl
   int l2_hint;  // bit 0: B loads evict-last, A loads evict-first; bit 1: A loads evict-last
@@ -116,13 +117,15 @@ __global__ void __launch_bounds__(kThreads, 1)
   volatile int *abort_flag = (volatile int *)(tslot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int nt = blockIdx.x, mt = blockIdx.y;
-  if (p.n_group > 0 && p.n_group < (int)gridDim.x) {
+  // the tiles of a batch run along grid.x, N tiles fastest (grid.y would end at 65535 M tiles)
+  const unsigned gx = (unsigned)p.gx;
+  int mt = (int)(blockIdx.x / gx), nt = (int)(blockIdx.x - (unsigned)mt * gx);
+  if (p.n_group > 0 && p.n_group < p.gx) {
     // column-grouped tile order: the linear block index walks group g's n_group N tiles (fastest)
     // for every M tile, then group g + 1; the last group may be narrower
-    const unsigned L = blockIdx.y * gridDim.x + blockIdx.x, span = (unsigned)p.n_group * gridDim.y;
+    const unsigned L = blockIdx.x, span = (unsigned)p.n_group * (gridDim.x / gx);
     const unsigned g = L / span, r = L - g * span;
-    const unsigned w = min((unsigned)p.n_group, gridDim.x - g * (unsigned)p.n_group);
+    const unsigned w = min((unsigned)p.n_group, gx - g * (unsigned)p.n_group);
     mt = (int)(r / w);
     nt = (int)(g * (unsigned)p.n_group + r % w);
   }
@@ -1154,7 +1157,9 @@ void launch_t(const UmmaGemm &g, cudaStream_t st, int *status) {
   static_assert(kThreads == 64 + 32 * kEpiWarps, "warp roles");
   auto kern = umma_gemm_kernel<BN, BK, AMN, BMN>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid(gx, gy, p.bloop ? 1 : g.batch * p.splits);
+  if ((long long)gx * gy >= (1LL << 31)) fail(kErrUnsupported, "tcgen05 GEMM: too many output tiles");
+  p.gx = gx;
+  dim3 grid((unsigned)gx * (unsigned)gy, 1, p.bloop ? 1 : g.batch * p.splits);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (profiling()) {
     CK(cudaEventCreate(&e0));

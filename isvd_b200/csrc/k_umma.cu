@@ -945,13 +945,15 @@ void launch_split(const T *src, long long s_rs, long long s_cs, long long rows, 
 
 // Transposed: plane(c, r) = piece(src(r, c)) through a 64 (r) x 32 (c) shared tile; each thread
 // writes 8 consecutive r of one output row c (16-byte vectors).  Plane rows beyond cols and
-// columns beyond rows are zeroed separately.
+// columns beyond rows are zeroed separately.  The tiles run along grid.x, the gx tiles of r fastest (grid.y
+// would end at 65535 tiles of c).
 template <class T>
 __global__ void split_t_kernel(const T *__restrict__ src, long long s_rs, long long s_cs, long long rows,
                                long long cols, long long rows_pad, int np, __nv_bfloat16 *__restrict__ dst,
-                               long long ld, long long ps) {
+                               long long ld, long long ps, unsigned gx) {
   __shared__ T tile[64][33];
-  const long long r0 = (long long)blockIdx.x * 64, c0 = (long long)blockIdx.y * 32;
+  const unsigned by = blockIdx.x / gx;
+  const long long r0 = (long long)(blockIdx.x - by * gx) * 64, c0 = (long long)by * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
   for (int j = ty; j < 64; j += 8) {
     const long long r = r0 + j, c = c0 + tx;
@@ -974,6 +976,16 @@ __global__ void split_t_kernel(const T *__restrict__ src, long long s_rs, long l
     for (int q = 0; q < 3; ++q)
       if (q < np) *(uint4 *)(dst + q * ps + c * ld + rr) = pack8(o[q]);
   }
+}
+
+template <class T>
+void launch_split_t(const T *src, long long s_rs, long long s_cs, long long rows, long long cols, long long rows_pad,
+                    int np, __nv_bfloat16 *dst, long long ld, long long ps, cudaStream_t st) {
+  const long long gx = (rows + 63) / 64, gy = (cols + 31) / 32;
+  if (gx * gy >= (1LL << 31)) fail(kErrUnsupported, "split of a transpose: too many tiles");
+  split_t_kernel<T><<<(unsigned)(gx * gy), 256, 0, st>>>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, ps,
+                                                         (unsigned)gx);
+  KLAUNCHED();
 }
 
 // Philox4x32-10 + Box-Muller (same stream as rng_gaussian in k_misc.cu), rounded to bf16 and
@@ -1286,9 +1298,7 @@ void split_planes(const T *src, long long s_rs, long long s_cs, long long rows, 
                              st));
     }
     if (ld % 8) fail(kErrArgument, "split_planes: ld must be a multiple of 8");
-    dim3 grid((unsigned)((rows + 63) / 64), (unsigned)((cols + 31) / 32));
-    split_t_kernel<T><<<grid, 256, 0, st>>>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, plane_stride);
-    KLAUNCHED();
+    launch_split_t<T>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, plane_stride, st);
   }
 }
 
@@ -1303,9 +1313,7 @@ void split_rows(const T *src, long long s_rs, long long s_cs, long long rows, lo
     // output rows = cols of src, output columns = rows of src; the grid covers ld when
     // ld == roundup(rows, 64)
     if (ld != (rows + 63) / 64 * 64) fail(kErrArgument, "split_rows: transposed rows need ld = roundup(rows, 64)");
-    dim3 grid((unsigned)((rows + 63) / 64), (unsigned)((cols + 31) / 32));
-    split_t_kernel<T><<<grid, 256, 0, st>>>(src, s_rs, s_cs, rows, cols, cols, np, dst, ld, plane_stride);
-    KLAUNCHED();
+    launch_split_t<T>(src, s_rs, s_cs, rows, cols, cols, np, dst, ld, plane_stride, st);
   }
 }
 template void split_rows<float>(const float *, long long, long long, long long, long long, int, bool, __nv_bfloat16 *,

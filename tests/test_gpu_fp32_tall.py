@@ -54,3 +54,12 @@ def test_stages_row_major(lib, tall, alg):
     lib.integrate("s", "KN", prm, q, nl, qt, L, argv=[2, 1e-9])
     assert lib.last_error()[0] == 0
     assert _worst(qt, q, torch.linalg.solve(_gram(q, q), _gram(q, qt))) <= 32 * U
+
+
+def test_sketch_column_major(lib, tall):
+    """The columns' planes are split through tiles of 32 rows of A."""
+    nl = L * NS
+    y = torch.zeros(M, nl, device="cuda")
+    lib.sketch("s", lib.create_param(M, N_COLS, L, 0, NS), tall.t().contiguous(), M, y, nl, 3, ordera=b"C")
+    assert lib.last_error()[0] == 0
+    assert _worst(y, tall, _omega(lib, N_COLS, nl, 3)) <= 13 * U

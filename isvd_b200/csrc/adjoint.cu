@@ -146,10 +146,9 @@ __global__ void cg_step2_kernel(T *p, const T *__restrict__ r, long long rows, i
 constexpr int kCgThreads = 512;
 constexpr int kCgBlocks = 128;
 
-// acc: this thread's sums of columns c0 + t % cw over its rows; adds the CTA's slices and, in the last CTA,
-// all of them (fin: column, sum).
+// Adds the CTAs' slices in the last CTA (fin: column, sum; one thread per column).
 template <class F>
-__device__ __forceinline__ void cg_dot_finish(double *sh, int kc, double *partial, unsigned *ctl, F fin) {
+__device__ __forceinline__ void cg_dot_finish(int kc, double *partial, unsigned *ctl, F fin) {
   __shared__ bool last;
   __threadfence();
   __syncthreads();
@@ -170,18 +169,18 @@ __device__ __forceinline__ void cg_dot_finish(double *sh, int kc, double *partia
         const int b = lane + 32 * w;
         v[u][w] = (c0 + u < kc && b < (int)gridDim.x) ? __ldcg(partial + (size_t)b * kc + c0 + u) : 0.0;
       }
+    double mine = 0.0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       double s = v[u][0];
 #pragma unroll
       for (int w = 1; w < kSl; ++w) s += v[u][w];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      if (lane == 0 && c0 + u < kc) sh[c0 + u] = s;
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == u) mine = s;
     }
+    if (lane < 4 && c0 + lane < kc) fin(c0 + lane, mine);
   }
-  __syncthreads();
-  for (int c = threadIdx.x; c < kc; c += kCgThreads) fin(c, sh[c]);
 }
 
 // Rows of this CTA; prep(column) returns f with f.load(element) and f.apply(element, loaded), which stores
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(kCgThreads)
     cg_apply_kernel(const float *__restrict__ p, const float *__restrict__ z, const float *__restrict__ s,
                     float *__restrict__ q,
                     long long rows, int kc, double *partial, unsigned *ctl, double *pq) {
-  extern __shared__ double sh[];
+  __shared__ double sh[kCgThreads];
   pdl_trigger();
   pdl_wait();
   if (((volatile unsigned *)ctl)[1]) return;
@@ -255,14 +254,14 @@ __global__ void __launch_bounds__(kCgThreads)
     const double sc = s[c];
     return CgApply{p, z, q, sc * sc};
   });
-  cg_dot_finish(sh, kc, partial, ctl, [&](int c, double v) { pq[c] = v; });
+  cg_dot_finish(kc, partial, ctl, [&](int c, double v) { pq[c] = v; });
 }
 
 __global__ void __launch_bounds__(kCgThreads)
     cg_update_kernel(float *__restrict__ x, float *__restrict__ r, const float *__restrict__ p, const float *__restrict__ q, long long rows, int kc,
                      double *rr, const double *__restrict__ bb, const double *__restrict__ pq, double *beta, double tol2,
                      double *partial, unsigned *ctl, double *host_done) {
-  extern __shared__ double sh[];
+  __shared__ double sh[kCgThreads];
   __shared__ int above;
   pdl_trigger();
   pdl_wait();
@@ -272,7 +271,7 @@ __global__ void __launch_bounds__(kCgThreads)
   });
   if (threadIdx.x == 0) above = 0;
   bool mine = false;  // this CTA is the last one
-  cg_dot_finish(sh, kc, partial, ctl, [&](int c, double v) {
+  cg_dot_finish(kc, partial, ctl, [&](int c, double v) {
     beta[c] = rr[c] > 0.0 ? v / rr[c] : 0.0;
     rr[c] = v;
     if (v > tol2 * bb[c]) above = 1;
@@ -778,7 +777,6 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
   // the launches of i + 1 find the done word set and leave x as it is.
   double *hpin = Runtime::get().host_pin;
   const int nb = (int)std::max<long long>(1, std::min<long long>(kCgBlocks, (n + 15) / 16));
-  const size_t dsm = (size_t)std::max(kCgThreads, kc) * sizeof(double);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at = pdl_attribute();
   cfg.stream = st;
@@ -788,7 +786,6 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
     product();
     cfg.gridDim = dim3(nb);
     cfg.blockDim = dim3(kCgThreads);
-    cfg.dynamicSmemBytes = dsm;
     CK(cudaLaunchKernelEx(&cfg, cg_apply_kernel, (const float *)pv.p, (const float *)z.p, (const float *)s2.p, q.p,
                           (long long)n, kc, part.p, ctl.p, pq.p));
     KLAUNCHED();
@@ -797,7 +794,6 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
     KLAUNCHED();
     cfg.gridDim = dim3((unsigned)((n + 63) / 64), (unsigned)((kc + 31) / 32));
     cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = 0;
     CK(cudaLaunchKernelEx(&cfg, cg_next_kernel, pv.p, (const float *)r.p, (const double *)beta.p, (long long)n, kc,
                           (const unsigned *)ctl.p, xp.buf.p, (long long)xp.P.ld, (long long)xp.P.plane_stride));
     KLAUNCHED();

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(WM * WN * 32)
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   if (g.upper && n0 + BN <= m0) return;  // tile strictly below the diagonal: mirrored by the caller
   // (128 x 128 tiles) computed on the int8 tensor cores already (k_i8.cu)
-  if (g.done_a && g.done_a[blockIdx.x] * g.done_b[blockIdx.y] <= g.done_lim) return;
+  if (g.done && g.done[(size_t)blockIdx.x * gridDim.y + blockIdx.y] >= g.done_need) return;
   const int b = blockIdx.z / splits, sp = blockIdx.z % splits;
   const int kb = sp * kchunk, ke = min(g.K, kb + kchunk);
 
@@ -502,10 +502,10 @@ bool dmma_apply_in_place(const Gemm<double, double> &g, cudaStream_t st) {
   return true;
 }
 
-void dmma_gemm_rest(const Gemm<double, double> &g, bool a_kc, bool b_nc, const float *done_a, const float *done_b,
-                    float lim, cudaStream_t st) {
+void dmma_gemm_rest(const Gemm<double, double> &g, bool a_kc, bool b_nc, const unsigned long long *done,
+                    unsigned long long need, cudaStream_t st) {
   Gemm<double, double> f = g;
-  f.done_a = done_a; f.done_b = done_b; f.done_lim = lim;
+  f.done = done; f.done_need = need;
   f.splits = 1;
   dmma_launch<128, 128, 2, 4>(f, a_kc, b_nc, st);
 }

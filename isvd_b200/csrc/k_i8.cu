@@ -8,18 +8,23 @@
 // eA_i is the exponent of the row's (eB_j: the column's) largest entry, so an entry keeps 55 bits below
 // it; the inner sums are exact in int32 (at most 16384 terms at a time), and what is left out, the digit
 // pairs with p + q >= 7 and the bits below 2^-55, is a random error of about 2^-56.3 sqrt(K) 2^eA 2^eB,
-// where a chain of K FP64 multiply-adds makes about 2^-54.5 K rms(a_i) rms(b_j).  A tile is computed here
-// when the bound is below the other for each of its rows and columns,
+// where a chain of K FP64 multiply-adds makes about 2^-54 sum_k |a_ik| |b_kj| (Gaussian: 2^-54.5 K rms(a_i)
+// rms(b_j)).  A tile is computed here when the one is below the other for each of its entries.  First by rows
+// and columns, from their splits,
 //   max_i (2^eA_i / rms a_i) max_j (2^eB_j / rms b_j) <= 2.5 sqrt(K)                       (*)
-// (Gaussian rows: 8 x 8 against 2.5 sqrt(K), so from K = 655 on); rows with outliers, zeros for most
-// entries, exponents beyond 2^400, infinities or NaN fail it, and their tiles are computed by the FP64
-// tensor-core kernel (k_dmma.cu), which is launched behind and skips the others.  Both decide from the
-// same two words per tile; the host does not wait.
+// (Gaussian rows: 8 x 8 against 2.5 sqrt(K), so from K = 655 on): rows with outliers, zeros for most entries,
+// exponents beyond 2^400, infinities or NaN fail it.  Then by entries, from the product of the leading bits
+// m = floor(|x| 2^(7 - e)), an eighth plane that takes the fourth accumulator of the second pass,
+//   2^-14 sum_k m(a_ik) m(b_kj) >= 0.2 sqrt(K)      (then the error is below 2^-54 sum |a_ik| |b_kj|)   (**)
+// which operands graded against each other fail (large entries of a row meeting small ones of a column:
+// all terms are small, and so is the chain's error).  The tiles that fail are computed by the FP64 tensor-core
+// kernel (k_dmma.cu), which is launched behind and skips the others: both go by the tile's sum over the
+// splits of the smallest sum in (**), zero where (*) failed; the host does not wait.
 //
 // One CTA per 128 x 128 tile (and K split, where the tiles alone leave SMs idle): warp 0 moves 64-byte deep
 // blocks of the digit planes by TMA (two stages of 14 planes), warp 1 issues the MMAs, warps 2..9 drain.
 // The seven sums s need 7 x 128 TMEM columns of 512, so a K chunk runs in two passes: s = 3..6 (22 products
-// of the 28, all 14 planes), then s = 0..2 (6 products, the three leading planes of either side).  The
+// of the 28, all 14 planes), then s = 0..2 (6 products, the three leading planes of either side) and (**).  The
 // drained int32 sums of a pass combine exactly in int64 and join the FP64 running sums in registers.
 //
 // Measured, mma.sync f64 -> here with the digits: 40000 x 1536 x 6000 26.6 -> 7.8 ms (6.6 ms of products at
@@ -45,6 +50,9 @@ namespace isvdb {
 namespace {
 
 constexpr int kSlices = 7;
+constexpr int kPlanes = kSlices + 1;                // and the leading bits of the magnitudes
+constexpr int kLead = 4;                            // planes per side of the second pass
+constexpr int kZeroRow = 1 << 20;                   // in place of a zero row's exponent
 constexpr int kTile = 128, kBk = 64;
 constexpr int kPlane = kTile * kBk;                 // bytes of one plane's tile
 constexpr int kStage = 2 * kSlices * kPlane;        // 112 KB
@@ -63,6 +71,8 @@ struct I8Params {
   const int *ea, *eb;          // exponents of the rows and columns
   const float *ra, *rb;        // 128-row (128-column) maxima of 2^e / rms
   float lim;
+  unsigned long long *sum;     // per tile (N tiles fastest): the left side of (**) over the splits, in units of 2^-14
+  unsigned long long need;     // its right side
   int *status;
 };
 
@@ -82,20 +92,28 @@ __device__ __forceinline__ void tmem_ld8i(uint32_t taddr, int *r) {
                : "r"(taddr));
 }
 
-__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+// 2^e of a row's exponent (anything for a zero row)
+__device__ __forceinline__ double pow2(int e) {
+  if (e == kZeroRow) e = 0;
+  return __longlong_as_double((long long)(e + 1023) << 52);
+}
 
-// The products of one pass: LO <= p + q <= HI, accumulator p + q - LO.
-template <int NS, int LO, int HI>
+// The products of one pass: LO <= p + q <= HI, accumulator p + q - LO; MAG: the last planes' product too, in
+// the accumulator behind.
+template <int NS, int LO, int HI, bool MAG>
 __device__ __forceinline__ void issue_pass(uint32_t tmem, uint64_t base, uint32_t more) {
+  constexpr int ND = MAG ? NS - 1 : NS;
 #pragma unroll
   for (int p = 0; p < NS; ++p)
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-      if (p + q < LO || p + q > HI) continue;
+      const bool mag = MAG && p == ND && q == ND;
+      if (!mag && (p >= ND || q >= ND || p + q < LO || p + q > HI)) continue;
+      const uint32_t d = tmem + (uint32_t)((mag ? HI + 1 - LO : p + q - LO) * kTile);
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk)
-        umma_i8(tmem + (uint32_t)((p + q - LO) * kTile), base + (uint32_t)(p * kPlane >> 4) + kk * 2,
-                base + (uint32_t)((NS + q) * kPlane >> 4) + kk * 2, kIdesc, (p > 0 || kk > 0) ? 1u : more);
+        umma_i8(d, base + (uint32_t)(p * kPlane >> 4) + kk * 2, base + (uint32_t)((NS + q) * kPlane >> 4) + kk * 2, kIdesc,
+                kk > 0 || (p > 0 && !mag) ? 1u : more);
     }
 }
 
@@ -104,8 +122,9 @@ __global__ void __launch_bounds__(kI8Threads, 1)
   const int nt = blockIdx.x, mt = blockIdx.y;
   const int m0 = mt * kTile, n0 = nt * kTile;
   if (p.upper && n0 + kTile <= m0) return;            // tile strictly below the diagonal: mirrored later
-  if (!(p.ra[mt] * p.rb[nt] <= p.lim)) return;        // (*) fails: the FP64 kernel computes this tile
+  if (!(p.ra[mt] * p.rb[nt] <= p.lim)) return;        // (*) fails (the tile's sum stays zero)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ unsigned least[8];  // of each epilogue warp, the smallest sum of (**)
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t *full = (uint64_t *)(smem + (size_t)kStages * kStage);
   uint64_t *empty = full + kStages;
@@ -143,7 +162,7 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     uint32_t ph = 1;
     for (int c = 0; c < nchunks && !*abort_flag; ++c)
       for (int pass = 0; pass < 2 && !*abort_flag; ++pass) {
-        const int ns = pass == 0 ? kSlices : 3;
+        const int ns = pass == 0 ? kSlices : kLead;
         const int kb1 = min(nkb, (c + 1) * kChunkBlocks);
         for (int kb = c * kChunkBlocks; kb < kb1; ++kb) {
           if (issued >= kStages && !mbar_try(&empty[s], ph) && !mbar_wait(&empty[s], ph, abort_flag)) {
@@ -152,8 +171,10 @@ __global__ void __launch_bounds__(kI8Threads, 1)
           }
           uint8_t *st = smem + (size_t)s * kStage;
           mbar_expect_tx(&full[s], (uint32_t)(2 * ns * kPlane));
-          for (int q = 0; q < ns; ++q) tma_load_3d(st + q * kPlane, &mapA, &full[s], (kfirst + kb) * kBk, m0, q);
-          for (int q = 0; q < ns; ++q) tma_load_3d(st + (ns + q) * kPlane, &mapB, &full[s], (kfirst + kb) * kBk, n0, q);
+          auto plane = [&](int q) { return q == kLead - 1 && pass ? kSlices : q; };
+          for (int q = 0; q < ns; ++q) tma_load_3d(st + q * kPlane, &mapA, &full[s], (kfirst + kb) * kBk, m0, plane(q));
+          for (int q = 0; q < ns; ++q)
+            tma_load_3d(st + (ns + q) * kPlane, &mapB, &full[s], (kfirst + kb) * kBk, n0, plane(q));
           ++issued;
           if (++s == kStages) {
             s = 0;
@@ -189,8 +210,8 @@ __global__ void __launch_bounds__(kI8Threads, 1)
           }
           tc_fence_after();
           const uint64_t base = d0 + (uint64_t)(smem16 + (uint32_t)s * (kStage >> 4));
-          if (pass == 0) issue_pass<kSlices, 3, 6>(tmem, base, kb > kb0);
-          else issue_pass<3, 0, 2>(tmem, base, kb > kb0);
+          if (pass == 0) issue_pass<kSlices, 3, 6, false>(tmem, base, kb > kb0);
+          else issue_pass<kLead, 0, 2, true>(tmem, base, kb > kb0);
           umma_commit(&empty[s]);
           if (++s == kStages) {
             s = 0;
@@ -206,6 +227,12 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     double acc[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) acc[j] = 0.0;
+    // the entries that (**) is asked of: not the padding, and not zero rows or columns, whose products are exact
+    const int row = m0 + q * 32 + lane, col = n0 + h * 64 + lane;
+    const bool ask = row < p.M && p.ea[row] != kZeroRow;
+    const unsigned cols0 = __ballot_sync(0xffffffffu, col < p.N && p.eb[col] != kZeroRow);
+    const unsigned cols1 = __ballot_sync(0xffffffffu, col + 32 < p.N && p.eb[col + 32] != kZeroRow);
+    unsigned long long sum = 0;  // over the chunks, of the smallest of this thread's entries
     bool ok = true;
     for (int t = 0; t < 2 * nchunks; ++t) {
       int okw = 0;
@@ -232,28 +259,34 @@ __global__ void __launch_bounds__(kI8Threads, 1)
                                    (long long)a6[i]);
         }
       } else {
+        int low = 0x7fffffff;
 #pragma unroll
         for (int j = 0; j < 64; j += 8) {
-          int a0[8], a1[8], a2[8];
+          int a0[8], a1[8], a2[8], mm[8];
           tmem_ld8i(tb + j, a0);
           tmem_ld8i(tb + kTile + j, a1);
           tmem_ld8i(tb + 2 * kTile + j, a2);
+          tmem_ld8i(tb + 3 * kTile + j, mm);
           tmem_wait();
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
+          for (int i = 0; i < 8; ++i) {
             acc[j + i] = fma((double)(((long long)a0[i] << 16) + ((long long)a1[i] << 8) + (long long)a2[i]), 0x1p32,
                              acc[j + i]);
+            if (((j < 32 ? cols0 : cols1) >> ((j + i) & 31)) & 1u) low = min(low, mm[i]);
+          }
         }
+        sum += (unsigned)low;
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(tempty)) : "memory");
     }
+    const unsigned small = __reduce_min_sync(0xffffffffu, ask ? (unsigned)min(sum, 0xffffffffull) : 0xffffffffu);
+    if (lane == 0) least[warp - 2] = small;
     if (ok) {
       // every MMA has completed, so the pipeline buffers are free: whole rows through them
       constexpr int SROW = 65;
       double *stg = (double *)smem + (size_t)(warp - 2) * 32 * SROW;
-      const int row = m0 + q * 32 + lane;
       // the sums count units of 2^(48 - 110)
       const double sa = row < p.M ? p.alpha * 0x1p-62 * pow2(p.ea[row]) : 0.0;
 #pragma unroll
@@ -276,6 +309,12 @@ __global__ void __launch_bounds__(kI8Threads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (threadIdx.x == 0 && !*abort_flag) {
+    unsigned low = least[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) low = min(low, least[i]);
+    atomicAdd(p.sum + (size_t)mt * gridDim.x + nt, (unsigned long long)low);
+  }
   if (warp == 1) {
     if (*abort_flag && lane == 0) {
       atomicExch(p.status, kErrTimeout);
@@ -294,7 +333,7 @@ __global__ void __launch_bounds__(256) i8_reduce_kernel(const I8Params p, int sp
   const long long total = (long long)p.M * p.N;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
     const int r = (int)(i / p.N), c = (int)(i - (long long)r * p.N);
-    if ((p.upper && c < r) || !(p.ra[r >> 7] * p.rb[c >> 7] <= p.lim)) continue;
+    if ((p.upper && c < r) || p.sum[(size_t)(r >> 7) * ((p.N + 127) >> 7) + (c >> 7)] < p.need) continue;
     double v = 0.0;
     for (int z = 0; z < splits; ++z) v += p.C[z * p.c_zs + i];
     C[r * c_rs + c * c_cs] = v;
@@ -320,12 +359,14 @@ __device__ __forceinline__ bool digit_exponent(double mx, int &e) {
 }
 
 // Digits of four entries, plane p's four bytes in w[p]; scale = 2^(55 - e).  With 128 added to each of the
-// six lower digits' places, the digits are the bytes less 128.
+// six lower digits' places, the digits are the bytes less 128.  The leading bits of the magnitudes go to w[7].
 __device__ __forceinline__ void digits4(const double *x, double scale, uint32_t *w) {
   uint32_t lo[4], hi[4];
+  w[7] = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const long long y = __double2ll_rn(x[i] * scale) + 0x808080808080LL;
+    const long long z = __double2ll_rn(x[i] * scale), y = z + 0x808080808080LL;
+    w[7] |= (uint32_t)((unsigned long long)(z < 0 ? -z : z) >> 48) << (8 * i);
     lo[i] = (uint32_t)y;
     hi[i] = (uint32_t)((unsigned long long)y >> 32);
   }
@@ -343,11 +384,11 @@ __device__ __forceinline__ void digits4(const double *x, double scale, uint32_t 
 
 // Digits of eight consecutive entries, stored to the planes at dst (8-byte aligned).
 __device__ __forceinline__ void store_digits8(const double *x, double scale, int8_t *dst, long long ps) {
-  uint32_t u[kSlices], v[kSlices];
+  uint32_t u[kPlanes], v[kPlanes];
   digits4(x, scale, u);
   digits4(x + 4, scale, v);
 #pragma unroll
-  for (int p = 0; p < kSlices; ++p) *(uint2 *)(dst + p * ps) = make_uint2(u[p], v[p]);
+  for (int p = 0; p < kPlanes; ++p) *(uint2 *)(dst + p * ps) = make_uint2(u[p], v[p]);
 }
 
 __device__ __forceinline__ void max_ratio(float *slot, float r) {  // r >= 0: ordered as integers
@@ -401,7 +442,7 @@ __global__ void __launch_bounds__(256)
   const bool ok = digit_exponent(mx, e) && !any_nan;  // |e| <= 400: the squares stay in range
   const float rr = !ok ? INFINITY : mx == 0.0 ? 0.f : (float)(ldexp(1.0, e) / sqrt(sq / (double)K));
   if (r < rows && tid == 0) {
-    ex[r] = e;
+    ex[r] = mx == 0.0 ? kZeroRow : e;
     max_ratio(ratio + (r >> 7), rr);
   }
   if (!(rr <= lim)) return;
@@ -458,7 +499,7 @@ __global__ void i8_colexp_kernel(const unsigned long long *__restrict__ mx, cons
   for (int b = 0; b < nb; ++b) sq += sqp[b * cols + c];
   int e;
   const bool ok = digit_exponent(__longlong_as_double((long long)mx[c]), e);
-  ex[c] = e;
+  ex[c] = mx[c] == 0 ? kZeroRow : e;
   max_ratio(ratio + (c >> 7), !ok ? INFINITY : mx[c] == 0 ? 0.f : (float)(ldexp(1.0, e) / sqrt(sq / K)));
 }
 
@@ -478,7 +519,8 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   const int cl = threadIdx.x >> 3, seg = threadIdx.x & 7;
   const long long c = c0 + cl;
-  const double scale = ldexp(1.0, 55 - (c < cols ? ex[c] : 0));
+  const int e = c < cols ? ex[c] : 0;
+  const double scale = ldexp(1.0, 55 - (e == kZeroRow ? 0 : e));
   double x[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) x[i] = tile[8 * seg + i][cl];
@@ -501,7 +543,7 @@ void make_digits(Digits &d, const double *src, long long ld, long long rows, lon
   d.rows = rows;
   d.ld = (K + 63) / 64 * 64;
   d.ps = rp * d.ld;
-  d.buf.ensure((size_t)kSlices * d.ps);
+  d.buf.ensure((size_t)kPlanes * d.ps);
   d.ex.ensure(rp);
   d.ratio.ensure(rp / 128);
   CK(cudaMemsetAsync(d.ratio.p, 0, rp / 128 * sizeof(float), st));
@@ -542,7 +584,7 @@ CUtensorMap digit_map(const Digits &d) {
   CUtensorMap m;
   memset(&m, 0, sizeof(m));
   // the padding rows and columns are stored (zero digits), so every box lies inside
-  cuuint64_t dims[3] = {(cuuint64_t)d.ld, (cuuint64_t)pad128(d.rows), (cuuint64_t)kSlices};
+  cuuint64_t dims[3] = {(cuuint64_t)d.ld, (cuuint64_t)pad128(d.rows), (cuuint64_t)kPlanes};
   cuuint64_t strides[2] = {(cuuint64_t)d.ld, (cuuint64_t)d.ps};
   cuuint32_t box[3] = {kBk, kTile, 1}, es[3] = {1, 1, 1};
   const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void *)d.buf.p, dims, strides, box, es,
@@ -571,11 +613,11 @@ int i8_splits(double M, double N, double K, bool upper) {
   return best;
 }
 
-// Either path's time: 26 TFLOP/s on mma.sync f64; here also 23 bytes per split element at about 4 TB/s, and
+// Either path's time: 26 TFLOP/s on mma.sync f64; here also 24 bytes per split element at about 4 TB/s, and
 // 60 us of launches.
 bool i8_pays(double M, double N, double K, bool same, bool upper) {
   const double dmma = (upper ? 0.55 : 1.0) * 2.0 * M * N * K / 26e12;
-  const double i8 = i8_gemm_time(M, N, K, upper, i8_splits(M, N, K, upper)) + (same ? M : M + N) * K * 23.0 / 4e12 + 60e-6;
+  const double i8 = i8_gemm_time(M, N, K, upper, i8_splits(M, N, K, upper)) + (same ? M : M + N) * K * 24.0 / 4e12 + 60e-6;
   return i8 < 0.8 * dmma;
 }
 
@@ -597,12 +639,13 @@ bool gemm_f64_int8(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStre
   long long cap = 4LL << 30;
   if (isvd_gpu_memory_limit > 0)
     cap = std::max<long long>(32LL << 20, std::min<long long>(cap, (long long)(isvd_gpu_memory_limit / 16)));
-  const long long ld = (g.K + 63) / 64 * 64, per = kSlices * ld;
+  const long long ld = (g.K + 63) / 64 * 64, per = kPlanes * ld;
   // rows of A at a time (a multiple of 128); the digits of B (or of A = B') are held whole
   const long long step = same ? g.M : std::min<long long>(g.M, std::max<long long>(128, cap / per / 128 * 128));
   if (per * pad128(g.N) > 3 * cap) return false;
   const float lim = (float)(2.5 * std::sqrt((double)g.K));
   Digits da, db;
+  DBuf<unsigned long long> sum;
   try {
     make_digits(db, g.B, b_nc ? g.b_rs : g.b_cs, g.N, g.K, !b_nc, lim, st);
     CK(cudaFuncSetAttribute(i8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kI8Smem));
@@ -627,8 +670,13 @@ bool gemm_f64_int8(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStre
       p.upper = g.upper ? 1 : 0;
       p.ea = d.ex.p; p.eb = db.ex.p; p.ra = d.ratio.p; p.rb = db.ratio.p;
       p.lim = lim;
-      p.status = reinterpret_cast<int *>(Runtime::get().ctl + 16);  // the stages' status word
       const dim3 grid((g.N + kTile - 1) / kTile, (rows + kTile - 1) / kTile, nz);
+      const size_t tiles = (size_t)grid.x * grid.y;
+      sum.ensure(tiles);
+      CK(cudaMemsetAsync(sum.p, 0, tiles * sizeof(unsigned long long), st));
+      p.sum = sum.p;
+      p.need = (unsigned long long)std::ceil(0.2 * std::sqrt((double)g.K) * 16384.0);
+      p.status = reinterpret_cast<int *>(Runtime::get().ctl + 16);  // the stages' status word
       i8_gemm_kernel<<<grid, kI8Threads, kI8Smem, st>>>(digit_map(d), mb, p);
       KLAUNCHED();
       if (nz > 1) {
@@ -636,11 +684,11 @@ bool gemm_f64_int8(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStre
         i8_reduce_kernel<<<blocks, 256, 0, st>>>(p, nz, C, g.c_rs, g.c_cs);
         KLAUNCHED();
       }
-      Gemm<double, double> f = g;  // the tiles that fail the bound
+      Gemm<double, double> f = g;  // the tiles that fail (*) or (**)
       f.M = rows;
       f.A = g.A + r0 * (a_kc ? g.a_rs : 1);
       f.C = C;
-      dmma_gemm_rest(f, a_kc, b_nc, d.ratio.p, db.ratio.p, lim, st);
+      dmma_gemm_rest(f, a_kc, b_nc, sum.p, p.need, st);
     }
     return true;
   } catch (const Error &e) {

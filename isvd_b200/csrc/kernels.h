@@ -38,9 +38,9 @@ struct Gemm {
   __nv_bfloat16 *pl_t = nullptr;
   long long pl_ld = 0, pl_ps = 0;
   int pl_batch = 0;
-  // FP64 tensor-core path, 128 x 128 tiles without split-K: skip tile (i, j) when done_a[i] done_b[j] <= done_lim
-  const float *done_a = nullptr, *done_b = nullptr;
-  float done_lim = 0.f;
+  // FP64 tensor-core path, 128 x 128 tiles without split-K: skip tile t (N tiles fastest) when done[t] >= done_need
+  const unsigned long long *done = nullptr;
+  unsigned long long done_need = 0;
 };
 
 template <class T, class Tout>
@@ -98,8 +98,8 @@ void dmma_grouped(const GroupedProd *prods, int nprod, int total, int shape, boo
 // A large FP64 product on the int8 tensor cores (k_i8.cu): true when it was enqueued there.
 // dmma_gemm_rest: the tiles that it leaves to k_dmma.cu.
 bool gemm_f64_int8(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStream_t st);
-void dmma_gemm_rest(const Gemm<double, double> &g, bool a_kc, bool b_nc, const float *done_a, const float *done_b,
-                    float lim, cudaStream_t st);
+void dmma_gemm_rest(const Gemm<double, double> &g, bool a_kc, bool b_nc, const unsigned long long *done,
+                    unsigned long long need, cudaStream_t st);
 
 // ------------------------------------------------------------------ elementwise
 // Omega(j, c) for j < rows, c < cols: standard normal values from Philox4x32-10 (key = seed)

@@ -38,7 +38,7 @@ struct Gemm {
   __nv_bfloat16 *pl_t = nullptr;
   long long pl_ld = 0, pl_ps = 0;
   int pl_batch = 0;
-  // FP64 tensor-core path, 128 x 128 tiles without split-K: skip tile t (N tiles fastest) when done[t] >= done_need
+  // FP64 tensor-core path, 128 x 128 tiles, beta = 0: skip tile t (N tiles fastest) when done[t] >= done_need
   const unsigned long long *done = nullptr;
   unsigned long long done_need = 0;
 };

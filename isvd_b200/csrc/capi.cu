@@ -273,13 +273,13 @@ void sketch_api(const isvd_Param &p, const T *argv, isvd_int_t argc, T *retv, is
     CK(cudaMemcpyAsync(Y.d, Yf.p + (size_t)p.rowidxbegin * Nl, (size_t)m * Nl * sizeof(T), cudaMemcpyDeviceToDevice,
                        c.sc.st));
     Y.back(c.sc.st);
-    sync();
+    read_status(c.sc, "Gaussian projection sketching");
     return;
   }
   sketch_dev<T>(c.sc, m, n, Nl, ordera_, a_use, lda, omega ? Om.d : nullptr, ldomega, (uint64_t)(uint32_t)seed, Y.d,
                 ldyst);
   Y.back(c.sc.st);
-  sync();
+  read_status(c.sc, "Gaussian projection sketching");
 }
 
 template <class T>

@@ -679,6 +679,7 @@ bool gemm_f64_int8(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStre
       p.status = reinterpret_cast<int *>(Runtime::get().ctl + 16);  // the stages' status word
       i8_gemm_kernel<<<grid, kI8Threads, kI8Smem, st>>>(digit_map(d), mb, p);
       KLAUNCHED();
+      inject_timeout("int8", p.status, st);
       if (nz > 1) {
         const int blocks = (int)std::min<long long>(((long long)rows * g.N + 255) / 256, 16LL * Runtime::get().num_sms);
         i8_reduce_kernel<<<blocks, 256, 0, st>>>(p, nz, C, g.c_rs, g.c_cs);

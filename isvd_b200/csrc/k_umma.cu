@@ -1416,6 +1416,7 @@ void umma_gemm(const UmmaGemm &g, cudaStream_t st) {
   } else {
     launch_t<256, 32, false, false>(g, st, status);
   }
+  inject_timeout(g.tag, status, st);
   if (g.status) return;  // the caller checks the status word (no host synchronisation here)
   int h = 0;
   CK(cudaMemcpyAsync(&h, status, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -244,6 +244,11 @@ void copy_to_device(void *dst, size_t dpitch, const void *src, size_t spitch, si
 
 void sync() { CK(cudaStreamSynchronize(Runtime::get().stream)); }
 
+void inject_timeout(const char *tag, int *status, cudaStream_t st) {
+  const char *e = getenv("ISVD_GPU_INJECT_TIMEOUT");
+  if (e && !strcmp(e, tag)) CK(cudaMemsetAsync(status, kErrTimeout, 1, st));  // the low byte
+}
+
 struct ProfEntry {
   double ms = 0.0, flops = 0.0;
   unsigned long long count = 0;

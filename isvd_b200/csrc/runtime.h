@@ -119,6 +119,9 @@ void copy_to_device(void *dst, size_t dpitch, const void *src, size_t spitch, si
 
 void sync();  // synchronise the library stream, converting errors into Error
 
+// Diagnostic: when ISVD_GPU_INJECT_TIMEOUT names `tag`, *status is set as if a wait of that launch had run out.
+void inject_timeout(const char *tag, int *status, cudaStream_t st);
+
 // Multi-rank execution through a caller-provided sum-AllReduce (isvd_gpu_set_allreduce).
 struct Collective {
   void (*fn)(void *, size_t, int, void *, void *) = nullptr;

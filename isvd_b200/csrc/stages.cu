@@ -31,15 +31,17 @@ inline void set_a(G &g, char ordera, long long lda, bool transpose) {
   g.a_rs = rs; g.a_cs = cs;
 }
 
+}  // namespace
+
 void read_status(const StageCtx &c, const char *what) {
   int h = 0;
   CK(cudaMemcpyAsync(&h, c.status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
   if (h == kErrTimeout) fail(kErrTimeout, "%s: a device-side wait timed out", what);
+  if (h == kStatusNotPD)
+    fail(kErrNumerical, "%s: a Cholesky factor broke down (the block is numerically rank deficient)", what);
   if (h) fail(kErrNumerical, "%s: small dense solver reported status %d", what, h);
 }
-
-}  // namespace
 
 // ------------------------------------------------------------------------------------ sketch
 template <class T>

@@ -54,7 +54,10 @@ struct WyArgs {
   double beta = 0.5, sigma = 1e-4, eta = 0.85;
 };
 
-// Y = A * Omega (reference core/stage/@x@_sketch.h:92-146).  omega == nullptr: drawn from seed.
+// Waits for the stage's work and turns its status word into an error.
+void read_status(const StageCtx &c, const char *what);
+
+// Y = A * Omega (reference core/stage/@x@_sketch.h:92-146), enqueued: the caller reads the status.  omega == nullptr: drawn from seed.
 template <class T>
 void sketch_dev(const StageCtx &c, int m, int n, int Nl, char ordera, const T *a, long long lda, const T *omega,
                 long long ldom, uint64_t seed, T *y, long long ldy);

@@ -20,16 +20,6 @@
 namespace isvdb {
 namespace {
 
-void read_status(const StageCtx &c, const char *what) {
-  int h = 0;
-  CK(cudaMemcpyAsync(&h, c.status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
-  CK(cudaStreamSynchronize(c.st));
-  if (h == kErrTimeout) fail(kErrTimeout, "%s: a device-side wait timed out", what);
-  if (h == kStatusNotPD)
-    fail(kErrNumerical, "%s: a Cholesky factor broke down (the block is numerically rank deficient)", what);
-  if (h) fail(kErrNumerical, "%s: small dense solver reported status %d", what, h);
-}
-
 // C = alpha op(A) op(B) + beta C, row-major FP64; op(X) = X' when the flag is set.
 void mul(cudaStream_t st, int M, int N, int K, const double *A, long long lda, bool ta, const double *B,
          long long ldb, bool tb, double *C, long long ldc, double alpha, double beta) {

@@ -1,0 +1,41 @@
+"""A wait that ran out inside a tensor-core product is reported by every entry point that ran it.  The status is
+injected from the host (ISVD_GPU_INJECT_TIMEOUT names the product); the kernels run as always."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+TIMEOUT = 4  # ISVD_GPU_ERROR_TIMEOUT
+
+
+@pytest.fixture
+def inject(monkeypatch):
+    def arm(tag):
+        monkeypatch.setenv("ISVD_GPU_INJECT_TIMEOUT", tag)
+    yield arm
+    monkeypatch.delenv("ISVD_GPU_INJECT_TIMEOUT", raising=False)
+
+
+@pytest.mark.parametrize("x,given,tag", [("s", False, "sketch"), ("s", True, "fp32"), ("d", False, "int8"), ("d", True, "int8")])
+@pytest.mark.parametrize("order", [b"R", b"C"])
+def test_sketch(lib, inject, monkeypatch, x, given, tag, order):
+    m, n, nl = 9000, 1500, 512
+    dt = torch.float32 if x == "s" else torch.float64
+    a, om = torch.randn(m, n, device="cuda", dtype=dt), torch.randn(n, nl, device="cuda", dtype=dt)
+    y = torch.zeros(m, nl, device="cuda", dtype=dt)
+    prm, lda = lib.create_param(m, n, nl, 0, 1), n if order == b"R" else m
+
+    def run():
+        if given:
+            lib.sketch_omega(x, prm, a, lda, om, nl, y, nl, ordera=order)
+        else:
+            lib.sketch(x, prm, a, lda, y, nl, 3, ordera=order)
+        code = lib.last_error()[0]
+        lib.clear_error()
+        return code
+
+    inject(tag)
+    assert run() == TIMEOUT
+    monkeypatch.delenv("ISVD_GPU_INJECT_TIMEOUT")
+    assert run() == 0

@@ -606,6 +606,7 @@ void run_own_sketches(Plan<T> &P, cudaStream_t st) {
     g.A = P.a[b]; g.a_rs = P.lda[b]; g.a_cs = 1;
     g.B = M.om.p; g.b_rs = P.Nl[b]; g.b_cs = 1;
     g.C = M.y.p; g.c_rs = P.Nl[b]; g.c_cs = 1;
+    g.status = P.status.p;
     gemm(g, st);
   }
 }
@@ -620,6 +621,7 @@ void run_gfull(Plan<T> &P, cudaStream_t st, bool measure) {
     g.B = M.qs.p; g.b_rs = P.Nl[b]; g.b_cs = 1;
     g.C = M.G.p; g.c_rs = P.Nl[b]; g.c_cs = 1;
     g.upper = true;
+    g.status = P.status.p;
     gemm(g, st);
   }
   P.gfull.run(st, measure);
@@ -840,6 +842,7 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
     int hstatus = 0;
     CK(cudaMemcpyAsync(&hstatus, P.status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (hstatus == kErrTimeout) fail(kErrTimeout, "batched iSVD: a device-side wait timed out");
     if (hstatus) fail(kErrNumerical, "batched iSVD: small dense solver reported status %d", hstatus);
   };
   launch(1, active);
@@ -875,10 +878,7 @@ void batch_solve(BatchPlan *plan, const T *const *a, const long long *lda, T *co
     mt.prepare(st);
     mt.launch(st);
     graphed(P.post, P.post_k, capture, st, [&] { run_post(P, st, !capture); });
-    int hstatus = 0;
-    CK(cudaMemcpyAsync(&hstatus, P.status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (hstatus) fail(kErrNumerical, "batched iSVD: small dense solver reported status %d", hstatus);
+    check_status();
   }
   for (int b = 0; b < B; ++b) {
     if (iters) iters[b] = it_of[b];

@@ -147,7 +147,7 @@ bool gemm_f32_planes(const Gemm<float, Tout> &g, bool a_kc, bool b_nc, cudaStrea
   u.C = g.C; u.c_double = sizeof(Tout) == 8; u.c_rs = g.c_rs; u.c_cs = g.c_cs;
   u.alpha = g.alpha;
   u.upper = g.upper;
-  u.status = engine_status();
+  u.status = g.status ? g.status : engine_status();
   u.tag = "fp32";
   u.chunk_k = f32_chunk();
   six_products(u);

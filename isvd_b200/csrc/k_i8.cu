@@ -676,7 +676,7 @@ bool gemm_f64_int8(const Gemm<double, double> &g, bool a_kc, bool b_nc, cudaStre
       CK(cudaMemsetAsync(sum.p, 0, tiles * sizeof(unsigned long long), st));
       p.sum = sum.p;
       p.need = (unsigned long long)std::ceil(0.2 * std::sqrt((double)g.K) * 16384.0);
-      p.status = reinterpret_cast<int *>(Runtime::get().ctl + 16);  // the stages' status word
+      p.status = g.status ? g.status : reinterpret_cast<int *>(Runtime::get().ctl + 16);  // the stages' status word
       i8_gemm_kernel<<<grid, kI8Threads, kI8Smem, st>>>(digit_map(d), mb, p);
       KLAUNCHED();
       inject_timeout("int8", p.status, st);

@@ -26,6 +26,7 @@ struct Gemm {
   long long c_rs = 0, c_cs = 0, c_bs = 0;
   int batch = 1;
   int splits = 0;  // 0: choose automatically
+  int *status = nullptr;  // status word of the tensor-core paths that wait (null: the stages' word)
   // C symmetric (M == N, A = B'): tiles entirely below the diagonal are not computed; the caller
   // completes C with mirror_upper
   bool upper = false;

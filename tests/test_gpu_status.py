@@ -39,3 +39,20 @@ def test_sketch(lib, inject, monkeypatch, x, given, tag, order):
     assert run() == TIMEOUT
     monkeypatch.delenv("ISVD_GPU_INJECT_TIMEOUT")
     assert run() == 0
+
+
+@pytest.mark.parametrize("x,tag", [("s", "fp32"), ("d", "int8")])
+def test_batch(lib, inject, monkeypatch, x, tag):
+    """The products of a matrix of its own (its sketch, Qs'Qs)."""
+    from test_gpu_batched import run_batch
+    dt = torch.float32 if x == "s" else torch.float64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    mats = [dict(m=m, n=n, k=k, p=k // 2, a=torch.randn(m, n, device="cuda", generator=g, dtype=dt))
+            for m, n, k in ((300, 200, 4), (9000, 2001, 32))]
+    inject(tag)
+    with pytest.raises(AssertionError):
+        run_batch(lib, x, mats, 8, [1, 2])
+    assert lib.last_error()[0] == TIMEOUT
+    lib.clear_error()
+    monkeypatch.delenv("ISVD_GPU_INJECT_TIMEOUT")
+    run_batch(lib, x, mats, 8, [1, 2])

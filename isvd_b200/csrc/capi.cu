@@ -849,7 +849,7 @@ int adjoint_api(isvd_int_t m, isvd_int_t n, isvd_int_t k, char ordera, const T *
     its = svd_adjoint_dev<T>(c.sc, m, n, k, ordera_, A.d, lda, U.d, ldut, S.d, V.d, ldvt, dut ? dU.d : nullptr, lddut,
                              ds ? dS.d : nullptr, dvt ? dV.d : nullptr, lddvt, dA.d, ldda, cg_iters, tol);
     dA.back(sst);
-    sync();
+    read_status(c.sc, "SVD adjoint");
   });
   if (iterations) *iterations = its;
   return st;

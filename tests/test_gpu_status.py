@@ -56,3 +56,27 @@ def test_batch(lib, inject, monkeypatch, x, tag):
     lib.clear_error()
     monkeypatch.delenv("ISVD_GPU_INJECT_TIMEOUT")
     run_batch(lib, x, mats, 8, [1, 2])
+
+
+@pytest.mark.parametrize("mixed,tag", [(1, "adjoint_a"), (1, "adjoint_gram_op"), (0, "adjoint_a2"), (0, "adjoint_a"),
+                                       (0, "fp32")])
+def test_adjoint(lib, inject, monkeypatch, mixed, tag):
+    from test_gpu_adjoint_sizes import _adjoint
+    x, dt = "s", torch.float32
+    m, n, k = 9519, 3072, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rn = lambda *sh: torch.randn(*sh, device="cuda", dtype=dt, generator=g)  # noqa: E731
+    u, v = torch.linalg.qr(rn(m, k))[0].contiguous(), torch.linalg.qr(rn(n, k))[0].contiguous()
+    s = torch.linspace(2.0, 1.0, k, device="cuda", dtype=dt)
+    args = ((u * s) @ v.t()).contiguous(), s, u, v, rn(k), rn(m, k), rn(n, k), 20, 1e-6
+    lib.lib.isvd_gpu_set_precision(mixed)
+    try:
+        inject(tag)
+        with pytest.raises(AssertionError):
+            _adjoint(lib, x, *args)
+        assert lib.last_error()[0] == TIMEOUT
+        lib.clear_error()
+        monkeypatch.delenv("ISVD_GPU_INJECT_TIMEOUT")
+        _adjoint(lib, x, *args)
+    finally:
+        lib.lib.isvd_gpu_set_precision(0)

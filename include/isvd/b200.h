@@ -31,6 +31,10 @@ int  isvd_gpu_get_last_error( void );
 const char *isvd_gpu_get_error_string( void );
 void isvd_gpu_clear_error( void );
 
+/* Diagnostic (0: off): device allocations that would take what the library holds above this many bytes fail as
+ * if the device were full, so that a program can test how it runs short of memory. */
+extern size_t isvd_gpu_alloc_limit;
+
 /* ---------------------------------------------------------------- precision */
 #define ISVD_GPU_PRECISION_NATIVE   0  /* products in the routine's own type (FP64 for isvd_d*, FP32 for isvd_s*); large
                                           FP32 products on tcgen05 from operands split exactly into three bf16

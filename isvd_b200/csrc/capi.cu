@@ -861,6 +861,7 @@ int adjoint_api(isvd_int_t m, isvd_int_t n, isvd_int_t k, char ordera, const T *
 extern "C" {
 
 size_t isvd_gpu_memory_limit = 0;
+size_t isvd_gpu_alloc_limit = 0;
 
 int isvd_gpu_get_last_error(void) { return t_last_error; }
 const char *isvd_gpu_get_error_string(void) { return t_last_msg.c_str(); }

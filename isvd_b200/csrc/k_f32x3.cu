@@ -354,9 +354,16 @@ void f32_sketch_rows(const Planes &omega_t, long long rows, int n, int Nl, char 
     }
     if (!fits) keep = nullptr;
   }
-  const long long P = f32_sketch_panel(rows, n), rp = plane_rows(keep ? rows : P), ps = rp * pld;
+  long long P = f32_sketch_panel(rows, n), rp = plane_rows(keep ? rows : P), ps = rp * pld;
   PlaneBuf pa;
-  if (!keep) pa.buf.alloc((size_t)3 * ps);
+  while (!keep && !pa.buf.p) try {
+    pa.buf.alloc((size_t)3 * ps);
+  } catch (const Error &e) {
+    if (e.code != kErrMemory || P <= 256) throw;
+    P = std::max<long long>(256, P / 2 / 256 * 256);  // smaller panels
+    rp = plane_rows(P);
+    ps = rp * pld;
+  }
   __nv_bfloat16 *base = keep ? keep->buf.p : pa.buf.p;
   auto split = [&](long long r0, long long cnt, __nv_bfloat16 *dst) {
     if (ordera == 'R') split_rows<float>(a + r0 * ld, ld, 1, cnt, n, 3, false, dst, pld, ps, st);

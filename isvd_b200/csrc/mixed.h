@@ -74,7 +74,8 @@ void sketch_tile_order(UmmaGemm &g, long long n, long long Nl, int bn);
 
 // NATIVE FP32 on the bf16 tensor cores (k_f32x3.cu): operands in three planes, exact to FP32.
 // The sketch: A's planes against the one exact plane of an Omega drawn here (offset: the value offset of
-// its first row).  keep: the planes of all rows stay there for f32_project when memory allows.
+// its first row).  keep: the planes of all rows stay there for f32_project when memory allows.  Throws kErrMemory
+// when not even the planes of 256 rows fit.
 bool f32_sketch_pays(long long m, long long n, long long Nl, long long offset);
 void f32_sketch_rows(const Planes &omega_t, long long rows, int n, int Nl, char ordera, const float *a, long long ld,
                      float *y, long long ldy, MixedCache *keep, cudaStream_t st);

@@ -14,6 +14,7 @@
 #include <vector>
 
 extern "C" size_t isvd_gpu_memory_limit;  // include/isvd/gpu/env.h
+extern "C" size_t isvd_gpu_alloc_limit;   // include/isvd/b200.h
 
 namespace isvdb {
 
@@ -99,7 +100,16 @@ void set_default_precision(int p) { g_precision = p; }
 void *dev_alloc(size_t bytes) {
   Runtime &rt = Runtime::get();
   void *p = nullptr;
-  cudaError_t e = cudaMallocAsync(&p, bytes, rt.stream);
+  cudaError_t e = cudaSuccess;
+  if (isvd_gpu_alloc_limit > 0) {  // diagnostic: as if the device had no more
+    cudaMemPool_t pool;
+    unsigned long long used = 0;
+    CK(cudaStreamSynchronize(rt.stream));
+    CK(cudaDeviceGetDefaultMemPool(&pool, rt.device));
+    CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    if (used + bytes > isvd_gpu_alloc_limit) e = cudaErrorMemoryAllocation;
+  }
+  if (e == cudaSuccess) e = cudaMallocAsync(&p, bytes, rt.stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
     fail(kErrMemory, "device allocation of %zu bytes failed (%s)", bytes, cudaGetErrorString(e));

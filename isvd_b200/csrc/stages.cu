@@ -54,28 +54,39 @@ void sketch_dev(const StageCtx &c, int m, int n, int Nl, char ordera, const T *a
   }
   DBuf<T> om;
   PlaneBuf om_t;  // FP32: Omega' as one exact bf16 plane, for the tensor-core sketch
+  auto no_planes = [&] {
+    om_t.buf.release();
+    om_t.P = Planes();
+  };
   if constexpr (std::is_same<T, float>::value) {
     const long long off = c.col_begin * (long long)Nl;
-    if (!omega && f32_sketch_pays(m, n, Nl, off)) {
-      const long long old = plane_ld(n), orp = plane_rows(Nl);
-      om_t.buf.alloc((size_t)orp * old);
-      rng_gaussian_bf16_t(om_t.buf.p, n, Nl, old, orp, seed, c.st, off);
-      Planes &P = om_t.P;
-      P.ptr = om_t.buf.p; P.np = 1; P.rows = Nl; P.cols = n; P.ld = old; P.plane_stride = orp * old;
-    }
-  }
-  if (!omega && !om_t.P.ptr) {
-    om.alloc((size_t)n * Nl);
-    rng_gaussian<T>(om.p, n, Nl, Nl, seed, (uint64_t)c.col_begin * Nl, c.st);  // column blocks: own rows
-    omega = om.p;
-    ldom = Nl;
+    if (!omega && f32_sketch_pays(m, n, Nl, off)) try {
+        const long long old = plane_ld(n), orp = plane_rows(Nl);
+        om_t.buf.alloc((size_t)orp * old);
+        rng_gaussian_bf16_t(om_t.buf.p, n, Nl, old, orp, seed, c.st, off);
+        Planes &P = om_t.P;
+        P.ptr = om_t.buf.p; P.np = 1; P.rows = Nl; P.cols = n; P.ld = old; P.plane_stride = orp * old;
+      } catch (const Error &e) {
+        if (e.code != kErrMemory) throw;
+        no_planes();
+      }
   }
   auto rows_times_omega = [&](long long r0, long long rows, const T *ap, long long ld) {
     if constexpr (std::is_same<T, float>::value) {
-      if (om_t.P.ptr) {
-        f32_sketch_rows(om_t.P, rows, n, Nl, ordera, ap, ld, y + r0 * ldy, ldy, ap == a ? c.cache : nullptr, c.st);
-        return;
-      }
+      if (om_t.P.ptr) try {
+          f32_sketch_rows(om_t.P, rows, n, Nl, ordera, ap, ld, y + r0 * ldy, ldy, ap == a ? c.cache : nullptr, c.st);
+          return;
+        } catch (const Error &e) {  // no room for planes: the CUDA-core product of these rows and the next
+          if (e.code != kErrMemory) throw;
+          no_planes();
+          if (c.cache) c.cache->buf.release();
+        }
+    }
+    if (!omega) {
+      om.alloc((size_t)n * Nl);
+      rng_gaussian<T>(om.p, n, Nl, Nl, seed, (uint64_t)c.col_begin * Nl, c.st);  // column blocks: own rows
+      omega = om.p;
+      ldom = Nl;
     }
     Gemm<T, T> g = gm<T>((int)rows, Nl, n);
     g.A = ap; set_a(g, ordera, ld, false);

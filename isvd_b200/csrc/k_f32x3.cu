@@ -233,12 +233,11 @@ template bool gemm_f32_planes<float>(const Gemm<float, float> &, bool, bool, cud
 template bool gemm_f32_planes<double>(const Gemm<float, double> &, bool, bool, cudaStream_t);
 
 // ------------------------------------------------------------------------- stages (mixed.h)
-bool f32_block_planes(PlaneBuf &pb, const float *y, long long ldy, long long rows, int l, int N, cudaStream_t st) {
-  if (planes_off() || Runtime::get().cc_major != 10) return false;
-  // the Grams and the applies from one split
-  if (!plane_product_pays((double)rows, l, l, N, 0.5 * rows * l * N, 0.0)) return false;
+// Runs f; false when it ran out of memory.
+template <class F>
+static bool fits_memory(F f) {
   try {
-    block_planes(pb, y, ldy, rows, N, l, l, (l + 7) & ~7, st);
+    f();
   } catch (const Error &e) {
     if (e.code != kErrMemory) throw;
     return false;
@@ -246,7 +245,14 @@ bool f32_block_planes(PlaneBuf &pb, const float *y, long long ldy, long long row
   return true;
 }
 
-void f32_block_gram(const PlaneBuf &yp, int rows, int l, int N, double *W, cudaStream_t st) {
+bool f32_block_planes(PlaneBuf &pb, const float *y, long long ldy, long long rows, int l, int N, cudaStream_t st) {
+  if (planes_off() || Runtime::get().cc_major != 10) return false;
+  // the Grams and the applies from one split
+  if (!plane_product_pays((double)rows, l, l, N, 0.5 * rows * l * N, 0.0)) return false;
+  return fits_memory([&] { block_planes(pb, y, ldy, rows, N, l, l, (l + 7) & ~7, st); });
+}
+
+bool f32_block_gram(const PlaneBuf &yp, int rows, int l, int N, double *W, cudaStream_t st) {
   UmmaGemm u;
   u.M = l; u.N = l; u.K = rows;
   u.A = u.B = yp.P;
@@ -257,15 +263,15 @@ void f32_block_gram(const PlaneBuf &yp, int rows, int l, int N, double *W, cudaS
   u.tag = "block_gram";
   u.chunk_k = f32_chunk();
   six_products(u);
-  umma_gemm(u, st);
+  return fits_memory([&] { umma_gemm(u, st); });
 }
 
-void f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp, float *out, long long ldo,
+bool f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp, float *out, long long ldo,
                      cudaStream_t st) {
   // K runs to the next multiple of 64, over columns of the next block that meet zeros of Wp's planes
   const int kp = (l + 63) / 64 * 64;
   PlaneBuf wt;
-  block_planes_t(wt, Wp, l, l, l, N, (long long)l * l, kp, st);
+  if (!fits_memory([&] { block_planes_t(wt, Wp, l, l, l, N, (long long)l * l, kp, st); })) return false;
   UmmaGemm u;
   u.M = rows; u.N = l; u.K = kp;
   u.A = yp.P; u.B = wt.P;
@@ -275,7 +281,7 @@ void f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp
   u.tag = "block_apply";
   u.chunk_k = f32_chunk();
   six_products(u);
-  umma_gemm(u, st);
+  return fits_memory([&] { umma_gemm(u, st); });
 }
 
 bool f32_operator_pays(long long m, long long n, int k) {
@@ -288,16 +294,10 @@ bool f32_operator_pays(long long m, long long n, int k) {
 bool f32_tall_planes(PlaneBuf &pb, const float *qs, long long ldq, long long rows, int Nl, cudaStream_t st) {
   if (planes_off() || Runtime::get().cc_major != 10) return false;
   if (!plane_product_pays(Nl, Nl, (double)rows, 1, (double)rows * Nl, 0.0)) return false;
-  try {
-    make_planes<float>(pb, qs, ldq, rows, Nl, 3, false, st);
-  } catch (const Error &e) {
-    if (e.code != kErrMemory) throw;
-    return false;
-  }
-  return true;
+  return fits_memory([&] { make_planes<float>(pb, qs, ldq, rows, Nl, 3, false, st); });
 }
 
-void f32_tall_gram(const PlaneBuf &qp, int rows, int Nl, double *G, cudaStream_t st) {
+bool f32_tall_gram(const PlaneBuf &qp, int rows, int Nl, double *G, cudaStream_t st) {
   UmmaGemm u;
   u.M = Nl; u.N = Nl; u.K = rows;
   u.A = u.B = qp.P;
@@ -308,14 +308,15 @@ void f32_tall_gram(const PlaneBuf &qp, int rows, int Nl, double *G, cudaStream_t
   u.tag = "gram_full";
   u.chunk_k = f32_chunk();
   six_products(u);
-  umma_gemm(u, st);
+  if (!fits_memory([&] { umma_gemm(u, st); })) return false;
   mirror_upper(G, Nl, Nl, st);
+  return true;
 }
 
-void f32_tall_apply(const PlaneBuf &qp, int rows, int Nl, int l, const float *M, long long ldm, float *out, long long ldo,
+bool f32_tall_apply(const PlaneBuf &qp, int rows, int Nl, int l, const float *M, long long ldm, float *out, long long ldo,
                     cudaStream_t st) {
   PlaneBuf mt;
-  make_planes<float>(mt, M, ldm, Nl, l, 3, true, st);  // M' planes (l x Nl)
+  if (!fits_memory([&] { make_planes<float>(mt, M, ldm, Nl, l, 3, true, st); })) return false;  // M' planes (l x Nl)
   UmmaGemm u;
   u.M = rows; u.N = l; u.K = Nl;
   u.A = qp.P; u.B = mt.P;
@@ -324,7 +325,7 @@ void f32_tall_apply(const PlaneBuf &qp, int rows, int Nl, int l, const float *M,
   u.tag = "coeff_apply";
   u.chunk_k = f32_chunk();
   six_products(u);
-  umma_gemm(u, st);
+  return fits_memory([&] { umma_gemm(u, st); });
 }
 
 // Rows of A per panel of the plane sketch: about plane_cap() of planes.

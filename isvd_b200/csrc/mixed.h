@@ -88,15 +88,16 @@ int f32_chunk();
 bool f32_operator_pays(long long m, long long n, int k);
 // Planes of the N column blocks (l columns, each block padded to a multiple of 8) of a tall matrix, and
 // W_i = Y_i' Y_i and out_i = Y_i Wp_i from them (out may be the matrix itself).  f32_block_planes: false
-// when the products are too small for planes or there is no memory for them.
+// when the products are too small for planes or there is no memory for them.  The products return false, with
+// nothing of their result to be used, when there is no memory for them.
 bool f32_block_planes(PlaneBuf &pb, const float *y, long long ldy, long long rows, int l, int N, cudaStream_t st);
-void f32_block_gram(const PlaneBuf &yp, int rows, int l, int N, double *W, cudaStream_t st);
-void f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp, float *out, long long ldo,
+bool f32_block_gram(const PlaneBuf &yp, int rows, int l, int N, double *W, cudaStream_t st);
+bool f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp, float *out, long long ldo,
                      cudaStream_t st);
 // Planes of a tall rows x Nl matrix, G = Qs'Qs (whole) and out = Qs M from them.
 bool f32_tall_planes(PlaneBuf &pb, const float *qs, long long ldq, long long rows, int Nl, cudaStream_t st);
-void f32_tall_gram(const PlaneBuf &qp, int rows, int Nl, double *G, cudaStream_t st);
-void f32_tall_apply(const PlaneBuf &qp, int rows, int Nl, int l, const float *M, long long ldm, float *out, long long ldo,
+bool f32_tall_gram(const PlaneBuf &qp, int rows, int Nl, double *G, cudaStream_t st);
+bool f32_tall_apply(const PlaneBuf &qp, int rows, int Nl, int l, const float *M, long long ldm, float *out, long long ldo,
                     cudaStream_t st);
 
 // The next four take bf16 planes `yp` of an m x Nl row-major matrix (split without transpose,

@@ -120,10 +120,12 @@ void gramian_pass(const StageCtx &c, int m, int l, int N, T *y, long long ldy, b
   else if (c.precision == kMixed) make_planes<T>(yp, y, ldy, m, Nl, 3, false, c.st);
   bool fp = false;  // FP32: yp holds the planes of Y's blocks
   if constexpr (std::is_same<T, float>::value)
-    if (c.precision != kMixed) fp = f32_block_planes(yp, y, ldy, m, l, N, c.st);
+    if (c.precision != kMixed) {
+      fp = f32_block_planes(yp, y, ldy, m, l, N, c.st) && f32_block_gram(yp, m, l, N, W.p, c.st);
+      if (!fp) yp.buf.release();
+    }
   // W_i = Y_i' Y_i   (reference :82-84)
   if (fp) {
-    f32_block_gram(yp, m, l, N, W.p, c.st);
   } else if (c.precision == kMixed) {
     mixed_block_gram<T>(c, yp.P, m, l, N, y, ldy, W.p);
   } else {
@@ -179,10 +181,8 @@ void gramian_pass(const StageCtx &c, int m, int l, int N, T *y, long long ldy, b
     return;
   }
   if constexpr (std::is_same<T, float>::value)
-    if (fp) {
-      f32_block_apply(yp, m, l, N, Wp.p, y, ldy, c.st);
-      return;
-    }
+    if (fp && f32_block_apply(yp, m, l, N, Wp.p, y, ldy, c.st)) return;
+  if (c.precision != kMixed) yp.buf.release();  // no room beside them
   if (from_hand) fail(kErrUnsupported, "plane hand-off into the Gramian orthogonalization needs l %% 64 == 0");
   Gemm<T, T> g = gm<T>(m, l, l);
   g.batch = N;
@@ -284,7 +284,10 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
   else if (c.precision == kMixed) make_planes<T>(qp, qs, ldq, m, Nl, 3, false, c.st);
   bool fp = false;  // FP32: qp holds the planes of Qs
   if constexpr (std::is_same<T, float>::value)
-    if (c.precision != kMixed && (fp = f32_tall_planes(qp, qs, ldq, m, Nl, c.st))) f32_tall_gram(qp, m, Nl, G.p, c.st);
+    if (c.precision != kMixed) {
+      fp = f32_tall_planes(qp, qs, ldq, m, Nl, c.st) && f32_tall_gram(qp, m, Nl, G.p, c.st);
+      if (!fp) qp.buf.release();
+    }
   if (fp) {
   } else if (c.precision == kMixed) {
     mixed_gram_full<T>(c, qp.P, m, Nl, qs, ldq, G.p);
@@ -427,10 +430,8 @@ IterResult integrate_kn_dev(const StageCtx &c, int m, int l, int N, const T *qs,
     DBuf<T> Mt(nl);
     copy2d<double, T>(Wp, lw, 1, Mt.p, l, 1, Nl, l, c.st);
     if constexpr (std::is_same<T, float>::value)
-      if (fp) {
-        f32_tall_apply(qp, m, Nl, l, Mt.p, l, qt, ldqt, c.st);
-        return res;
-      }
+      if (fp && f32_tall_apply(qp, m, Nl, l, Mt.p, l, qt, ldqt, c.st)) return res;
+    qp.buf.release();
     Gemm<T, T> g = gm<T>(m, l, Nl);
     g.A = qs; g.a_rs = ldq; g.a_cs = 1;
     g.B = Mt.p; g.b_rs = l; g.b_cs = 1;

@@ -112,8 +112,10 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
     PlaneBuf yp;
     bool fp = false;  // FP32: yp holds the planes of the blocks, the product may overwrite them
     if constexpr (std::is_same<T, float>::value)
-      if (!mixed && (fp = f32_block_planes(yp, src, lds, rows, l, N, c.st)))
-        f32_block_gram(yp, (int)rows, l, N, W.p, c.st);
+      if (!mixed) {
+        fp = f32_block_planes(yp, src, lds, rows, l, N, c.st) && f32_block_gram(yp, (int)rows, l, N, W.p, c.st);
+        if (!fp) yp.buf.release();
+      }
     if (fp) {
     } else if (mixed) {
       make_planes<T>(yp, src, lds, rows, Nl, 3, false, c.st);
@@ -152,10 +154,8 @@ void cholqr3_blocks(const StageCtx &c, long long rows, int l, int N, T *y, long 
     }
     copy2d<double, T>(X.p, l, 1, Xt.p, l, 1, (long long)N * l, l, c.st);
     if constexpr (std::is_same<T, float>::value)
-      if (fp) {
-        f32_block_apply(yp, (int)rows, l, N, Xt.p, src, lds, c.st);
-        continue;
-      }
+      if (fp && f32_block_apply(yp, (int)rows, l, N, Xt.p, src, lds, c.st)) continue;
+    if (!mixed) yp.buf.release();  // no room beside them
     Gemm<T, T> g;
     g.M = (int)rows; g.N = l; g.K = l; g.batch = N;
     g.A = src; g.a_rs = lds; g.a_cs = 1; g.a_bs = l;
@@ -217,7 +217,10 @@ IterResult integrate_wy_dev(const StageCtx &c, int m, int l, int N, const T *qs,
   PlaneBuf qp;  // MIXED: bf16 planes of Qs, shared by G and the final Qbar = Qs M
   bool fp = false;  // FP32: qp holds the planes of Qs
   if constexpr (std::is_same<T, float>::value)
-    if (!mixed && (fp = f32_tall_planes(qp, qs, ldq, m, Nl, st))) f32_tall_gram(qp, m, Nl, G.p, st);
+    if (!mixed) {
+      fp = f32_tall_planes(qp, qs, ldq, m, Nl, st) && f32_tall_gram(qp, m, Nl, G.p, st);
+      if (!fp) qp.buf.release();
+    }
   if (fp) {
   } else if (mixed) {
     if (c.handoff && c.handoff->holds(qs, ldq)) qp.P = c.handoff->pb.P;  // the Gramian apply's planes
@@ -369,10 +372,8 @@ IterResult integrate_wy_dev(const StageCtx &c, int m, int l, int N, const T *qs,
     DBuf<T> Mt(nl);
     copy2d<double, T>(Mp, l, 1, Mt.p, l, 1, Nl, l, st);
     if constexpr (std::is_same<T, float>::value)
-      if (fp) {
-        f32_tall_apply(qp, m, Nl, l, Mt.p, l, qt, ldqt, st);
-        return res;
-      }
+      if (fp && f32_tall_apply(qp, m, Nl, l, Mt.p, l, qt, ldqt, st)) return res;
+    qp.buf.release();
     Gemm<T, T> g;
     g.M = m; g.N = l; g.K = Nl;
     g.A = qs; g.a_rs = ldq; g.a_cs = 1;

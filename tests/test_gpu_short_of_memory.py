@@ -41,3 +41,43 @@ def test_sketch(lib, room, order, megabytes):
     assert lib.last_error()[0] == 0, lib.last_error()
     # a chain of n FP32 multiply-adds rounds like a random walk: under u sqrt(n) / 2, twice that for the margin
     assert _rel(y, ref) <= U * n ** 0.5
+
+
+def _blocks(m, l, N):
+    g = torch.Generator(device="cuda").manual_seed(l)
+    return torch.randn(m, N * l, device="cuda", generator=g)
+
+
+@pytest.mark.parametrize("alg", ["GR", "TS"])
+@pytest.mark.parametrize("megabytes", [85, 119, 121, 300])
+def test_orthogonalization(lib, room, alg, megabytes):
+    """The blocks' planes are 118 MB; the temporary of the CUDA-core product is 78 MB."""
+    m, l, N = 40000, 64, 8
+    y = _blocks(m, l, N)
+    q = y.clone()
+    room(megabytes)
+    lib.orthogonalize("s", alg, lib.create_param(m, m, l, 0, N), q, N * l)
+    assert lib.last_error()[0] == 0, lib.last_error()
+    for i in (0, N - 1):
+        qi, yi = (t[:, i * l:(i + 1) * l].double() for t in (q, y))
+        # as test_gpu_fp32_planes.py, with the CUDA cores' chains of m / 16 terms: u sqrt(2500) / 2 = 25 u, times four
+        assert float((qi.t() @ qi - torch.eye(l, device="cuda")).abs().max()) <= 100 * U
+        assert float((yi - qi @ (qi.t() @ yi)).norm() / yi.norm()) <= 100 * U
+
+
+@pytest.mark.parametrize("alg", ["KN", "WY"])
+@pytest.mark.parametrize("megabytes", [60, 119, 123, 300])
+def test_integration(lib, room, alg, megabytes):
+    m, l, N = 40000, 64, 8
+    g = torch.Generator(device="cuda").manual_seed(2)
+    base = torch.randn(m, l, device="cuda", generator=g)
+    y = _blocks(m, l, N)
+    qs = torch.cat([torch.linalg.qr(base + 0.2 * y[:, i * l:(i + 1) * l])[0] for i in range(N)], 1).contiguous()
+    prm = lib.create_param(m, m, l, 0, N)
+    qt, ref = torch.zeros(m, l, device="cuda"), torch.zeros(m, l, device="cuda")
+    lib.integrate("s", alg, prm, qs, N * l, ref, l, argv=[3, 1e-9])
+    assert lib.last_error()[0] == 0
+    room(megabytes)
+    lib.integrate("s", alg, prm, qs, N * l, qt, l, argv=[3, 1e-9])
+    assert lib.last_error()[0] == 0, lib.last_error()
+    assert _rel(qt, ref) <= 200 * U

@@ -401,15 +401,20 @@ void f32_sketch_rows(const Planes &omega_t, long long rows, int n, int Nl, char 
   if (keep) {
     keep->src = a; keep->m = rows; keep->n = n; keep->ordera = ordera;
     keep->A = all;
+    keep->spare(true);
   }
 }
 
-bool f32_project(const MixedCache *mc, int m, int n, int l, char ordera, const float *a, const float *qt, long long ldqt,
+bool f32_project(MixedCache *mc, int m, int n, int l, char ordera, const float *a, const float *qt, long long ldqt,
                  float *z, cudaStream_t st) {
   if (!mc || mc->src != a || mc->m != m || mc->n != n || mc->ordera != ordera || !mc->buf.p || mc->A.np != 3)
     return false;
+  mc->spare(false);  // read below
   PlaneBuf qp;
-  make_planes<float>(qp, qt, ldqt, m, l, 3, true, st);  // Qbar' planes (l x m)
+  if (!fits_memory([&] { make_planes<float>(qp, qt, ldqt, m, l, 3, true, st); })) {  // Qbar' planes (l x m)
+    mc->drop();
+    return false;
+  }
   UmmaGemm u;
   u.M = l; u.N = n; u.K = m;
   u.A = qp.P;
@@ -420,8 +425,9 @@ bool f32_project(const MixedCache *mc, int m, int n, int l, char ordera, const f
   u.tag = "project";
   u.chunk_k = f32_chunk();
   six_products(u);
-  umma_gemm(u, st);
-  return true;
+  if (fits_memory([&] { umma_gemm(u, st); })) return true;
+  mc->drop();
+  return false;
 }
 
 }  // namespace isvdb

@@ -48,8 +48,27 @@ struct MixedGProduct {
              bool split = true);
 };
 
-// A's bf16 planes (m x n, K-major along n), made by the sketch and reused by the postprocess.
-struct MixedCache {
+// A's bf16 planes (m x n, K-major along n), made by the sketch and reused by the postprocess.  spare(true): until
+// then they may be given back when the device is full (NATIVE, whose projection does without them).
+struct MixedCache : Spare {
+  MixedCache() = default;
+  MixedCache(const MixedCache &) = delete;
+  MixedCache &operator=(const MixedCache &) = delete;
+  ~MixedCache() override { spare(false); }
+  void spare(bool on) {
+    if (on) g_spare = this;
+    else if (g_spare == this) g_spare = nullptr;
+  }
+  void drop() {
+    spare(false);
+    buf.release();
+    src = nullptr;
+  }
+  bool give_back() override {
+    const bool any = buf.p != nullptr;
+    drop();
+    return any;
+  }
   const void *src = nullptr;
   long long m = 0, n = 0;
   char ordera = 0;
@@ -79,8 +98,8 @@ void sketch_tile_order(UmmaGemm &g, long long n, long long Nl, int bn);
 bool f32_sketch_pays(long long m, long long n, long long Nl, long long offset);
 void f32_sketch_rows(const Planes &omega_t, long long rows, int n, int Nl, char ordera, const float *a, long long ld,
                      float *y, long long ldy, MixedCache *keep, cudaStream_t st);
-// Z = A' Qbar from the sketch's planes of A; false when mc does not hold them.
-bool f32_project(const MixedCache *mc, int m, int n, int l, char ordera, const float *a, const float *qt, long long ldqt,
+// Z = A' Qbar from the sketch's planes of A; false when mc does not hold them or there is no memory beside them.
+bool f32_project(MixedCache *mc, int m, int n, int l, char ordera, const float *a, const float *qt, long long ldqt,
                  float *z, cudaStream_t st);
 // Accumulation chunk of FP32-exact plane products; whether repeated products of an m x n A with
 // k columns are faster from A's three planes.

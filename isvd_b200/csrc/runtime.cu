@@ -97,23 +97,35 @@ int default_precision() {
 
 void set_default_precision(int p) { g_precision = p; }
 
-void *dev_alloc(size_t bytes) {
+Spare *g_spare = nullptr;
+
+static cudaError_t try_alloc(void **p, size_t bytes) {
   Runtime &rt = Runtime::get();
-  void *p = nullptr;
-  cudaError_t e = cudaSuccess;
   if (isvd_gpu_alloc_limit > 0) {  // diagnostic: as if the device had no more
     cudaMemPool_t pool;
     unsigned long long used = 0;
     CK(cudaStreamSynchronize(rt.stream));
     CK(cudaDeviceGetDefaultMemPool(&pool, rt.device));
     CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
-    if (used + bytes > isvd_gpu_alloc_limit) e = cudaErrorMemoryAllocation;
+    if (used + bytes > isvd_gpu_alloc_limit) return cudaErrorMemoryAllocation;
   }
-  if (e == cudaSuccess) e = cudaMallocAsync(&p, bytes, rt.stream);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
+  const cudaError_t e = cudaMallocAsync(p, bytes, rt.stream);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
+void *dev_alloc(size_t bytes) {
+  void *p = nullptr;
+  cudaError_t e = try_alloc(&p, bytes);
+  if (e != cudaSuccess && g_spare && g_spare->give_back()) {
+    cudaMemPool_t pool;  // the freed block as device memory for any size
+    CK(cudaStreamSynchronize(Runtime::get().stream));
+    CK(cudaDeviceGetDefaultMemPool(&pool, Runtime::get().device));
+    CK(cudaMemPoolTrimTo(pool, 0));
+    e = try_alloc(&p, bytes);
+  }
+  if (e != cudaSuccess)
     fail(kErrMemory, "device allocation of %zu bytes failed (%s)", bytes, cudaGetErrorString(e));
-  }
   return p;
 }
 

@@ -92,6 +92,13 @@ struct DBuf {
   operator T *() const { return p; }
 };
 
+// A buffer that its owner can do without: dev_alloc has it given back before it fails (under the API lock).
+struct Spare {
+  virtual ~Spare() = default;
+  virtual bool give_back() = 0;  // false: nothing to give
+};
+extern Spare *g_spare;  // at most one, null when there is none
+
 void *dev_alloc(size_t bytes);
 void dev_free(void *p);
 

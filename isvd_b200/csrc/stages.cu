@@ -79,7 +79,7 @@ void sketch_dev(const StageCtx &c, int m, int n, int Nl, char ordera, const T *a
         } catch (const Error &e) {  // no room for planes: the CUDA-core product of these rows and the next
           if (e.code != kErrMemory) throw;
           no_planes();
-          if (c.cache) c.cache->buf.release();
+          if (c.cache) c.cache->drop();
         }
     }
     if (!omega) {

@@ -81,3 +81,29 @@ def test_integration(lib, room, alg, megabytes):
     lib.integrate("s", alg, prm, qs, N * l, qt, l, argv=[3, 1e-9])
     assert lib.last_error()[0] == 0, lib.last_error()
     assert _rel(qt, ref) <= 200 * U
+
+
+@pytest.mark.parametrize("algs", [("GP", "GR", "KN", "GR"), ("GP", "TS", "WY", "TS"), ("GP", "TS", "HR", "GR")])
+@pytest.mark.parametrize("megabytes", [260, 1015, 1030, 1100, 4000])
+def test_solve(lib, room, algs, megabytes):
+    """The planes of A that the sketch keeps for the projection are 927 MB, Y, Qbar and Omega 92 MB, the rest of the
+    solve up to 160 MB."""
+    m, n, k, p, N = 40000, 4000, 48, 16, 8
+    l = k + p
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, w = (torch.randn(q, 2 * l, device="cuda", generator=g) for q in (m, n))
+    a = (x * torch.linspace(1, 0.1, 2 * l, device="cuda")) @ w.t() + 0.01 * torch.randn(m, n, device="cuda", generator=g)
+    prm = lib.create_param(m, n, k, p, N)
+
+    def solve():
+        s, u, v = (torch.zeros(*sh, device="cuda") for sh in ((l,), (m, l), (n, l)))
+        _, _, status = lib.isvd("s", prm, algs, a, n, s, u, l, v, l, seed=3, retc=(0, 0, 0, 0), precision=0)
+        assert status == 0, lib.last_error()
+        return s, (u[:, :k].double() * s[:k]) @ v[:, :k].double().t()
+
+    s0, a0 = solve()
+    room(megabytes)
+    s1, a1 = solve()
+    # FP32 solves of the same sketch by other roundings: a few tens of u sqrt(n) at most
+    assert float((s1 - s0).abs().max()) <= 20 * U * n ** 0.5 * float(s0[0])
+    assert _rel(a1, a0) <= 100 * U * n ** 0.5

@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           // lies above it (infinity; NaN, which is 0x7fffffff here) stay as they are
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const uint32_t odd = (v[i] << 1) < 0xfefffffeu ? v[i] & 1u : 0u;
-            v[i] += BK == 64 ? odd + (odd & (v[i] >> 1)) : odd;
+            const uint32_t odd = v[i] & 1u;
+            if (fabsf(__uint_as_float(v[i])) < 3.402823466e38f) v[i] += BK == 64 ? odd + (odd & (v[i] >> 1)) : odd;
           }
         }
 #pragma unroll
@@ -945,15 +945,13 @@ void launch_split(const T *src, long long s_rs, long long s_cs, long long rows, 
 
 // Transposed: plane(c, r) = piece(src(r, c)) through a 64 (r) x 32 (c) shared tile; each thread
 // writes 8 consecutive r of one output row c (16-byte vectors).  Plane rows beyond cols and
-// columns beyond rows are zeroed separately.  The tiles run along grid.x, the gx tiles of r fastest (grid.y
-// would end at 65535 tiles of c).
+// columns beyond rows are zeroed separately.  The tiles of c run along grid.y and grid.z (grid.y ends at 65535).
 template <class T>
 __global__ void split_t_kernel(const T *__restrict__ src, long long s_rs, long long s_cs, long long rows,
                                long long cols, long long rows_pad, int np, __nv_bfloat16 *__restrict__ dst,
-                               long long ld, long long ps, unsigned gx) {
+                               long long ld, long long ps) {
   __shared__ T tile[64][33];
-  const unsigned by = blockIdx.x / gx;
-  const long long r0 = (long long)(blockIdx.x - by * gx) * 64, c0 = (long long)by * 32;
+  const long long r0 = (long long)blockIdx.x * 64, c0 = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
   for (int j = ty; j < 64; j += 8) {
     const long long r = r0 + j, c = c0 + tx;
@@ -981,10 +979,9 @@ __global__ void split_t_kernel(const T *__restrict__ src, long long s_rs, long l
 template <class T>
 void launch_split_t(const T *src, long long s_rs, long long s_cs, long long rows, long long cols, long long rows_pad,
                     int np, __nv_bfloat16 *dst, long long ld, long long ps, cudaStream_t st) {
-  const long long gx = (rows + 63) / 64, gy = (cols + 31) / 32;
-  if (gx * gy >= (1LL << 31)) fail(kErrUnsupported, "split of a transpose: too many tiles");
-  split_t_kernel<T><<<(unsigned)(gx * gy), 256, 0, st>>>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, ps,
-                                                         (unsigned)gx);
+  const long long gy = (cols + 31) / 32, gz = (gy + 65534) / 65535;  // the last z may start beyond cols and rows_pad
+  const dim3 grid((unsigned)((rows + 63) / 64), (unsigned)((gy + gz - 1) / gz), (unsigned)gz);
+  split_t_kernel<T><<<grid, 256, 0, st>>>(src, s_rs, s_cs, rows, cols, rows_pad, np, dst, ld, ps);
   KLAUNCHED();
 }
 

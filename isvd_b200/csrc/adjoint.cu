@@ -146,9 +146,9 @@ __global__ void cg_step2_kernel(T *p, const T *__restrict__ r, long long rows, i
 constexpr int kCgThreads = 512;
 constexpr int kCgBlocks = 128;
 
-// Adds the CTAs' slices in the last CTA (fin: column, sum; one thread per column).
+// Adds the CTAs' slices in the last CTA (fin: column, sum; one thread per column), kCgThreads columns at a time.
 template <class F>
-__device__ __forceinline__ void cg_dot_finish(int kc, double *partial, unsigned *ctl, F fin) {
+__device__ __forceinline__ void cg_dot_finish(double *sh, int kc, double *partial, unsigned *ctl, F fin) {
   __shared__ bool last;
   __threadfence();
   __syncthreads();
@@ -160,26 +160,30 @@ __device__ __forceinline__ void cg_dot_finish(int kc, double *partial, unsigned 
   // four columns per warp at a time, lanes over the slices: sixteen loads in flight
   constexpr int kSl = (kCgBlocks + 31) / 32;
   const int lane = threadIdx.x & 31;
-  for (int c0 = 4 * (threadIdx.x >> 5); c0 < kc; c0 += 4 * (kCgThreads / 32)) {
-    double v[4][kSl];
+  for (int base = 0; base < kc; base += kCgThreads) {
+    const int kb = min(kCgThreads, kc - base);
+    for (int c0 = 4 * (threadIdx.x >> 5); c0 < kb; c0 += 4 * (kCgThreads / 32)) {
+      double v[4][kSl];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int w = 0; w < kSl; ++w) {
-        const int b = lane + 32 * w;
-        v[u][w] = (c0 + u < kc && b < (int)gridDim.x) ? __ldcg(partial + (size_t)b * kc + c0 + u) : 0.0;
+        for (int w = 0; w < kSl; ++w) {
+          const int b = lane + 32 * w;
+          v[u][w] = (c0 + u < kb && b < (int)gridDim.x) ? __ldcg(partial + (size_t)b * kc + base + c0 + u) : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        double s = v[u][0];
+#pragma unroll
+        for (int w = 1; w < kSl; ++w) s += v[u][w];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0 && c0 + u < kb) sh[c0 + u] = s;
       }
-    double mine = 0.0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      double s = v[u][0];
-#pragma unroll
-      for (int w = 1; w < kSl; ++w) s += v[u][w];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == u) mine = s;
     }
-    if (lane < 4 && c0 + lane < kc) fin(c0 + lane, mine);
+    __syncthreads();
+    if ((int)threadIdx.x < kb) fin(base + (int)threadIdx.x, sh[threadIdx.x]);
+    __syncthreads();
   }
 }
 
@@ -254,7 +258,7 @@ __global__ void __launch_bounds__(kCgThreads)
     const double sc = s[c];
     return CgApply{p, z, q, sc * sc};
   });
-  cg_dot_finish(kc, partial, ctl, [&](int c, double v) { pq[c] = v; });
+  cg_dot_finish(sh, kc, partial, ctl, [&](int c, double v) { pq[c] = v; });
 }
 
 __global__ void __launch_bounds__(kCgThreads)
@@ -271,7 +275,7 @@ __global__ void __launch_bounds__(kCgThreads)
   });
   if (threadIdx.x == 0) above = 0;
   bool mine = false;  // this CTA is the last one
-  cg_dot_finish(kc, partial, ctl, [&](int c, double v) {
+  cg_dot_finish(sh, kc, partial, ctl, [&](int c, double v) {
     beta[c] = rr[c] > 0.0 ? v / rr[c] : 0.0;
     rr[c] = v;
     if (v > tol2 * bb[c]) above = 1;
@@ -400,12 +404,13 @@ struct AProducts {
   int np = 0;  // planes of A (0: strided GEMM)
   PlaneBuf ap;
   PlaneBuf xpn, xpm;  // the other operand's planes (n or m rows), kept across products
-  AProducts(const StageCtx &c_, int m_, int n_, int k, char ordera_, const T *a_, long long lda_)
+  // planes: whether NATIVE may take A's planes at all
+  AProducts(const StageCtx &c_, int m_, int n_, int k, char ordera_, const T *a_, long long lda_, bool planes)
       : c(c_), m(m_), n(n_), ordera(ordera_), a(a_), lda(lda_),
         mixed(c_.precision == kMixed && sizeof(T) == sizeof(float)) {
     np = mixed ? 2 : 0;
     if constexpr (std::is_same<T, float>::value)
-      if (!mixed && f32_operator_pays(m, n, k)) np = 3;
+      if (!mixed && planes && f32_operator_pays(m, n, k)) np = 3;
     if (!np) return;
     try {
       if (ordera == 'R') make_planes<T>(ap, a, lda, m, n, np, false, c.st);  // m x n, n contiguous
@@ -704,22 +709,33 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
   dprod(k, k, n, vd.p, 1, k, hv.p, k, 1, cm.p, k, 1.0, 0.0);        // C = V' H V
   dprod(n, k, k, vd.p, k, 1, cm.p, k, 1, hv.p, k, -0.5, 1.0);       // Z = H V - V C / 2
   {
+    const double *left[3] = {b1d.p, vd.p, hv.p}, *right[3] = {b1d.p, hv.p, vd.p};  // B1' B1, V Z', Z V'
     const long long k3 = 3LL * k;
-    DBuf<double> lhs((size_t)n * k3), rhs((size_t)n * k3);           // [B1' | V | Z], [B1' | Z | V]
-    const double *parts[3] = {b1d.p, vd.p, hv.p};
-    for (int i = 0; i < 3; ++i) {
-      copy2d<double, double>(parts[i], k, 1, lhs.p + i * k, k3, 1, n, k, st);
-      copy2d<double, double>(parts[i == 0 ? 0 : 3 - i], k, 1, rhs.p + i * k, k3, 1, n, k, st);
-    }
+    DBuf<double> lhs, rhs;
     Gemm<double, double> g;
-    g.M = n; g.N = n; g.K = (int)k3;
-    g.A = lhs.p; g.a_rs = k3; g.a_cs = 1;
-    g.B = rhs.p; g.b_rs = 1; g.b_cs = k3;
+    g.M = n; g.N = n;
     g.C = G.p; g.c_rs = n; g.c_cs = 1;
     g.alpha = -1.0; g.beta = 1.0;
     g.upper = true;
     g.splits = 1;
-    gemm(g, st);
+    if (fits_memory([&] { lhs.alloc((size_t)n * k3); rhs.alloc((size_t)n * k3); })) {
+      for (int i = 0; i < 3; ++i) {
+        copy2d<double, double>(left[i], k, 1, lhs.p + i * k, k3, 1, n, k, st);
+        copy2d<double, double>(right[i], k, 1, rhs.p + i * k, k3, 1, n, k, st);
+      }
+      g.K = (int)k3;
+      g.A = lhs.p; g.a_rs = k3; g.a_cs = 1;
+      g.B = rhs.p; g.b_rs = 1; g.b_cs = k3;
+      gemm(g, st);
+    } else {
+      lhs.release();
+      g.K = k;
+      for (int i = 0; i < 3; ++i) {
+        g.A = left[i]; g.a_rs = k; g.a_cs = 1;
+        g.B = right[i]; g.b_rs = 1; g.b_cs = k;
+        gemm(g, st);
+      }
+    }
     mirror_upper(G.p, n, n, st);
   }
   PlaneBuf gp;
@@ -833,12 +849,11 @@ int complement_gram_cg(const StageCtx &c, AProducts<T> &A, int k, const T *u, lo
   return its * ns;
 }
 
-}  // namespace
-
+// As svd_adjoint_dev; planes: AProducts.
 template <class T>
-int svd_adjoint_dev(const StageCtx &c, int m, int n, int k, char ordera, const T *a, long long lda, const T *u,
-                    long long ldu, const T *s, const T *v, long long ldv, const T *du, long long lddu, const T *ds,
-                    const T *dv, long long lddv, T *da, long long ldda, int cg_iters, double tol) {
+int adjoint_with(const StageCtx &c, int m, int n, int k, char ordera, const T *a, long long lda, const T *u,
+                 long long ldu, const T *s, const T *v, long long ldv, const T *du, long long lddu, const T *ds,
+                 const T *dv, long long lddv, T *da, long long ldda, int cg_iters, double tol, bool planes) {
   cudaStream_t st = c.st;
   const size_t mk = (size_t)m * k, nk = (size_t)n * k, kk = (size_t)k * k;
   DBuf<T> ru(mk), rv(nk), lam(mk), gam(nk), w1(nk), w2(mk), tk(kk), J(kk);
@@ -869,7 +884,7 @@ int svd_adjoint_dev(const StageCtx &c, int m, int n, int k, char ordera, const T
   }
   adj_core_kernel<T><<<egrid((long long)kk), 256, 0, st>>>(k, s, ds, K1.p, K2.p, J.p);
   KLAUNCHED();
-  AProducts<T> A(c, m, n, k, ordera, a, lda);
+  AProducts<T> A(c, m, n, k, ordera, a, lda, planes);
   if (!du) CK(cudaMemsetAsync(lam.p, 0, mk * sizeof(T), st));
   if (!dv) CK(cudaMemsetAsync(gam.p, 0, nk * sizeof(T), st));
   // MIXED, n <= m: the systems in the n-dimensional coordinates of B'B (ISVD_GPU_ADJOINT_CG_A=1 keeps
@@ -899,19 +914,49 @@ int svd_adjoint_dev(const StageCtx &c, int m, int n, int k, char ordera, const T
   colscale_add<T>(st, w2.p, lam.p, s, 1, 1.0, w2.p, m, k);
   // dA = U Q1' + P2 V'  (stored per ordera)
   const long long crs = (ordera == 'R') ? ldda : 1, ccs = (ordera == 'R') ? 1 : ldda;
-  {  // one product [U | P2] [Q1 | V]': dA is written once
-    const long long k2 = 2LL * k;
-    DBuf<T> lhs((size_t)m * k2), rhs((size_t)n * k2);
+  Gemm<T, T> g;
+  g.M = m; g.N = n; g.K = k;
+  g.C = da; g.c_rs = crs; g.c_cs = ccs;
+  DBuf<T> lhs, rhs;
+  const long long k2 = 2LL * k;
+  if (fits_memory([&] { lhs.alloc((size_t)m * k2); rhs.alloc((size_t)n * k2); })) {
+    // one product [U | P2] [Q1 | V]': dA is written once
     copy2d<T, T>(u, ldu, 1, lhs.p, k2, 1, m, k, st);
     copy2d<T, T>(w2.p, k, 1, lhs.p + k, k2, 1, m, k, st);
     copy2d<T, T>(w1.p, k, 1, rhs.p, k2, 1, n, k, st);
     copy2d<T, T>(v, ldv, 1, rhs.p + k, k2, 1, n, k, st);
-    Gemm<T, T> g;
-    g.M = m; g.N = n; g.K = (int)k2;
+    g.K = (int)k2;
     g.A = lhs.p; g.a_rs = k2; g.a_cs = 1;
     g.B = rhs.p; g.b_rs = 1; g.b_cs = k2;
-    g.C = da; g.c_rs = crs; g.c_cs = ccs;
     gemm(g, st);
+  } else {
+    lhs.release();
+    g.A = u; g.a_rs = ldu; g.a_cs = 1;
+    g.B = w1.p; g.b_rs = 1; g.b_cs = k;
+    gemm(g, st);
+    g.A = w2.p; g.a_rs = k;
+    g.B = v; g.b_cs = ldv;
+    g.beta = 1.0;
+    gemm(g, st);
+  }
+  return iters;
+}
+
+}  // namespace
+
+template <class T>
+int svd_adjoint_dev(const StageCtx &c, int m, int n, int k, char ordera, const T *a, long long lda, const T *u,
+                    long long ldu, const T *s, const T *v, long long ldv, const T *du, long long lddu, const T *ds,
+                    const T *dv, long long lddv, T *da, long long ldda, int cg_iters, double tol) {
+  auto run = [&](bool planes) {
+    return adjoint_with<T>(c, m, n, k, ordera, a, lda, u, ldu, s, v, ldv, du, lddu, ds, dv, lddv, da, ldda, cg_iters,
+                           tol, planes);
+  };
+  if (c.precision == kMixed || sizeof(T) == sizeof(double)) return run(true);
+  int iters = 0;  // NATIVE FP32 has fitted without A's planes: again, when something beside them does not
+  if (!fits_memory([&] { iters = run(true); })) {
+    trim_pool();
+    iters = run(false);
   }
   return iters;
 }

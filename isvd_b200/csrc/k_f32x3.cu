@@ -233,18 +233,6 @@ template bool gemm_f32_planes<float>(const Gemm<float, float> &, bool, bool, cud
 template bool gemm_f32_planes<double>(const Gemm<float, double> &, bool, bool, cudaStream_t);
 
 // ------------------------------------------------------------------------- stages (mixed.h)
-// Runs f; false when it ran out of memory.
-template <class F>
-static bool fits_memory(F f) {
-  try {
-    f();
-  } catch (const Error &e) {
-    if (e.code != kErrMemory) throw;
-    return false;
-  }
-  return true;
-}
-
 bool f32_block_planes(PlaneBuf &pb, const float *y, long long ldy, long long rows, int l, int N, cudaStream_t st) {
   if (planes_off() || Runtime::get().cc_major != 10) return false;
   // the Grams and the applies from one split
@@ -287,6 +275,7 @@ bool f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp
 bool f32_operator_pays(long long m, long long n, int k) {
   // A is split once for all the products of the iterations: each reads its planes
   if (planes_off() || Runtime::get().cc_major != 10) return false;
+  if (isvd_gpu_memory_limit > 0 && 6.0 * m * n > isvd_gpu_memory_limit / 2.0) return false;
   const double kp = std::ceil(k / 64.0) * 64;
   return (double)m * n * 6.0 / 5e12 + 6.0 * 2.0 * m * n * kp / 1.1e15 + 20e-6 < 0.7 * 2.0 * m * n * kp / 30e12;
 }

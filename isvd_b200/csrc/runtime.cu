@@ -99,9 +99,15 @@ void set_default_precision(int p) { g_precision = p; }
 
 Spare *g_spare = nullptr;
 
+static bool capturing() {
+  cudaStreamCaptureStatus s;
+  CK(cudaStreamIsCapturing(Runtime::get().stream, &s));
+  return s != cudaStreamCaptureStatusNone;
+}
+
 static cudaError_t try_alloc(void **p, size_t bytes) {
   Runtime &rt = Runtime::get();
-  if (isvd_gpu_alloc_limit > 0) {  // diagnostic: as if the device had no more
+  if (isvd_gpu_alloc_limit > 0 && !capturing()) {  // diagnostic: as if the device had no more
     cudaMemPool_t pool;
     unsigned long long used = 0;
     CK(cudaStreamSynchronize(rt.stream));
@@ -114,14 +120,19 @@ static cudaError_t try_alloc(void **p, size_t bytes) {
   return e;
 }
 
+void trim_pool() {
+  Runtime &rt = Runtime::get();
+  cudaMemPool_t pool;
+  CK(cudaStreamSynchronize(rt.stream));
+  CK(cudaDeviceGetDefaultMemPool(&pool, rt.device));
+  CK(cudaMemPoolTrimTo(pool, 0));
+}
+
 void *dev_alloc(size_t bytes) {
   void *p = nullptr;
   cudaError_t e = try_alloc(&p, bytes);
-  if (e != cudaSuccess && g_spare && g_spare->give_back()) {
-    cudaMemPool_t pool;  // the freed block as device memory for any size
-    CK(cudaStreamSynchronize(Runtime::get().stream));
-    CK(cudaDeviceGetDefaultMemPool(&pool, Runtime::get().device));
-    CK(cudaMemPoolTrimTo(pool, 0));
+  if (e != cudaSuccess && g_spare && !capturing() && g_spare->give_back()) {
+    trim_pool();
     e = try_alloc(&p, bytes);
   }
   if (e != cudaSuccess)

@@ -101,6 +101,19 @@ extern Spare *g_spare;  // at most one, null when there is none
 
 void *dev_alloc(size_t bytes);
 void dev_free(void *p);
+void trim_pool();  // after the stream's work: what the pool holds and does not use goes back to the device
+
+// Runs f; false when it ran out of device memory.
+template <class F>
+bool fits_memory(F &&f) {
+  try {
+    f();
+  } catch (const Error &e) {
+    if (e.code != kErrMemory) throw;
+    return false;
+  }
+  return true;
+}
 
 template <class T>
 void DBuf<T>::alloc(size_t count) {

@@ -107,3 +107,21 @@ def test_solve(lib, room, algs, megabytes):
     # FP32 solves of the same sketch by other roundings: a few tens of u sqrt(n) at most
     assert float((s1 - s0).abs().max()) <= 20 * U * n ** 0.5 * float(s0[0])
     assert _rel(a1, a0) <= 100 * U * n ** 0.5
+
+
+@pytest.mark.parametrize("megabytes", [40, 176, 180, 184, 188, 192, 196, 200, 208, 400])
+def test_native_adjoint(lib, room, megabytes):
+    """The planes of A are 171 MB, everything else up to 40 MB."""
+    from test_gpu_adjoint_sizes import _adjoint
+    m, n, k = 9519, 3069, 48
+    g = torch.Generator(device="cuda").manual_seed(m)
+    rn = lambda *sh: torch.randn(*sh, device="cuda", dtype=torch.float64, generator=g)  # noqa: E731
+    r = 4 * k
+    uu, vv = torch.linalg.qr(rn(m, r))[0], torch.linalg.qr(rn(n, r))[0]
+    sig = torch.cat([torch.arange(2 * k, k, -1), torch.linspace(0.3 * k, 0.1, r - k)]).to("cuda", torch.float64)
+    f = lambda t: t.to(torch.float32).contiguous()  # noqa: E731
+    args = f((uu * sig) @ vv.t()), f(sig[:k]), f(uu[:, :k]), f(vv[:, :k]), f(rn(k)), f(rn(m, k)), f(rn(n, k)), 200, 1e-9
+    ref, _ = _adjoint(lib, "s", *args)
+    room(megabytes)
+    da, _ = _adjoint(lib, "s", *args)
+    assert _rel(da, ref) <= 20 * U  # either within 10 u of the FP64 adjoint (test_gpu_adjoint_native.py)

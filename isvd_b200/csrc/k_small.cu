@@ -72,12 +72,12 @@ template <bool VS, int NT = kEigThreads>
 __global__ void __launch_bounds__(NT)
     sym_eig_kernel(int n_uniform, const double *__restrict__ Ag, double *__restrict__ Vg, double *__restrict__ wg,
                    int order, bool absval, double *__restrict__ scratch, int *status, const EigDesc *desc,
-                   const double *refined, size_t refined_stride) {
+                   const double *refined, size_t refined_stride, bool rest) {
   extern __shared__ double sm[];
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int n = desc ? desc[b].n : n_uniform;
-  // after eig_refined: only the matrices it did not settle
-  const double *rw = desc ? desc[b].work : refined ? refined + (size_t)b * refined_stride : nullptr;
+  // rest (after eig_refined): only the matrices it did not settle
+  const double *rw = !rest ? nullptr : desc ? desc[b].work : refined ? refined + (size_t)b * refined_stride : nullptr;
   if (rw && !*(const int *)(rw + eig_need_at(n))) return;
   const double *A0 = desc ? desc[b].A : Ag + (size_t)b * n * n;
   double *V = desc ? desc[b].V : Vg + (size_t)b * n * n;
@@ -997,7 +997,7 @@ void sym_eig_batched(int n, int batch, const double *A, double *V, double *w, in
   if (smem_vs <= rt.smem_optin) {
     CK(cudaFuncSetAttribute(sym_eig_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_vs));
     sym_eig_kernel<true><<<batch, kEigThreads, smem_vs, st>>>(n, A, V, w, order, absval, nullptr, status, nullptr,
-                                                              work.p, stride);
+                                                              work.p, stride, work.p != nullptr);
     KLAUNCHED();
     return;
   }
@@ -1006,7 +1006,7 @@ void sym_eig_batched(int n, int batch, const double *A, double *V, double *w, in
   DBuf<double> scratch((size_t)batch * n * n);
   CK(cudaFuncSetAttribute(sym_eig_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   sym_eig_kernel<false><<<batch, kEigThreads, smem, st>>>(n, A, V, w, order, absval, scratch.p, status,
-                                                            nullptr, work.p, stride);
+                                                            nullptr, work.p, stride, work.p != nullptr);
   KLAUNCHED();
 }
 
@@ -1016,12 +1016,13 @@ void sym_eig_grouped(const EigDesc *desc, int count, int max_n, int order, bool 
   const size_t smem = eig_smem(max_n, true);
   if (smem > Runtime::get().smem_optin)
     fail(kErrUnsupported, "symmetric eigensolver: l = %d exceeds on-chip capacity", max_n);
-  if (!eig_refined_usable(max_n)) fail(kErrUnsupported, "grouped eigensolver: no thread-block cluster launch");
-  eig_refined(max_n, count, nullptr, nullptr, nullptr, nullptr, order, absval, desc, st);
-  // the matrices that did not settle; the smallest CTA that holds the largest matrix: small matrices leave room for many CTAs per SM
+  const bool refined = eig_refined_usable(max_n);
+  if (refined) eig_refined(max_n, count, nullptr, nullptr, nullptr, nullptr, order, absval, desc, st);
+  // the matrices that did not settle, or all; the smallest CTA that holds the largest matrix: small matrices leave
+  // room for many CTAs per SM
   auto go = [&](auto kernel, int nt) {
     CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<count, nt, smem, st>>>(0, nullptr, nullptr, nullptr, order, absval, nullptr, status, desc, nullptr, 0);
+    kernel<<<count, nt, smem, st>>>(0, nullptr, nullptr, nullptr, order, absval, nullptr, status, desc, nullptr, 0, refined);
     KLAUNCHED();
   };
   if (max_n <= eig_max_n(128)) go(sym_eig_kernel<true, 128>, 128);

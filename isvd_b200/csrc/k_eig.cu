@@ -11,7 +11,10 @@
 // The error is squared by every refinement, which also restores orthonormality: three to five take
 // it from single precision to FP64 rounding.  A matrix that they do not settle (clusters that FP32
 // cannot separate, a Cholesky breakdown, non-finite entries) sets its `need` word and is solved by
-// the FP64 two-sided Jacobi of k_small.cu instead.
+// the FP64 two-sided Jacobi of k_small.cu instead; so is a graded one, whose row norms differ by more than
+// kGraded: the refinement's eigenvalues are good to rounding of ||W||, Jacobi's to rounding of their own rows
+// (singular values from Gram matrices D H D, l = 64, relative to themselves: D down to 1e-3 8e-15 by either,
+// 1e-4 1e-14 by Jacobi and 7e-14 refined, 1e-6 9e-15 and 1e-10).
 //
 // Why: the two-sided Jacobi in FP64 is bound by the latency of its n - 1 rounds a sweep, nine to ten
 // sweeps (about 2.5 us a round: FP64 root and division chains, 2 n^2 doubles through shared memory,
@@ -39,6 +42,9 @@ constexpr int kMaxN = kKrMaxL;
 constexpr int kOsjSweeps = 16;
 constexpr int kRefine = 8;
 constexpr int kEigBlocks = 4;  // X, T = X W, R (then E'), S
+// (row norms of D H D differ by about the range of D; those of a solve's Gram matrices, whose bases mix the
+// singular directions, by factors of 2 to 6)
+constexpr double kGraded = 500.0;
 
 // work of one matrix (doubles): X0 | X1 | W (symmetrised) | S | lambda | slots[64], scalars
 struct EigWork {
@@ -152,7 +158,7 @@ __device__ __forceinline__ void osj_rotate(f2 (&x)[8][EPL], float &al, float &be
 // floats each way; blocks of four move a quarter of that), in FP32 pairs.
 template <int EPL>
 __global__ void __launch_bounds__(256) osj_kernel(int n_uniform, const double *__restrict__ Ag, double *workg,
-                                                  size_t work_stride, int psd, const EigDesc *desc) {
+                                                  size_t work_stride, int psd, bool loose, const EigDesc *desc) {
   extern __shared__ double sm[];
   const int b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
@@ -197,6 +203,35 @@ __global__ void __launch_bounds__(256) osj_kernel(int n_uniform, const double *_
   dm = 0.0;
   for (int i = 0; i < nwarp; ++i) dm = fmax(dm, red[i]);
   const double fro = scal[0];
+
+  if (!loose) {  // graded: Jacobi's
+    double lo = INFINITY, hi = 0.0;
+    for (int i = warp; i < n; i += nwarp) {
+      double s = 0.0;
+      for (int j = lane; j < n; j += 32) {
+        const double v = L[j <= i ? pl(i, j) : pl(j, i)];
+        s += v * v;
+      }
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      lo = fmin(lo, s);
+      hi = fmax(hi, s);
+    }
+    __syncthreads();  // red has been read
+    if (lane == 0) {
+      red[warp] = lo;
+      red[8 + warp] = hi;
+    }
+    __syncthreads();
+    for (int i = 0; i < nwarp; ++i) {
+      lo = fmin(lo, red[i]);
+      hi = fmax(hi, red[8 + i]);
+    }
+    __syncthreads();
+    if (hi > kGraded * kGraded * lo) {
+      if (tid == 0) *w.need = 1;
+      return;
+    }
+  }
 
   // Cholesky (right-looking, one column per step); a Gram matrix that is singular to rounding is
   // factored once more with a shift that leaves its eigenvectors alone
@@ -547,7 +582,7 @@ void eig_refined(int n, int count, const double *A, double *work, double *V, dou
   const size_t osm = osj_smem(n);
   with_epl(n, [&](auto kern) {
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)osm));
-    kern<<<count, osj_threads(n), osm, st>>>(n, A, work, stride, absval ? 1 : 0, desc);
+    kern<<<count, osj_threads(n), osm, st>>>(n, A, work, stride, absval ? 1 : 0, loose, desc);
     KLAUNCHED();
   });
   const int cs = refine_cluster(n, count);

@@ -392,6 +392,9 @@ __global__ void __launch_bounds__(256) osj_kernel(int n_uniform, const double *_
   }
 }
 
+// The larger of two magnitudes; a NaN, once met, stays.
+__device__ __forceinline__ double larger(double a, double b) { return isnan(a) ? a : (isnan(b) || b > a) ? b : a; }
+
 // One cluster per matrix: the FP64 refinement on the rows of X' (row i = eigenvector i), then the
 // eigenpairs in order (as sym_eig_batched).  loose: eigenvectors that are not separated stay mixed, as
 // orthonormal as the others.
@@ -470,13 +473,12 @@ __global__ void __launch_bounds__(kKrThreads, 1)
         }
       }
       R[e] = v;
-      if (!(m <= mx)) mx = m;
+      mx = larger(mx, m);
     });
     if (bad) sbad = 1;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      const double v = __shfl_xor_sync(0xffffffffu, mx, o);
-      if (!(v <= mx)) mx = v;
+      mx = larger(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
     if ((tid & 31) == 0) red[tid >> 5] = mx;
     __syncthreads();
@@ -487,16 +489,14 @@ __global__ void __launch_bounds__(kKrThreads, 1)
     });
     if (tid == 0) {
       double m = 0.0;
-      for (int i = 0; i < kKrWarps; ++i)
-        if (!(red[i] <= m)) m = red[i];
+      for (int i = 0; i < kKrWarps; ++i) m = larger(m, red[i]);
       g.slots[k.rank] = m;
       g.slots[16 + k.rank] = sbad;
     }
     cluster.sync();
     double m = 0.0, nbad = 0.0;
     for (int r = 0; r < k.cs; ++r) {
-      const double v = __ldcg(g.slots + r);
-      if (!(v <= m)) m = v;
+      m = larger(m, __ldcg(g.slots + r));
       nbad += __ldcg(g.slots + 16 + r);
     }
     settled = nbad == 0.0 && m <= 3e-9;  // what is left is of the order of m^2

@@ -9,7 +9,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -200,14 +199,22 @@ bool pageable(const void *p) {
   return attr.type == cudaMemoryTypeUnregistered;
 }
 
+// The pinned buffers and their events, all or none.
 bool stage_ready(Runtime &rt) {
   if (rt.stage) return true;
   void *p = nullptr;
-  if (cudaMallocHost(&p, Runtime::kStageSlots * Runtime::kStageBytes) != cudaSuccess) {
+  cudaError_t e = cudaMallocHost(&p, Runtime::kStageSlots * Runtime::kStageBytes);
+  int made = 0;
+  while (e == cudaSuccess && made < Runtime::kStageSlots) {
+    e = cudaEventCreateWithFlags(&rt.stage_ev[made], cudaEventDisableTiming);
+    if (e == cudaSuccess) ++made;
+  }
+  if (e != cudaSuccess) {
     cudaGetLastError();
+    while (made > 0) cudaEventDestroy(rt.stage_ev[--made]);
+    if (p) cudaFreeHost(p);
     return false;
   }
-  for (cudaEvent_t &e : rt.stage_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   rt.stage = static_cast<unsigned char *>(p);
   return true;
 }
@@ -267,8 +274,9 @@ void copy_to_device(void *dst, size_t dpitch, const void *src, size_t spitch, si
   std::vector<std::thread> pool;
   const int count = (int)std::min<size_t>(threads, pieces);
   try {
+    pool.reserve(count);
     for (int t = 1; t < count; ++t) pool.emplace_back(work, t);
-  } catch (const std::system_error &) {  // no more threads: the ones that run take all pieces
+  } catch (const std::exception &) {  // no more threads or memory: the threads that run take all pieces
   }
   work(0);
   for (std::thread &t : pool) t.join();

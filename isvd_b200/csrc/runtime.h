@@ -132,8 +132,8 @@ void DBuf<T>::release() {
 bool is_device_pointer(const void *p);
 
 // Copy of `rows` lines of `width` bytes from host memory (line stride spitch) to device memory (dpitch),
-// ordered on st; the host memory has been read when it returns.  Pageable memory of several MB goes
-// through pinned buffers filled by several host threads (runtime.cu).
+// ordered on st; pageable host memory has been read when it returns, page-locked memory when the copy has run.
+// Pageable memory of several MB goes through pinned buffers filled by several host threads (runtime.cu).
 void copy_to_device(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, size_t rows,
                     cudaStream_t st);
 

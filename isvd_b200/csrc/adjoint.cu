@@ -433,7 +433,7 @@ struct AProducts {
         ++g.nprod;
       }
     }
-    g.chunk_k = mixed ? 0 : f32_chunk();
+    g.chunk_k = mixed ? 0 : 1;  // NATIVE: one k-block
     g.unbias = !mixed;
   }
   // Y = A X (m x k) or, transpose, A' X (n x k)

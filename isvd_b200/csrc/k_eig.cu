@@ -8,8 +8,8 @@
 //                   decomposition", Japan J. Indust. Appl. Math. 35 (2018)): with R = I - X'X,
 //                   S = X'WX and lambda_i = s_ii / (1 - r_ii),
 //                   e_ij = (s_ij + lambda_j r_ij) / (lambda_j - lambda_i), e_ii = r_ii / 2.
-// The error is squared by every refinement, which also restores orthonormality: three to five take
-// it from single precision to FP64 rounding.  A matrix that they do not settle (clusters that FP32
+// The error is squared by every refinement, which also restores orthonormality: two or three take it from single
+// precision to FP64 rounding.  A matrix that they do not settle (clusters that FP32
 // cannot separate, a Cholesky breakdown, non-finite entries) sets its `need` word and is solved by
 // the FP64 two-sided Jacobi of k_small.cu instead; so is a graded one, whose row norms differ by more than
 // kGraded: the refinement's eigenvalues are good to rounding of ||W||, Jacobi's to rounding of their own rows

@@ -1,8 +1,11 @@
 // FP32 products on the bf16 tensor cores: an FP32 operand is the sum of three bf16 planes to its last
-// bit (8 + 8 + 8 significant bits), and the six plane pairs (p, q) with p + q < 3 leave out terms below
-// 2^-24 of a term, under the rounding of one FP32 multiply-add.  The tcgen05 engine (umma.h) adds them
-// in FP32 in chunks of 128 terms, and the chunks round-to-nearest in FP32, so that long sums carry less
-// rounding than the single FP32 chain per output of the CUDA-core kernel (k_gemm.cu).
+// bit (8 + 8 + 8 significant bits; below 2^-110 the last plane runs out of bf16's exponents), and the six
+// plane pairs (p, q) with p + q < 3 leave out terms below 2^-24 of a term, under the rounding of one FP32
+// multiply-add.  The tcgen05 engine (umma.h) adds them in FP32 in chunks of one k-block (32 or 64 terms, by
+// the tile shape), and the chunks round-to-nearest in FP32, so that long sums carry less rounding than the
+// single FP32 chain per output of the CUDA-core kernel (k_gemm.cu).  A NaN or an infinity in an operand makes
+// its outputs non-finite (an infinity meets the other operand's zero planes as NaN; a sketch with a drawn
+// Omega, one plane, keeps it infinite).
 //
 // gemm<float, .> comes here for products that are large enough to pay for the splits (plane_product_pays).
 #include <algorithm>
@@ -97,6 +100,7 @@ void six_products(UmmaGemm &g) {
   for (int s = 2; s >= 0; --s)
     for (int p = 0; p <= s; ++p) { g.pa[g.nprod] = p; g.pb[g.nprod] = s - p; ++g.nprod; }
   g.unbias = true;
+  g.chunk_k = 1;  // one k-block
 }
 
 int *engine_status() { return reinterpret_cast<int *>(Runtime::get().ctl + 16); }  // the stages' status word
@@ -111,13 +115,12 @@ long long plane_cap() {
 
 }  // namespace
 
-// Depth of an accumulation chunk.  The tensor core truncates at every 16-deep step of a chunk, the
-// chunks are added in round-to-nearest.  The plane pairs run smallest first, so that in a chunk of one
-// k-block only the last steps truncate at the full magnitude.  Relative error of A Omega against 64 bits
+// Depth of an accumulation chunk: one k-block, except in long sketches.  The tensor core truncates at every
+// 16-deep step of a chunk, the chunks are added in round-to-nearest.  The plane pairs run smallest first, so that
+// in a chunk of one k-block only the last steps truncate at the full magnitude.  Relative error of A Omega against 64 bits
 // at n = 150 / 300 / 1000 / 10000: CUDA-core FP32 2.2e-7 / 3.1e-7 / 4.0e-7 / 1.8e-6; chunks of 128 3.5e-7 /
 // 3.6e-7 / 3.8e-7 / 4.1e-7, of 64 1.7e-7 / 1.8e-7 / 1.8e-7 / 2.9e-7, of 32 0.7e-7 / 0.9e-7 / 0.8e-7 / 3.2e-7.
 // Long sketches, which are bound by the tensor pipe, take 64 (32 costs 9 % at n = 10000).
-int f32_chunk() { return 32; }
 static int f32_sketch_chunk(int n) { return n <= 1024 ? 32 : 64; }
 
 // Time of the product by either path.  CUDA cores: 30 TFLOP/s on whole tiles (64 x 64 when either side
@@ -149,7 +152,6 @@ bool gemm_f32_planes(const Gemm<float, Tout> &g, bool a_kc, bool b_nc, cudaStrea
   u.upper = g.upper;
   u.status = g.status ? g.status : engine_status();
   u.tag = "fp32";
-  u.chunk_k = f32_chunk();
   six_products(u);
   u.unbias = g.unbias;
   PlaneBuf pa, pb;
@@ -249,7 +251,6 @@ bool f32_block_gram(const PlaneBuf &yp, int rows, int l, int N, double *W, cudaS
   u.C = W; u.c_double = true; u.c_rs = l; u.c_cs = 1;
   u.status = engine_status();
   u.tag = "block_gram";
-  u.chunk_k = f32_chunk();
   six_products(u);
   return fits_memory([&] { umma_gemm(u, st); });
 }
@@ -267,7 +268,6 @@ bool f32_block_apply(const PlaneBuf &yp, int rows, int l, int N, const float *Wp
   u.C = out; u.c_rs = ldo; u.c_cs = 1;
   u.status = engine_status();
   u.tag = "block_apply";
-  u.chunk_k = f32_chunk();
   six_products(u);
   return fits_memory([&] { umma_gemm(u, st); });
 }
@@ -295,7 +295,6 @@ bool f32_tall_gram(const PlaneBuf &qp, int rows, int Nl, double *G, cudaStream_t
   u.upper = true;
   u.status = engine_status();
   u.tag = "gram_full";
-  u.chunk_k = f32_chunk();
   six_products(u);
   if (!fits_memory([&] { umma_gemm(u, st); })) return false;
   mirror_upper(G, Nl, Nl, st);
@@ -312,7 +311,6 @@ bool f32_tall_apply(const PlaneBuf &qp, int rows, int Nl, int l, const float *M,
   u.C = out; u.c_rs = ldo; u.c_cs = 1;
   u.status = engine_status();
   u.tag = "coeff_apply";
-  u.chunk_k = f32_chunk();
   six_products(u);
   return fits_memory([&] { umma_gemm(u, st); });
 }
@@ -412,7 +410,6 @@ bool f32_project(MixedCache *mc, int m, int n, int l, char ordera, const float *
   u.C = z; u.c_rs = 1; u.c_cs = l;  // Z' tile written into Z (n x l)
   u.status = engine_status();
   u.tag = "project";
-  u.chunk_k = f32_chunk();
   six_products(u);
   if (fits_memory([&] { umma_gemm(u, st); })) return true;
   mc->drop();

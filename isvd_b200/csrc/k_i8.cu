@@ -27,11 +27,12 @@
 // of the 28, all 14 planes), then s = 0..2 (6 products, the three leading planes of either side) and (**).  The
 // drained int32 sums of a pass combine exactly in int64 and join the FP64 running sums in registers.
 //
-// Measured, mma.sync f64 -> here with the digits: 40000 x 1536 x 6000 26.6 -> 7.8 ms (6.6 ms of products at
-// 3.1e15 int8 op/s, the tensor cores' rate); 20011 x 1024 x 1501 2.35 -> 0.80 ms; Gram 1536 x 1536 x 40000
-// 7.0 -> 1.4 ms; 777 x 1000 x 9001 0.71 -> 0.30 ms.  Errors against exact sums, rms relative to |a_i||b_j|:
-// 6.7e-18 (mma.sync f64: 3.3e-17) at K = 1501, 5.4e-18 (3.3e-17) at 6000, 4.4e-18 (4.4e-17) at 40000, with
-// positive entries 2.3e-17 (6.2e-16) at 1501.  Operands of which every tile fails (*) cost 8 % more.
+// Measured, mma.sync f64 -> here with the digits: 40000 x 1536 x 6000 26.6 -> 8.2 ms (7.2 ms of products at
+// 2.9e15 int8 op/s of the 28 pairs, the tensor cores' rate with (**)'s 29th product); 20011 x 1024 x 1501
+// 2.35 -> 0.85 ms; Gram 1536 x 1536 x 40000 7.0 -> 1.4 ms; 777 x 1000 x 9001 0.71 -> 0.31 ms.  (**) costs 4 to 5 %
+// of that.  Errors against exact sums, rms relative to sum |a_ik| |b_kj|: 1.1e-17 (mma.sync f64: 3.7e-17) at K = 1501,
+// 8.9e-18 (5.3e-17) at 6000, with positive entries 3.7e-17 (4.9e-16) at 1501.  Operands of which every tile fails (*)
+// cost 4 to 10 % more than mma.sync alone, those of which every tile fails only (**) 30 to 36 %.
 #include <cuda.h>
 
 #include <algorithm>

@@ -101,9 +101,7 @@ void f32_sketch_rows(const Planes &omega_t, long long rows, int n, int Nl, char 
 // Z = A' Qbar from the sketch's planes of A; false when mc does not hold them or there is no memory beside them.
 bool f32_project(MixedCache *mc, int m, int n, int l, char ordera, const float *a, const float *qt, long long ldqt,
                  float *z, cudaStream_t st);
-// Accumulation chunk of FP32-exact plane products; whether repeated products of an m x n A with
-// k columns are faster from A's three planes.
-int f32_chunk();
+// Whether repeated products of an m x n A with k columns are faster from A's three planes.
 bool f32_operator_pays(long long m, long long n, int k);
 // Planes of the N column blocks (l columns, each block padded to a multiple of 8) of a tall matrix, and
 // W_i = Y_i' Y_i and out_i = Y_i Wp_i from them (out may be the matrix itself).  f32_block_planes: false

@@ -41,7 +41,7 @@ struct UmmaGemm {
   double alpha = 1.0;
   int splits = 0;      // split-K (0: automatic); partial sums are added in FP64
   bool upper = false;  // symmetric output: only tiles touching the upper triangle, j >= i written
-  int chunk_k = 0;     // K depth of one tensor-memory accumulation chunk (0: 128)
+  int chunk_k = 0;     // K depth of one tensor-memory accumulation chunk (0: 128; at least one k-block)
   // FP32-exact products.  The tensor core truncates its FP32 accumulator, which shrinks every sum alike:
   // with chunks of one k-block, pairs ordered smallest first, by 4.5e-8 (32-deep) or 9e-8 (64-deep)
   // of Gaussian products and as much of positive ones.  unbias gives the mean of the cut, half or three

@@ -37,8 +37,10 @@ extern size_t isvd_gpu_alloc_limit;
 
 /* ---------------------------------------------------------------- precision */
 #define ISVD_GPU_PRECISION_NATIVE   0  /* products in the routine's own type (FP64 for isvd_d*, FP32 for isvd_s*); large
-                                          FP32 products on tcgen05 from operands split exactly into three bf16
-                                          planes, with less rounding than an FP32 multiply-add chain */
+                                          FP32 products on tcgen05 from operands split exactly (above 2^-110) into
+                                          three bf16 planes, with less rounding than an FP32 multiply-add chain;
+                                          large FP64 products on int8 tensor cores from 55-bit operands, where
+                                          that leaves every entry within the rounding of an FP64 chain */
 #define ISVD_GPU_PRECISION_MIXED    1  /* bf16 split products (2 or 3 planes per operand) on tcgen05 tensor
                                           cores, FP32 accumulation; l x l steps (eigensolves, inverse square
                                           roots, small SVDs) in FP64 */

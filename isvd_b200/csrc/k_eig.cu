@@ -21,7 +21,7 @@
 // the barriers).  The one-sided rounds in FP32 need no eigenvector matrix; the refinement is four
 // products of a cluster (rows.cuh), 10 to 20 us a step, two or three steps.  Measured for the Gram of a
 // solve, two-sided -> this: l = 11 84 -> 37 us, l = 32 273 -> 73, l = 65 987 -> 224, l = 96 2098 -> 364,
-// l = 128 3492 (on a 16-CTA cluster) -> 608.  What is left is the FP32 Jacobi on one SM: six to eight
+// l = 128 3492 (on a 16-CTA cluster) -> 608, plus 2 to 9 us for the row norms of the test for grading.  What is left is the FP32 Jacobi on one SM: six to eight
 // sweeps of n rounds of n / 2 rotations, 0.2 us a round at l = 32 (latency of the reduction and the
 // rotation), 0.5 us at l = 128 (FP32 pipe and shuffles of the SM).
 #include <algorithm>
